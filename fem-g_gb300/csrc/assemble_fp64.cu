@@ -1,331 +1,548 @@
 // Plain FP64 / complex<double> assembly.
 //
-// K1-K3 + K5 (element kernel, one warp per element): for each quadrature
-// point the warp forms the Jacobian, its inverse and determinant (gmsh
-// getJacobians, src/term/Assembler.cpp:131-139), evaluates the coefficient
-// programs at the physical point (EquationEvaluator::initialize,
-// src/term/evaluator/EquationEvaluator.h:155-168), maps the reference
+// K1-K3 + K5, the quadrature loop: for each quadrature point the Jacobian,
+// its inverse and determinant (gmsh getJacobians, src/term/Assembler.cpp:131-139),
+// the coefficient programs at the physical point (EquationEvaluator::initialize,
+// src/term/evaluator/EquationEvaluator.h:155-168), the map of the reference
 // gradients with J^-T (FieldEvaluator<Form1>, src/term/evaluator/FieldEvaluator.h:67-70)
-// and accumulates Ke += w det (c L)^T conj(R) (BilinearTerm::evaluate,
+// and Ke += w det (c L)^T conj(R) (BilinearTerm::evaluate,
 // src/term/BilinearTerm.cpp:314-326) with the AFrequency factors
 // (src/term/Assembler.cpp:283-295), and b_e += w det conj(phi) f
-// (LinearTerm::evaluate, src/term/LinearTerm.cpp:182-191). The tensor
-// grad-grad term (a TensorFunction times grad(dof), the left-order evaluator
-// src/term/evaluator/EquationEvaluator.h:134-173 with a degree-2 function)
-// maps the unknown's gradients by w det c D before the product; D is
-// symmetric here. Ke is symmetric for these terms, so each lane owns
-// upper-triangle entries.
+// (LinearTerm::evaluate, src/term/LinearTerm.cpp:182-191).
+//
+// GB300's FP64 pipe takes 64 cycles per warp instruction and scheduler,
+// whether one lane is active or 32, so what counts is the number of FP64
+// warp instructions and how full their lanes are. Hence:
+//  - The geometry and the coefficients of a point become one small matrix D
+//    in reference coordinates, e.g. w det c J^-1 J^-T, that maps the unknown's
+//    reference tables once (H = D t_j); an entry is then a plain dot product
+//    with the test function's reference table, Ke[i][j] += t_i . H_j.
+//  - Blocks work on several elements, and every phase spreads its items over
+//    all threads: elements (Jacobians), (element, point) pairs (D), (element,
+//    point, function) triples (H), and (element, entry) pairs (the sums).
+//    The entries of all elements of a block are numbered through, so that
+//    small element matrices fill the lanes too.
 //
 // The element matrices and vectors then go through the deterministic CSR
 // reduction of gather.cu.
+#include <algorithm>
+#include <cstring>
+
 #include "common.cuh"
 
 namespace femg {
 
-constexpr int kWarpsPerBlockElem = 4;
+constexpr int kQuadThreads = 128;
+constexpr int kQuadMaxElems = 64;             // elements per block
+constexpr size_t kQuadSmem = 47 * 1024;       // shared memory of a block: no opt-in, room for the tables in L1 at three blocks per SM
+constexpr int kQuadGeom = 31;                 // per element: J, J^-1, det, det J^-1 J^-T, J^T J / det (HCurl)
 
-struct ElemWarpSmem {
-  double X[kMaxNodes * 3];
-  double J0[9], J[9], Jinv[9];
-  double det0, det;
-  double2 a, b, s;  // w det c_gradgrad, w det c_mass, w det f
-  double2 Aw[6];    // w det times the diffusion tensor (tensor grad-grad term)
-  double G[3][kMaxDofs];
-  double phi[kMaxDofs];
-  double Gs[2][3][kMaxDofs];
-  double phis[2][kMaxDofs];
+// Shape and switches of one launch
+struct QuadArgs {
+  int NE;          // elements per block
+  int QD, QC;      // points per chunk of D, and of H within it
+  int nEnt;        // entries accumulated per element: the upper triangle, or all n x nc
+  int comps;       // mask of the table components that contribute (see tableComps)
+  int uniform;     // the scalar bilinear coefficients are constant on each element
+  int needX;       // some coefficient or modificator reads the physical point
 };
 
-template <int MAXENT, bool CPLX>
-__global__ void __launch_bounds__(32 * kWarpsPerBlockElem)
-    k_element_fp64(const PlanDev p, const DevTerms *__restrict__ terms, double *__restrict__ ke, double2 *__restrict__ be) {
-  __shared__ ElemWarpSmem smem[kWarpsPerBlockElem];
-  __shared__ uint8_t pairI[kMaxDofs * (kMaxDofs + 1) / 2], pairJ[kMaxDofs * (kMaxDofs + 1) / 2];
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int n = p.nb;  // scalar field here: n == nb
+// Kinds of element matrices. The table components of a function: H1, the
+// reference gradient and the value (4); HCurl, the reference curl and value
+// (6). D: kQuadSym S (00 11 22 01 02 12) and the mass weight (7); kQuadHcurl
+// the same for curls and for values (12); kQuadFull a 4 x 4 matrix.
+enum { kQuadSym = 0, kQuadHcurl = 1, kQuadFull = 2 };
+__host__ __device__ constexpr int quadComps(int kind) { return kind == kQuadHcurl ? 6 : 4; }
+__host__ __device__ constexpr int quadD(int kind) { return kind == kQuadSym ? 7 : kind == kQuadHcurl ? 12 : 16; }
+
+// Offsets (in doubles) of a block's shared memory
+struct QuadLayout {
+  int X, geom, coef, D, src, be, H, pairs, orient, total;
+};
+// nd: doubles per point, nh: doubles per (point, unknown function), n: test
+// functions (right-hand side entries), nU: unknown functions
+__host__ __device__ inline QuadLayout quadLayout(int NE, int QD, int QC, int nn, int n, int nU, int nd, int nh, bool be, int nPairs) {
+  QuadLayout L;
+  int o = 0;
+  L.be = o;  // double2
+  o += be ? 2 * NE * n : 0;
+  L.X = o;
+  o += NE * nn * 3;
+  L.geom = o;
+  o += NE * kQuadGeom;
+  L.coef = o;
+  o += NE * 6;
+  L.D = o;
+  o += NE * QD * nd;
+  L.src = o;
+  o += be ? NE * QD * 8 : 0;
+  L.H = o;
+  o += NE * QC * nh * nU;
+  L.pairs = o;
+  o += (nPairs * 2 + 7) / 8;
+  L.orient = o;
+  o += NE;  // two ints per element
+  L.total = o;
+  return L;
+}
+
+// One copy of the coefficient interpreter per file (it is large), called
+// where a coefficient is not constant
+__device__ __noinline__ double2 evalExprCall(const DevExpr *ex, int64_t e, const double *x, const double *phi, int nb, int q, int nq) {
+  return evalExpr(*ex, e, x, phi, nb, q, nq);
+}
+struct CoefPoint {
+  int64_t e;
+  const double *x, *phi;
+  int nb, q, nq;
+};
+__device__ __forceinline__ double2 evalAt(const DevExpr &ex, const CoefPoint &c) {
+  if (ex.cls == kExprConst) return ex.cval;
+  return evalExprCall(&ex, c.e, c.x, c.phi, c.nb, c.q, c.nq);
+}
+// A = c0 I + factor c D of tensor term `term` (coefTensor of common.cuh with
+// the shared interpreter)
+__device__ inline void tensorAt(const DevTerms *terms, int term, const DevExpr *D, int g, const CoefPoint &c, double2 c0, double2 *A) {
+  for (int k = 0; k < 6; ++k) A[k] = k < 3 ? c0 : make_double2(0.0, 0.0);
+  if (term < 0 || terms->t[term].mod != g) return;
+  const double2 fc = cmul(terms->t[term].factor, evalAt(terms->t[term].coef, c));
+  for (int k = 0; k < 6; ++k) A[k] = cadd(A[k], cmul(fc, evalAt(D[k], c)));
+}
+// summed scalar coefficients of group g: c[0] grad-grad (curl-curl), c[1]
+// mass; elastic fields: c[0] lambda, c[1] mass, c[2] mu
+__device__ inline void scalarCoefs(const DevTerms *terms, int g, const CoefPoint &cp, double2 *c) {
+  c[0] = c[1] = c[2] = make_double2(0.0, 0.0);
+  for (int t = 0; t < terms->n; ++t) {
+    const DevTerm &T = terms->t[t];
+    if (T.mod != g) continue;
+    if (T.kind == FG_TERM_GRAD_GRAD || T.kind == FG_TERM_ELASTIC) c[0] = cadd(c[0], cmul(T.factor, evalAt(T.coef, cp)));
+    else if (T.kind == FG_TERM_MASS) c[1] = cadd(c[1], cmul(T.factor, evalAt(T.coef, cp)));
+    if (T.kind == FG_TERM_ELASTIC) c[2] = cadd(c[2], cmul(T.factor, evalAt(T.coef2, cp)));
+  }
+}
+
+// J^-1, det J^-1 J^-T and (HCurl fields) J^T J / det, six entries each (00 11
+// 22 01 02 12), from J and its determinant. With the cofactors C,
+// J^-1 = C^T / det, so det J^-1 J^-T = (C^T C) / det. One division: a lane's
+// FP64 instructions here cost the block as much as full warps' do.
+template <bool HCURL>
+__device__ inline void geomMaps(const double *J, double det, double *Ji, double *K6, double *M6) {
+  auto Jm = [&](int r, int c) { return J[3 * c + r]; };
+  double C[9];  // C[3a + r] = (adj J)(a, r)
+  C[0] = Jm(1, 1) * Jm(2, 2) - Jm(1, 2) * Jm(2, 1);
+  C[1] = Jm(0, 2) * Jm(2, 1) - Jm(0, 1) * Jm(2, 2);
+  C[2] = Jm(0, 1) * Jm(1, 2) - Jm(0, 2) * Jm(1, 1);
+  C[3] = Jm(1, 2) * Jm(2, 0) - Jm(1, 0) * Jm(2, 2);
+  C[4] = Jm(0, 0) * Jm(2, 2) - Jm(0, 2) * Jm(2, 0);
+  C[5] = Jm(0, 2) * Jm(1, 0) - Jm(0, 0) * Jm(1, 2);
+  C[6] = Jm(1, 0) * Jm(2, 1) - Jm(1, 1) * Jm(2, 0);
+  C[7] = Jm(0, 1) * Jm(2, 0) - Jm(0, 0) * Jm(2, 1);
+  C[8] = Jm(0, 0) * Jm(1, 1) - Jm(0, 1) * Jm(1, 0);
+  const double id = 1.0 / det;
+  for (int k = 0; k < 9; ++k) Ji[k] = C[k] * id;
+  const int ab[6][2] = {{0, 0}, {1, 1}, {2, 2}, {0, 1}, {0, 2}, {1, 2}};
+  for (int k = 0; k < 6; ++k) {
+    const int a = ab[k][0], b = ab[k][1];
+    K6[k] = (C[3 * a] * C[3 * b] + C[3 * a + 1] * C[3 * b + 1] + C[3 * a + 2] * C[3 * b + 2]) * id;
+    if (HCURL) M6[k] = (J[3 * a] * J[3 * b] + J[3 * a + 1] * J[3 * b + 1] + J[3 * a + 2] * J[3 * b + 2]) * id;
+  }
+}
+
+// Nodes and, for affine elements, the geometry of the block's elements
+// (J, J^-1, det, det J^-1 J^-T and J^T J / det)
+template <bool HCURL>
+__device__ inline void quadElements(const PlanDev &p, const DevTerms *terms, int64_t e0, int live, double *X, double *geom, int *orient) {
+  // the term list (its first 16 KB: the scalar terms) towards L1 while the
+  // nodes come in: small meshes are bound by the latency of such loads
+  static_assert(sizeof(DevTerms) >= 128 * kQuadThreads, "one 128-byte line per thread");
+  asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char *>(terms) + 128 * threadIdx.x));
+  for (int t = threadIdx.x; t < live * p.nn * 3; t += kQuadThreads)
+    X[t] = p.xyz[3 * (int64_t)p.enodes[e0 * p.nn + t / 3] + t % 3];
+  for (int t = threadIdx.x; t < live; t += kQuadThreads) {
+    orient[2 * t] = p.orient ? p.orient[e0 + t] : 0;
+    orient[2 * t + 1] = p.orientU ? p.orientU[e0 + t] : 0;
+  }
+  __syncthreads();
+  if (p.affine) {
+    for (int t = threadIdx.x; t < live; t += kQuadThreads) {
+      double *g = geom + t * kQuadGeom;
+      double J[9], Ji[9];
+      const double det = p.p1geom ? jacobianP1(p.dim, X + t * p.nn * 3, J) : jacobian(p.dim, p.nn, X + t * p.nn * 3, p.geoGrad, J);
+      geomMaps<HCURL>(J, det, Ji, g + 19, g + 25);
+      for (int k = 0; k < 9; ++k) {
+        g[k] = J[k];
+        g[9 + k] = Ji[k];
+      }
+      g[18] = det;
+    }
+    __syncthreads();
+  }
+}
+
+// Geometry of one (element, point) for the terms of modificator group g:
+// from the element's where the Jacobian is constant, else formed here
+struct PointGeom {
+  double J[9], Ji[9], det;
+  double K6[6], M6[6];  // det J^-1 J^-T, J^T J / det
+  double x[3];
+};
+template <bool HCURL>
+__device__ inline void quadPoint(const PlanDev &p, const DevTerms *terms, int g, int q, const double *X, const double *geom, bool needX,
+                                 PointGeom &P) {
+  P.x[0] = P.x[1] = P.x[2] = 0.0;
+  const DevJacMod &m = terms->mods[g];
+  if (needX)
+    for (int k = 0; k < p.nn; ++k) {
+      const double v = p.geoVal[q * p.nn + k];
+      P.x[0] += v * X[3 * k];
+      P.x[1] += v * X[3 * k + 1];
+      P.x[2] += v * X[3 * k + 2];
+    }
+  if (p.affine && m.kind == FG_JACMOD_NONE) {
+    for (int k = 0; k < 9; ++k) {
+      P.J[k] = geom[k];
+      P.Ji[k] = geom[9 + k];
+    }
+    P.det = geom[18];
+    for (int k = 0; k < 6; ++k) {
+      P.K6[k] = geom[19 + k];
+      if (HCURL) P.M6[k] = geom[25 + k];
+    }
+    return;
+  }
+  if (p.affine) {
+    for (int k = 0; k < 9; ++k) P.J[k] = geom[k];
+    P.det = geom[18];
+  } else {
+    P.det = jacobian(p.dim, p.nn, X, p.geoGrad + (size_t)q * p.nn * 3, P.J);
+  }
+  if (m.kind != FG_JACMOD_NONE && !applyJacMod(m, P.x, P.J, P.det)) atomicOr(p.jmErr, 1);
+  geomMaps<HCURL>(P.J, P.det, P.Ji, P.K6, P.M6);
+}
+
+// Upper-triangle entry k -> (i << 8 | j), i <= j, row-major
+__device__ inline void fillPairs(uint16_t *pairs, int n) {
   const int nEnt = n * (n + 1) / 2;
-  for (int k = threadIdx.x; k < nEnt; k += blockDim.x) {
-    // k -> (i, j), i <= j, row-major over the upper triangle
+  for (int k = threadIdx.x; k < nEnt; k += kQuadThreads) {
     int i = 0, rem = k;
     while (rem >= n - i) {
       rem -= n - i;
       ++i;
     }
-    pairI[k] = (uint8_t)i;
-    pairJ[k] = (uint8_t)(i + rem);
-  }
-  __syncthreads();
-  ElemWarpSmem &S = smem[warp];
-  const int64_t stride = (int64_t)gridDim.x * kWarpsPerBlockElem;
-  for (int64_t e = (int64_t)blockIdx.x * kWarpsPerBlockElem + warp; e < p.E; e += stride) {
-    const int o = p.orient ? p.orient[e] : 0;
-    for (int t = lane; t < p.nn * 3; t += 32) S.X[t] = p.xyz[3 * (int64_t)p.enodes[e * p.nn + t / 3] + t % 3];
-    __syncwarp();
-    double accR[MAXENT], accI[MAXENT];
-#pragma unroll
-    for (int m = 0; m < MAXENT; ++m) {
-      accR[m] = 0.0;
-      accI[m] = 0.0;
-    }
-    double2 bacc[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
-    // one pass over the points per group of terms sharing a Jacobian modificator
-    const int nG = terms->nMod > 1 ? terms->nMod : 1;
-    for (int gq = 0; gq < nG * p.nq; ++gq) {
-      const int g = gq / p.nq, q = gq - g * p.nq;
-      if (lane == 0) {
-        double xq[3];
-        pointGeometry(p, terms, g, q, S.X, S.J0, S.det0, S.J, S.det, S.Jinv, xq);
-        double2 cgg = make_double2(0.0, 0.0), cm = make_double2(0.0, 0.0), f = make_double2(0.0, 0.0);
-        const double *phq = p.bval + ((size_t)o * p.nq + q) * p.nb;  // for field-node coefficients
-        for (int t = 0; t < terms->n; ++t) {
-          const DevTerm &T = terms->t[t];
-          if (T.mod != g) continue;
-          const double2 v = evalExpr(T.coef, e, xq, phq, p.nb, q, p.nq);
-          if (T.kind == FG_TERM_GRAD_GRAD) cgg = cadd(cgg, cmul(T.factor, v));
-          else if (T.kind == FG_TERM_MASS) cm = cadd(cm, cmul(T.factor, v));
-          else if (T.kind == FG_TERM_SOURCE) f = cadd(f, v);
-        }
-        const double wd = p.w[q] * S.det;
-        S.a = make_double2(wd * cgg.x, wd * cgg.y);
-        S.b = make_double2(wd * cm.x, wd * cm.y);
-        S.s = make_double2(wd * f.x, wd * f.y);
-        if (terms->tensorTerm >= 0) {
-          double2 A[6];
-          diffusionTensor(terms, g, e, xq, cgg, A, phq, p.nb, q, p.nq);
-          for (int k = 0; k < 6; ++k) S.Aw[k] = make_double2(wd * A[k].x, wd * A[k].y);
-        }
-      }
-      __syncwarp();
-      const size_t base = ((size_t)o * p.nq + q) * p.nb;
-      const bool tensor = terms->tensorTerm >= 0;
-      for (int i = lane; i < n; i += 32) {
-        const double g0 = p.bgrad[3 * (base + i)], g1 = p.bgrad[3 * (base + i) + 1], g2 = p.bgrad[3 * (base + i) + 2];
-        const double ph = p.bval[base + i];
-        double G[3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-          G[r] = S.Jinv[r] * g0 + S.Jinv[3 + r] * g1 + S.Jinv[6 + r] * g2;
-          S.G[r][i] = G[r];
-        }
-        if (tensor) {
-          // (w det A) G with A symmetric: rows (00 01 02), (01 11 12), (02 12 22)
-          const int row[3][3] = {{0, 3, 4}, {3, 1, 5}, {4, 5, 2}};
-#pragma unroll
-          for (int r = 0; r < 3; ++r) {
-            S.Gs[0][r][i] = S.Aw[row[r][0]].x * G[0] + S.Aw[row[r][1]].x * G[1] + S.Aw[row[r][2]].x * G[2];
-            if (CPLX) S.Gs[1][r][i] = S.Aw[row[r][0]].y * G[0] + S.Aw[row[r][1]].y * G[1] + S.Aw[row[r][2]].y * G[2];
-          }
-        } else {
-#pragma unroll
-          for (int r = 0; r < 3; ++r) {
-            S.Gs[0][r][i] = S.a.x * G[r];
-            if (CPLX) S.Gs[1][r][i] = S.a.y * G[r];
-          }
-        }
-        S.phi[i] = ph;
-        S.phis[0][i] = S.b.x * ph;
-        if (CPLX) S.phis[1][i] = S.b.y * ph;
-        // b_e[i] += w det conj(phi_i) f
-        const int slot = i >> 5;
-        bacc[slot].x += S.s.x * ph;
-        bacc[slot].y += S.s.y * ph;
-      }
-      __syncwarp();
-#pragma unroll
-      for (int m = 0; m < MAXENT; ++m) {
-        const int k = lane + 32 * m;
-        if (k < nEnt) {
-          const int i = pairI[k], j = pairJ[k];
-          accR[m] += S.G[0][i] * S.Gs[0][0][j] + S.G[1][i] * S.Gs[0][1][j] + S.G[2][i] * S.Gs[0][2][j] + S.phi[i] * S.phis[0][j];
-          if (CPLX)
-            accI[m] += S.G[0][i] * S.Gs[1][0][j] + S.G[1][i] * S.Gs[1][1][j] + S.G[2][i] * S.Gs[1][2][j] + S.phi[i] * S.phis[1][j];
-        }
-      }
-      __syncwarp();
-    }
-    // Ke layout [E][ncomp][n][n], row = local test index, column = local unknown index
-    const int ncomp = CPLX ? 2 : 1;
-    double *K = ke + (size_t)e * ncomp * n * n;
-#pragma unroll
-    for (int m = 0; m < MAXENT; ++m) {
-      const int k = lane + 32 * m;
-      if (k < nEnt) {
-        const int i = pairI[k], j = pairJ[k];
-        K[i * n + j] = accR[m];
-        K[j * n + i] = accR[m];
-        if (CPLX) {
-          K[n * n + i * n + j] = accI[m];
-          K[n * n + j * n + i] = accI[m];
-        }
-      }
-    }
-    if (be)
-      for (int i = lane; i < n; i += 32) be[(size_t)e * n + i] = bacc[i >> 5];
-    __syncwarp();
+    pairs[k] = (uint16_t)(i << 8 | (i + rem));
   }
 }
 
-// Scalar H1 field with terms whose element matrix is not symmetric: a general
-// TensorFunction D in integral(c D grad(dof u), grad(tf u)) and the advection
-// integral(c b . grad(dof u), tf(u)) with a VectorFunction b, beside the
-// symmetric terms. One warp per element; at each point lane 0 forms
-//   M = w det (c_gg I + A_sym + c_full D)   (the unknown's gradient map),
-//   v = w det c_adv b,  m = w det c_mass,
-// the lanes map the unknown's gradients (U_j = M G_j, a_j = v . G_j + m phi_j)
-// and each lane owns entries (i, j) of the full n x n matrix:
-//   Ke[i][j] += G_i . U_j + phi_i a_j
-// (BilinearTerm::evaluate's Hermitian product with real test functions,
-// src/term/BilinearTerm.cpp:314-326: the test side is conj(field), the
-// unknown side carries the coefficient).
-struct FullWarpSmem {
-  double X[kMaxNodes * 3];
-  double J0[9], J[9], Jinv[9];
-  double det0, det;
-  double2 M[9], v[3], m, s;
-  double2 vb[3], sg[3];      // w det c b (vector times dof, tested against gradients), w det f (vector source)
-  double G[3][kMaxDofs];     // test functions: physical gradients
-  double phi[kMaxDofs];      // and values
-  double U[2][3][kMaxDofs];  // unknown functions: M G_j (real, imaginary parts)
-  double a[2][kMaxDofs];     // and v . G_j + m phi_j
-};
+__device__ __forceinline__ void sym3(const double *S, double g0, double g1, double g2, double *h) {
+  h[0] = S[0] * g0 + S[3] * g1 + S[4] * g2;
+  h[1] = S[3] * g0 + S[1] * g1 + S[5] * g2;
+  h[2] = S[4] * g0 + S[5] * g1 + S[2] * g2;
+}
 
-// Full (non-symmetric) element matrices: Ke[i][j] = sum_q G_i . (M G_j) +
-// phi_i (v . G_j + m phi_j) with the test function i (rows) and the unknown
-// function j (columns), M the scaled diffusion tensor (isotropic, symmetric
-// and general parts), v the advection vector, m the mass coefficient. A
-// two-field plan takes the test functions from the test field's tables and
-// the unknown functions from the unknown field's (BilinearTerm with
-// _field[0] != _field[1], src/term/BilinearTerm.cpp:304-343): Ke is n x nc.
-template <int MAXENT, bool CPLX>
-__global__ void __launch_bounds__(32 * kWarpsPerBlockElem)
-    k_element_full_fp64(const PlanDev p, const DevTerms *__restrict__ terms, double *__restrict__ ke, double2 *__restrict__ be) {
-  __shared__ FullWarpSmem smem[kWarpsPerBlockElem];
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int n = p.nb, nU = p.nbU;
-  const int nEnt = n * nU;
-  FullWarpSmem &S = smem[warp];
-  const int64_t stride = (int64_t)gridDim.x * kWarpsPerBlockElem;
-  for (int64_t e = (int64_t)blockIdx.x * kWarpsPerBlockElem + warp; e < p.E; e += stride) {
-    const int o = p.orient ? p.orient[e] : 0;
-    const int oU = p.orientU ? p.orientU[e] : 0;
-    for (int t = lane; t < p.nn * 3; t += 32) S.X[t] = p.xyz[3 * (int64_t)p.enodes[e * p.nn + t / 3] + t % 3];
-    __syncwarp();
-    double accR[MAXENT], accI[MAXENT];
+// The element matrices and vectors of blocks of NE elements.
+//   kQuadSym:   scalar H1, symmetric: D = (w det c J^-1 A J^-T, w det c_m)
+//   kQuadHcurl: HCurl values P = J^-T v and curls C = J c / det
+//               (FieldEvaluator<Form1/Form2>, src/term/evaluator/FieldEvaluator.h:59-105):
+//               D = (w J^T A J / det, w det J^-1 B J^-T)
+//   kQuadFull:  scalar H1, terms whose element matrix is not symmetric (a
+//               general TensorFunction, VectorFunction terms) or a two-field
+//               plan (BilinearTerm with _field[0] != _field[1],
+//               src/term/BilinearTerm.cpp:304-343; test functions from the
+//               test tables, unknown functions from the unknown field's):
+//               Ke[i][j] = G_i . (M G_j + b' phi_j) + phi_i (v . G_j + m phi_j),
+//               D = w det [J^-1 M J^-T, J^-1 b'; (J^-1 v)^T, m].
+// CPLX: complex D. SPLIT: complex coefficients that are constant on each
+// element: the real integrals of the two term kinds are summed apart and
+// combined at the end, half the FP64 work of complex D. MASKED: some table
+// components vanish or have no term (a.comps); otherwise all contribute.
+// Bound by the FP64 pipe: 82,944 tetrahedra of order 3 (24 points, real,
+// constant on each element) take 3.98 ms, of which the entries' products
+// alone are 2.7 ms at one warp instruction per 64 cycles and scheduler; a warp
+// per element, with the geometry and coefficients on its first lane, took
+// 9.93 ms. Order 2 with complex coefficients that vary inside the elements
+// (55,566 tetrahedra): 1.47 ms, before 7.93. HCurl of order 1 (34,992
+// tetrahedra): 1.64 ms, before 5.32.
+template <int KIND, bool CPLX, bool SPLIT, bool MASKED, int MAXE>
+__global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 3)
+    k_element_fp64(const PlanDev p, const DevTerms *__restrict__ terms, const QuadArgs a, double *__restrict__ ke, double2 *__restrict__ be) {
+  constexpr int R = quadComps(KIND), ND = quadD(KIND);
+  constexpr int NC = CPLX ? 2 : 1;           // parts of D and H
+  constexpr int NA = (CPLX || SPLIT) ? 2 : 1;  // sums per entry
+  extern __shared__ __align__(16) double qsm[];
+  const int n = p.nb, nU = p.nbU, tid = threadIdx.x;
+  const QuadLayout L = quadLayout(a.NE, a.QD, a.QC, p.nn, n, nU, ND * NC, R * NC, be != nullptr, KIND == kQuadFull ? 0 : a.nEnt);
+  double *X = qsm + L.X, *geom = qsm + L.geom, *D = qsm + L.D, *src = qsm + L.src, *H = qsm + L.H;
+  double2 *bs = reinterpret_cast<double2 *>(qsm + L.be);
+  double *coef = qsm + L.coef;
+  uint16_t *pairs = reinterpret_cast<uint16_t *>(qsm + L.pairs);
+  int *orient = reinterpret_cast<int *>(qsm + L.orient);
+  const int64_t e0 = (int64_t)blockIdx.x * a.NE;
+  const int live = (int)min((int64_t)a.NE, p.E - e0);
+  if (KIND != kQuadFull && ke) fillPairs(pairs, n);
+  quadElements<KIND == kQuadHcurl>(p, terms, e0, live, X, geom, orient);
+  if (be)
+    for (int t = tid; t < live * n; t += kQuadThreads) bs[t] = make_double2(0.0, 0.0);
+
+  // this thread's entries: test row in the tables, unknown column in H
+  double acc[NA][MAXE];
+  int offT[MAXE], offH[MAXE], mine = 0;
 #pragma unroll
-    for (int k = 0; k < MAXENT; ++k) {
-      accR[k] = 0.0;
-      accI[k] = 0.0;
+  for (int m = 0; m < MAXE; ++m) {
+#pragma unroll
+    for (int c = 0; c < NA; ++c) acc[c][m] = 0.0;
+    offT[m] = offH[m] = 0;
+    const int k = tid + kQuadThreads * m;
+    if (ke && k < live * a.nEnt) {
+      const int el = k / a.nEnt, r = k - el * a.nEnt;
+      const int i = KIND == kQuadFull ? r / nU : pairs[r] >> 8, j = KIND == kQuadFull ? r % nU : pairs[r] & 255;
+      offT[m] = orient[2 * el] * p.nq * n + i;
+      offH[m] = el * a.QC * (R * NC) * nU + j;
+      mine = m + 1;
     }
-    double2 bacc[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
-    const int nG = terms->nMod > 1 ? terms->nMod : 1;
-    for (int gq = 0; gq < nG * p.nq; ++gq) {
-      const int g = gq / p.nq, q = gq - g * p.nq;
-      if (lane == 0) {
-        double xq[3];
-        pointGeometry(p, terms, g, q, S.X, S.J0, S.det0, S.J, S.det, S.Jinv, xq);
-        const double *phq = p.bval + ((size_t)o * p.nq + q) * p.nb;
-        double2 cgg = make_double2(0.0, 0.0), cm = make_double2(0.0, 0.0), f = make_double2(0.0, 0.0);
-        for (int t = 0; t < terms->n; ++t) {
-          const DevTerm &T = terms->t[t];
-          if (T.mod != g) continue;
-          if (T.kind == FG_TERM_GRAD_GRAD) cgg = cadd(cgg, cmul(T.factor, evalExpr(T.coef, e, xq, phq, p.nb, q, p.nq)));
-          else if (T.kind == FG_TERM_MASS) cm = cadd(cm, cmul(T.factor, evalExpr(T.coef, e, xq, phq, p.nb, q, p.nq)));
-          else if (T.kind == FG_TERM_SOURCE) f = cadd(f, evalExpr(T.coef, e, xq, phq, p.nb, q, p.nq));
-        }
-        const double wd = p.w[q] * S.det;
-        double2 A6[6];
-        diffusionTensor(terms, g, e, xq, cgg, A6, phq, p.nb, q, p.nq);  // c_gg I (+ the symmetric tensor term)
-        const int sym[3][3] = {{0, 3, 4}, {3, 1, 5}, {4, 5, 2}};
-        double2 M[9];
-        for (int r = 0; r < 3; ++r)
-          for (int c = 0; c < 3; ++c) M[3 * r + c] = A6[sym[r][c]];
-        if (terms->tensorFullTerm >= 0 && terms->t[terms->tensorFullTerm].mod == g) {
-          const DevTerm &T = terms->t[terms->tensorFullTerm];
-          const double2 fc = cmul(T.factor, evalExpr(T.coef, e, xq, phq, p.nb, q, p.nq));
-          for (int k = 0; k < 9; ++k) M[k] = cadd(M[k], cmul(fc, evalExpr(terms->tensorFull[k], e, xq, phq, p.nb, q, p.nq)));
-        }
-        double2 v[3] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
-        if (terms->advectTerm >= 0 && terms->t[terms->advectTerm].mod == g) {
-          const DevTerm &T = terms->t[terms->advectTerm];
-          const double2 fc = cmul(T.factor, evalExpr(T.coef, e, xq, phq, p.nb, q, p.nq));
-          for (int k = 0; k < 3; ++k) v[k] = cmul(fc, evalExpr(terms->advect[k], e, xq, phq, p.nb, q, p.nq));
-        }
-        double2 vb[3] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
-        if (terms->vecGradTerm >= 0 && terms->t[terms->vecGradTerm].mod == g) {
-          const DevTerm &T = terms->t[terms->vecGradTerm];
-          const double2 fc = cmul(T.factor, evalExpr(T.coef, e, xq, phq, p.nb, q, p.nq));
-          for (int k = 0; k < 3; ++k) vb[k] = cmul(fc, evalExpr(terms->vecGrad[k], e, xq, phq, p.nb, q, p.nq));
-        }
-        double2 sg[3] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
-        if (terms->srcGradTerm >= 0 && terms->t[terms->srcGradTerm].mod == g) {
-          const DevTerm &T = terms->t[terms->srcGradTerm];
-          const double2 fc = evalExpr(T.coef, e, xq, phq, p.nb, q, p.nq);
-          for (int k = 0; k < 3; ++k) sg[k] = cmul(fc, evalExpr(terms->srcGrad[k], e, xq, phq, p.nb, q, p.nq));
-        }
-        for (int k = 0; k < 9; ++k) S.M[k] = make_double2(wd * M[k].x, wd * M[k].y);
-        for (int k = 0; k < 3; ++k) S.v[k] = make_double2(wd * v[k].x, wd * v[k].y);
-        for (int k = 0; k < 3; ++k) S.vb[k] = make_double2(wd * vb[k].x, wd * vb[k].y);
-        for (int k = 0; k < 3; ++k) S.sg[k] = make_double2(wd * sg[k].x, wd * sg[k].y);
-        S.m = make_double2(wd * cm.x, wd * cm.y);
-        S.s = make_double2(wd * f.x, wd * f.y);
-      }
-      __syncwarp();
-      const size_t base = ((size_t)o * p.nq + q) * p.nb;
-      for (int i = lane; i < n; i += 32) {
-        const double g0 = p.bgrad[3 * (base + i)], g1 = p.bgrad[3 * (base + i) + 1], g2 = p.bgrad[3 * (base + i) + 2];
-        const double ph = p.bval[base + i];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) S.G[r][i] = S.Jinv[r] * g0 + S.Jinv[3 + r] * g1 + S.Jinv[6 + r] * g2;
-        S.phi[i] = ph;
-        const int slot = i >> 5;
-        bacc[slot].x += S.s.x * ph + S.sg[0].x * S.G[0][i] + S.sg[1].x * S.G[1][i] + S.sg[2].x * S.G[2][i];
-        bacc[slot].y += S.s.y * ph + S.sg[0].y * S.G[0][i] + S.sg[1].y * S.G[1][i] + S.sg[2].y * S.G[2][i];
-      }
-      const size_t baseU = ((size_t)oU * p.nq + q) * nU;
-      for (int j = lane; j < nU; j += 32) {
-        const double g0 = p.bgradU[3 * (baseU + j)], g1 = p.bgradU[3 * (baseU + j) + 1], g2 = p.bgradU[3 * (baseU + j) + 2];
-        const double ph = p.bvalU[baseU + j];
-        double G[3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) G[r] = S.Jinv[r] * g0 + S.Jinv[3 + r] * g1 + S.Jinv[6 + r] * g2;
-        // U_j = M G_j + vb phi_j: the unknown's vector field, tested against G_i
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-          S.U[0][r][j] = S.M[3 * r].x * G[0] + S.M[3 * r + 1].x * G[1] + S.M[3 * r + 2].x * G[2] + S.vb[r].x * ph;
-          if (CPLX) S.U[1][r][j] = S.M[3 * r].y * G[0] + S.M[3 * r + 1].y * G[1] + S.M[3 * r + 2].y * G[2] + S.vb[r].y * ph;
-        }
-        S.a[0][j] = S.v[0].x * G[0] + S.v[1].x * G[1] + S.v[2].x * G[2] + S.m.x * ph;
-        if (CPLX) S.a[1][j] = S.v[0].y * G[0] + S.v[1].y * G[1] + S.v[2].y * G[2] + S.m.y * ph;
-      }
-      __syncwarp();
-#pragma unroll
-      for (int m = 0; m < MAXENT; ++m) {
-        const int k = lane + 32 * m;
-        if (k < nEnt) {
-          const int i = k / nU, j = k - i * nU;
-          accR[m] += S.G[0][i] * S.U[0][0][j] + S.G[1][i] * S.U[0][1][j] + S.G[2][i] * S.U[0][2][j] + S.phi[i] * S.a[0][j];
-          if (CPLX)
-            accI[m] += S.G[0][i] * S.U[1][0][j] + S.G[1][i] * S.U[1][1][j] + S.G[2][i] * S.U[1][2][j] + S.phi[i] * S.a[1][j];
-        }
-      }
-      __syncwarp();
-    }
-    const int ncomp = CPLX ? 2 : 1;
-    double *K = ke + (size_t)e * ncomp * nEnt;
-#pragma unroll
-    for (int m = 0; m < MAXENT; ++m) {
-      const int k = lane + 32 * m;
-      if (k < nEnt) {
-        K[k] = accR[m];
-        if (CPLX) K[nEnt + k] = accI[m];
-      }
-    }
-    if (be)
-      for (int i = lane; i < n; i += 32) be[(size_t)e * n + i] = bacc[i >> 5];
-    __syncwarp();
   }
+  const bool tensor = terms->tensorTerm >= 0 || terms->tensorMassTerm >= 0;
+  const int nG = terms->nMod > 1 ? terms->nMod : 1;
+  for (int g = 0; g < nG; ++g) {
+    if (a.uniform && ke)
+      for (int t = tid; t < live; t += kQuadThreads) {
+        double2 c[3];
+        const CoefPoint cp = {e0 + t, X, nullptr, 0, 0, p.nq};
+        scalarCoefs(terms, g, cp, c);
+        for (int k = 0; k < 2; ++k) {
+          coef[6 * t + 2 * k] = c[k].x;
+          coef[6 * t + 2 * k + 1] = c[k].y;
+        }
+      }
+    __syncthreads();
+    for (int d0 = 0; d0 < p.nq; d0 += a.QD) {
+      const int dn = min(a.QD, p.nq - d0);
+      // D (and the source) of every (element, point)
+      for (int t = tid; t < live * dn; t += kQuadThreads) {
+        const int el = t / dn, qd = t - el * dn, q = d0 + qd;
+        PointGeom P;
+        quadPoint<KIND == kQuadHcurl>(p, terms, g, q, X + el * p.nn * 3, geom + el * kQuadGeom, a.needX != 0, P);
+        const double w = p.w[q];
+        CoefPoint cp = {e0 + el, P.x, nullptr, 0, q, p.nq};
+        if (KIND != kQuadHcurl) {  // field-node coefficients read the point's row of the basis table
+          cp.phi = p.bval + ((size_t)orient[2 * el] * p.nq + q) * n;
+          cp.nb = n;
+        }
+        double2 c[3];
+        if (SPLIT || !ke) {
+          c[0] = c[1] = make_double2(1.0, 0.0);
+        } else if (a.uniform) {
+          c[0] = make_double2(coef[6 * el], coef[6 * el + 1]);
+          c[1] = make_double2(coef[6 * el + 2], coef[6 * el + 3]);
+        } else {
+          scalarCoefs(terms, g, cp, c);
+        }
+        double *d = D + (size_t)(el * a.QD + qd) * (ND * NC);
+        if (!ke) {
+          // the right-hand side alone: no D
+        } else if (KIND != kQuadFull) {
+          double2 A[6], B[6];
+          if (tensor) {
+            tensorAt(terms, terms->tensorTerm, terms->tensor, g, cp, c[0], A);
+            if (KIND == kQuadHcurl) tensorAt(terms, terms->tensorMassTerm, terms->tensorMass, g, cp, c[1], B);
+          }
+#pragma unroll
+          for (int part = 0; part < NC; ++part) {
+            const double cg = w * (part ? c[0].y : c[0].x), cm = w * (part ? c[1].y : c[1].x);
+            double *dp = d + part * ND;
+            if (tensor) {
+              double F[6];
+              if (KIND == kQuadSym) {
+                congruence6(P.Ji, A, part, F);
+                for (int k = 0; k < 6; ++k) dp[k] = w * P.det * F[k];
+                dp[6] = cm * P.det;
+              } else {
+                congruence6(P.J, A, part, F);
+                for (int k = 0; k < 6; ++k) dp[k] = w * F[k] / P.det;
+                congruence6(P.Ji, B, part, F);
+                for (int k = 0; k < 6; ++k) dp[6 + k] = w * P.det * F[k];
+              }
+            } else if (KIND == kQuadSym) {
+              for (int k = 0; k < 6; ++k) dp[k] = cg * P.K6[k];
+              dp[6] = cm * P.det;
+            } else {
+              for (int k = 0; k < 6; ++k) {
+                dp[k] = cg * P.M6[k];
+                dp[6 + k] = cm * P.K6[k];
+              }
+            }
+          }
+        } else {
+          double2 A6[6], M[9], v[3], vb[3];
+          tensorAt(terms, terms->tensorTerm, terms->tensor, g, cp, c[0], A6);  // c_gg I (+ the symmetric tensor term)
+          const int sym[9] = {0, 3, 4, 3, 1, 5, 4, 5, 2};
+          for (int k = 0; k < 9; ++k) M[k] = A6[sym[k]];
+          if (terms->tensorFullTerm >= 0 && terms->t[terms->tensorFullTerm].mod == g) {
+            const DevTerm &T = terms->t[terms->tensorFullTerm];
+            const double2 fc = cmul(T.factor, evalAt(T.coef, cp));
+            for (int k = 0; k < 9; ++k) M[k] = cadd(M[k], cmul(fc, evalAt(terms->tensorFull[k], cp)));
+          }
+          for (int k = 0; k < 3; ++k) v[k] = vb[k] = make_double2(0.0, 0.0);
+          if (terms->advectTerm >= 0 && terms->t[terms->advectTerm].mod == g) {
+            const DevTerm &T = terms->t[terms->advectTerm];
+            const double2 fc = cmul(T.factor, evalAt(T.coef, cp));
+            for (int k = 0; k < 3; ++k) v[k] = cmul(fc, evalAt(terms->advect[k], cp));
+          }
+          if (terms->vecGradTerm >= 0 && terms->t[terms->vecGradTerm].mod == g) {
+            const DevTerm &T = terms->t[terms->vecGradTerm];
+            const double2 fc = cmul(T.factor, evalAt(T.coef, cp));
+            for (int k = 0; k < 3; ++k) vb[k] = cmul(fc, evalAt(terms->vecGrad[k], cp));
+          }
+          const double wd = w * P.det;
+#pragma unroll
+          for (int part = 0; part < NC; ++part) {
+            double *dp = d + part * ND;
+            auto re = [&](double2 z) { return part ? z.y : z.x; };
+            for (int r = 0; r < 3; ++r) {
+              double QM[3];  // row r of J^-1 M
+              for (int s = 0; s < 3; ++s)
+                QM[s] = P.Ji[3 * r] * re(M[s]) + P.Ji[3 * r + 1] * re(M[3 + s]) + P.Ji[3 * r + 2] * re(M[6 + s]);
+              for (int s = 0; s < 3; ++s)
+                dp[4 * r + s] = wd * (QM[0] * P.Ji[3 * s] + QM[1] * P.Ji[3 * s + 1] + QM[2] * P.Ji[3 * s + 2]);
+              dp[4 * r + 3] = wd * (P.Ji[3 * r] * re(vb[0]) + P.Ji[3 * r + 1] * re(vb[1]) + P.Ji[3 * r + 2] * re(vb[2]));
+              dp[12 + r] = wd * (P.Ji[3 * r] * re(v[0]) + P.Ji[3 * r + 1] * re(v[1]) + P.Ji[3 * r + 2] * re(v[2]));
+            }
+            dp[15] = wd * re(c[1]);
+          }
+        }
+        if (be) {
+          double2 f = make_double2(0.0, 0.0);
+          for (int k = 0; k < terms->n; ++k)
+            if (terms->t[k].kind == FG_TERM_SOURCE && terms->t[k].mod == g) f = cadd(f, evalAt(terms->t[k].coef, cp));
+          double *s = src + (size_t)(el * a.QD + qd) * 8;
+          const double wd = w * P.det;
+          s[0] = wd * f.x;
+          s[1] = wd * f.y;
+          if (KIND == kQuadFull) {
+            double2 sg[3] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+            if (terms->srcGradTerm >= 0 && terms->t[terms->srcGradTerm].mod == g) {
+              const double2 fc = evalAt(terms->t[terms->srcGradTerm].coef, cp);
+              for (int k = 0; k < 3; ++k) sg[k] = cmul(fc, evalAt(terms->srcGrad[k], cp));
+            }
+            for (int r = 0; r < 3; ++r) {
+              s[2 + r] = wd * (P.Ji[3 * r] * sg[0].x + P.Ji[3 * r + 1] * sg[1].x + P.Ji[3 * r + 2] * sg[2].x);
+              s[5 + r] = wd * (P.Ji[3 * r] * sg[0].y + P.Ji[3 * r + 1] * sg[1].y + P.Ji[3 * r + 2] * sg[2].y);
+            }
+          }
+        }
+      }
+      __syncthreads();
+      // b_e[i] += w det conj(phi_i) f (+ the vector source against gradients)
+      if (be)
+        for (int t = tid; t < live * n; t += kQuadThreads) {
+          const int el = t / n, i = t - el * n;
+          double2 b = bs[t];
+          for (int qd = 0; qd < dn; ++qd) {
+            const size_t row = ((size_t)orient[2 * el] * p.nq + d0 + qd) * n + i;
+            const double *s = src + (size_t)(el * a.QD + qd) * 8;
+            const double ph = p.bval[row];
+            b.x += s[0] * ph;
+            b.y += s[1] * ph;
+            if (KIND == kQuadFull && terms->srcGradTerm >= 0) {
+              const double *gr = p.bgrad + 3 * row;
+              b.x += s[2] * gr[0] + s[3] * gr[1] + s[4] * gr[2];
+              b.y += s[5] * gr[0] + s[6] * gr[1] + s[7] * gr[2];
+            }
+          }
+          bs[t] = b;
+        }
+      if (!ke) __syncthreads();  // the sources are read before the next ones are written
+      for (int q0 = d0; ke && q0 < d0 + dn; q0 += a.QC) {
+        const int qn = min(a.QC, d0 + dn - q0);
+        if (q0 > d0) __syncthreads();  // H has been read
+        // H = D t_j of every (element, point, unknown function)
+        for (int t = tid; t < live * qn * nU; t += kQuadThreads) {
+          const int ep = t / nU, j = t - ep * nU, el = ep / qn, qc = ep - el * qn, q = q0 + qc;
+          const size_t row = ((size_t)orient[2 * el + 1] * p.nq + q) * nU + j;
+          const double *d = D + (size_t)(el * a.QD + q - d0) * (ND * NC);
+          double *h = H + (size_t)(el * a.QC + qc) * (R * NC) * nU + j;
+          const double *gr = p.bgradU + 3 * row;
+          const double g0 = gr[0], g1 = gr[1], g2 = gr[2];
+          double v[3] = {0.0, 0.0, 0.0};
+          if (KIND == kQuadHcurl) {
+            v[0] = p.bvalU[3 * row];
+            v[1] = p.bvalU[3 * row + 1];
+            v[2] = p.bvalU[3 * row + 2];
+          } else {
+            v[0] = p.bvalU[row];
+          }
+#pragma unroll
+          for (int part = 0; part < NC; ++part) {
+            const double *dp = d + part * ND;
+            double o[6];
+            if (KIND == kQuadFull) {
+#pragma unroll
+              for (int r = 0; r < 4; ++r) o[r] = dp[4 * r] * g0 + dp[4 * r + 1] * g1 + dp[4 * r + 2] * g2 + dp[4 * r + 3] * v[0];
+            } else {
+              if (!MASKED || (a.comps & 7)) sym3(dp, g0, g1, g2, o);
+              if (KIND == kQuadSym) o[3] = dp[6] * v[0];
+              else if (!MASKED || (a.comps & 56)) sym3(dp + 6, v[0], v[1], v[2], o + 3);
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+              if (!MASKED || (a.comps >> r & 1)) h[(part * R + r) * nU] = o[r];
+          }
+        }
+        __syncthreads();
+        // Ke[i][j] += t_i . H_j. The next D may be written meanwhile: it is
+        // read after the barrier that follows.
+        for (int qc = 0; qc < qn; ++qc) {
+          const double *bg = p.bgrad + 3 * (size_t)(q0 + qc) * n;
+          const double *bv = p.bval + (size_t)(KIND == kQuadHcurl ? 3 : 1) * (q0 + qc) * n;
+          const double *Hq = H + (size_t)qc * (R * NC) * nU;
+#pragma unroll
+          for (int m = 0; m < MAXE; ++m)
+            if (m < mine) {
+              const double *gi = bg + 3 * offT[m], *vi = bv + (KIND == kQuadHcurl ? 3 : 1) * offT[m], *h = Hq + offH[m];
+#pragma unroll
+              for (int r = 0; r < R; ++r) {
+                if (MASKED && !(a.comps >> r & 1)) continue;
+                const double t = r < 3 ? gi[r] : vi[r - 3];
+                if (SPLIT) {
+                  acc[r < 3 ? 0 : NA - 1][m] = fma(t, h[r * nU], acc[r < 3 ? 0 : NA - 1][m]);
+                } else {
+                  acc[0][m] = fma(t, h[r * nU], acc[0][m]);
+                  if (CPLX) acc[NA - 1][m] = fma(t, h[(R + r) * nU], acc[NA - 1][m]);
+                }
+              }
+            }
+        }
+      }
+    }
+  }
+  // Ke layout [E][ncomp][n][nc], row = local test index, column = local unknown index
+  const int nn2 = n * nU;
+#pragma unroll
+  for (int m = 0; m < MAXE; ++m)
+    if (m < mine) {
+      const int k = tid + kQuadThreads * m, el = k / a.nEnt, r = k - el * a.nEnt;
+      double re = acc[0][m], im = acc[NA - 1][m];
+      if (SPLIT) {
+        const double *c = coef + 6 * el;
+        const double sg = re, sm = im;
+        re = c[0] * sg + c[2] * sm;
+        im = c[1] * sg + c[3] * sm;
+      }
+      double *K = ke + (size_t)(e0 + el) * NA * nn2;
+      if (KIND == kQuadFull) {
+        K[r] = re;
+        if (NA == 2) K[nn2 + r] = im;
+      } else {
+        const int i = pairs[r] >> 8, j = pairs[r] & 255;
+        K[i * n + j] = re;
+        K[j * n + i] = re;
+        if (NA == 2) {
+          K[nn2 + i * n + j] = im;
+          K[nn2 + j * n + i] = im;
+        }
+      }
+    }
+  if (be)
+    for (int t = tid; t < live * n; t += kQuadThreads) be[(size_t)e0 * n + t] = bs[t];
 }
 
 // Compound (3-component) field with the isotropic Tensor4 term
@@ -335,298 +552,338 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlockElem)
 // with C_ijkl = lambda d_ij d_kl + mu (d_ik d_jl + d_il d_jk) gives, for the
 // test DOF (i, a) and the unknown DOF (j, b) (local index = basis * 3 + component),
 //   Ke = w det [ lambda dj_b di_a + mu d_ab (gi . gj) + mu dj_a di_b ] + w det c_m d_ab phi_i phi_j
-// with g = J^-T grad phi. Lanes own scalar basis pairs (i <= j) and their 3x3
-// blocks; the element matrix is symmetric.
-struct ElasticWarpSmem {
-  double X[kMaxNodes * 3];
-  double J0[9], J[9], Jinv[9];
-  double det0, det;
-  double2 lam, mu, cm, s;  // scaled by w det
-  double G[3][kMaxDofs / 3 + 1];
-  double phi[kMaxDofs / 3 + 1];
-};
-
-template <int MAXP, bool CPLX>
-__global__ void __launch_bounds__(32 * kWarpsPerBlockElem)
-    k_element_elastic_fp64(const PlanDev p, const DevTerms *__restrict__ terms, double *__restrict__ ke, double2 *__restrict__ be) {
-  __shared__ ElasticWarpSmem smem[kWarpsPerBlockElem];
-  __shared__ uint8_t pairI[256], pairJ[256];
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int ns = p.nb, n = 3 * ns;
-  const int nPairs = ns * (ns + 1) / 2;
-  for (int k = threadIdx.x; k < nPairs; k += blockDim.x) {
-    int i = 0, rem = k;
-    while (rem >= ns - i) {
-      rem -= ns - i;
-      ++i;
+// with g = J^-T grad phi. Items are scalar basis pairs (i <= j) with their
+// 3x3 blocks; the element matrix is symmetric. With coefficients constant on
+// each element (UNIFORM) only T_ab = sum w det gi_a gj_b and the mass are
+// summed, 10 products per pair and point, and
+//   Ke_ab = lambda T_ab + mu T_ba + d_ab (mu tr T + c_m mass)
+// is formed once; otherwise the lambda- and mu-weighted sums are kept apart
+// (19 products, twice for complex coefficients). a.comps: 1 the elastic
+// term, 2 the mass term. Bound by the FP64 pipe: order 2, 20,250 tetrahedra,
+// Lame coefficients per element: 0.468 ms (with the weighted terms formed for
+// every entry, a warp per element, it took 3.15 ms).
+template <bool UNIFORM, bool CPLX, int MAXP>
+__global__ void __launch_bounds__(kQuadThreads, UNIFORM ? 3 : 2)
+    k_element_elastic_fp64(const PlanDev p, const DevTerms *__restrict__ terms, const QuadArgs a, double *__restrict__ ke,
+                           double2 *__restrict__ be) {
+  constexpr int NC = (!UNIFORM && CPLX) ? 2 : 1;
+  constexpr int ND = 10 + (UNIFORM ? 0 : 3 * NC);  // J^-1, w det; lambda, mu, c_m times w det
+  constexpr int NH = UNIFORM ? 7 : 3 + 7 * NC;     // g, then w det g and w det phi, or per part lambda g, mu g, c_m phi
+  constexpr int NS = UNIFORM ? 10 : 19 * NC;       // sums per pair
+  extern __shared__ __align__(16) double qsm[];
+  const int ns = p.nb, n = 3 * ns, tid = threadIdx.x;
+  const QuadLayout L = quadLayout(a.NE, a.QD, a.QC, p.nn, 0, ns, ND, NH, false, a.nEnt);
+  double *X = qsm + L.X, *geom = qsm + L.geom, *D = qsm + L.D, *H = qsm + L.H, *coef = qsm + L.coef;
+  uint16_t *pairs = reinterpret_cast<uint16_t *>(qsm + L.pairs);
+  int *orient = reinterpret_cast<int *>(qsm + L.orient);
+  const int64_t e0 = (int64_t)blockIdx.x * a.NE;
+  const int live = (int)min((int64_t)a.NE, p.E - e0);
+  fillPairs(pairs, ns);
+  quadElements<false>(p, terms, e0, live, X, geom, orient);
+  double acc[MAXP][NS];
+  int offI[MAXP], offJ[MAXP], rowI[MAXP], mine = 0;
+#pragma unroll
+  for (int m = 0; m < MAXP; ++m) {
+#pragma unroll
+    for (int c = 0; c < NS; ++c) acc[m][c] = 0.0;
+    offI[m] = offJ[m] = rowI[m] = 0;
+    const int k = tid + kQuadThreads * m;
+    if (k < live * a.nEnt) {
+      const int el = k / a.nEnt, pr = pairs[k - el * a.nEnt];
+      offI[m] = el * a.QC * NH * ns + (pr >> 8);
+      offJ[m] = el * a.QC * NH * ns + (pr & 255);
+      rowI[m] = orient[2 * el] * p.nq * ns + (pr >> 8);
+      mine = m + 1;
     }
-    pairI[k] = (uint8_t)i;
-    pairJ[k] = (uint8_t)(i + rem);
   }
-  __syncthreads();
-  ElasticWarpSmem &S = smem[warp];
-  const int64_t stride = (int64_t)gridDim.x * kWarpsPerBlockElem;
-  for (int64_t e = (int64_t)blockIdx.x * kWarpsPerBlockElem + warp; e < p.E; e += stride) {
-    const int o = p.orient ? p.orient[e] : 0;
-    for (int t = lane; t < p.nn * 3; t += 32) S.X[t] = p.xyz[3 * (int64_t)p.enodes[e * p.nn + t / 3] + t % 3];
-    __syncwarp();
-    double accR[MAXP][9], accI[MAXP][9];
-#pragma unroll
-    for (int m = 0; m < MAXP; ++m)
-#pragma unroll
-      for (int b = 0; b < 9; ++b) {
-        accR[m][b] = 0.0;
-        accI[m][b] = 0.0;
-      }
-    const int nG = terms->nMod > 1 ? terms->nMod : 1;
-    for (int gq = 0; gq < nG * p.nq; ++gq) {
-      const int g = gq / p.nq, q = gq - g * p.nq;
-      if (lane == 0) {
-        double xq[3];
-        pointGeometry(p, terms, g, q, S.X, S.J0, S.det0, S.J, S.det, S.Jinv, xq);
-        double2 lam = make_double2(0.0, 0.0), mu = make_double2(0.0, 0.0), cm = make_double2(0.0, 0.0);
-        const double *phq = p.bval + ((size_t)o * p.nq + q) * p.nb;  // scalar basis values (field nodes)
-        for (int t = 0; t < terms->n; ++t) {
-          const DevTerm &T = terms->t[t];
-          if (T.mod != g) continue;
-          if (T.kind == FG_TERM_ELASTIC) {
-            lam = cadd(lam, cmul(T.factor, evalExpr(T.coef, e, xq, phq, p.nb, q, p.nq)));
-            mu = cadd(mu, cmul(T.factor, evalExpr(T.coef2, e, xq, phq, p.nb, q, p.nq)));
-          } else if (T.kind == FG_TERM_MASS) {
-            cm = cadd(cm, cmul(T.factor, evalExpr(T.coef, e, xq, phq, p.nb, q, p.nq)));
-          }
-        }
-        const double wd = p.w[q] * S.det;
-        S.lam = make_double2(wd * lam.x, wd * lam.y);
-        S.mu = make_double2(wd * mu.x, wd * mu.y);
-        S.cm = make_double2(wd * cm.x, wd * cm.y);
-      }
-      __syncwarp();
-      const size_t base = ((size_t)o * p.nq + q) * p.nb;
-      for (int i = lane; i < ns; i += 32) {
-        const double g0 = p.bgrad[3 * (base + i)], g1 = p.bgrad[3 * (base + i) + 1], g2 = p.bgrad[3 * (base + i) + 2];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) S.G[r][i] = S.Jinv[r] * g0 + S.Jinv[3 + r] * g1 + S.Jinv[6 + r] * g2;
-        S.phi[i] = p.bval[base + i];
-      }
-      __syncwarp();
-#pragma unroll
-      for (int m = 0; m < MAXP; ++m) {
-        const int k = lane + 32 * m;
-        if (k < nPairs) {
-          const int i = pairI[k], j = pairJ[k];
-          const double gi[3] = {S.G[0][i], S.G[1][i], S.G[2][i]};
-          const double gj[3] = {S.G[0][j], S.G[1][j], S.G[2][j]};
-          const double dot = gi[0] * gj[0] + gi[1] * gj[1] + gi[2] * gj[2];
-          const double pp = S.phi[i] * S.phi[j];
-#pragma unroll
-          for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) {
-              const double tl = gj[b] * gi[a];
-              const double tm = gj[a] * gi[b] + (a == b ? dot : 0.0);
-              const double tc = a == b ? pp : 0.0;
-              accR[m][3 * a + b] += S.lam.x * tl + S.mu.x * tm + S.cm.x * tc;
-              if (CPLX) accI[m][3 * a + b] += S.lam.y * tl + S.mu.y * tm + S.cm.y * tc;
-            }
+  const bool elastic = a.comps & 1, mass = a.comps & 2;
+  const int nG = terms->nMod > 1 ? terms->nMod : 1;
+  for (int g = 0; g < nG; ++g) {
+    if (UNIFORM) {
+      for (int t = tid; t < live; t += kQuadThreads) {
+        double2 c[3];
+        const CoefPoint cp = {e0 + t, X, nullptr, 0, 0, p.nq};
+        scalarCoefs(terms, g, cp, c);
+        for (int k = 0; k < 3; ++k) {
+          coef[6 * t + 2 * k] = c[k].x;
+          coef[6 * t + 2 * k + 1] = c[k].y;
         }
       }
-      __syncwarp();
+      __syncthreads();
     }
-    const int ncomp = CPLX ? 2 : 1;
-    double *K = ke + (size_t)e * ncomp * n * n;
-#pragma unroll
-    for (int m = 0; m < MAXP; ++m) {
-      const int k = lane + 32 * m;
-      if (k < nPairs) {
-        const int i = pairI[k], j = pairJ[k];
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-          for (int b = 0; b < 3; ++b) {
-            const int ii = 3 * i + a, jj = 3 * j + b;  // test (i, a), unknown (j, b)
-            K[ii * n + jj] = accR[m][3 * a + b];
-            K[jj * n + ii] = accR[m][3 * a + b];
-            if (CPLX) {
-              K[n * n + ii * n + jj] = accI[m][3 * a + b];
-              K[n * n + jj * n + ii] = accI[m][3 * a + b];
-            }
-          }
-      }
-    }
-    if (be)
-      for (int i = lane; i < n; i += 32) be[(size_t)e * n + i] = make_double2(0.0, 0.0);
-    __syncwarp();
-  }
-}
-
-// Lowest-order-and-up HCurl field (FG_FORM_1): with the Form1 values
-// P = J^-T v and the Form2 curls C = J c / det (FieldEvaluator<Form1/Form2>,
-// src/term/evaluator/FieldEvaluator.h:59-105),
-//   Ke[i][j] = sum_q w det (c_curl C_j . C_i + c_m P_j . P_i),
-// or, with tensor terms (TensorFunction * curl, TensorFunction * dof: the
-// Maxwell PML), sum_q w det (C_i . A C_j + P_i . B P_j) with A = c_curl I + c D.
-// Warp per element, lanes over the pairs i <= j (the matrix is symmetric),
-// 256 pairs at a time: the points are visited once per 256 pairs.
-struct HcurlWarpSmem {
-  double X[kMaxNodes * 3];
-  double J0[9], J[9], Jinv[9];
-  double det0, det;
-  double2 a, b;  // w det c_curl, w det c_m
-  double2 Aw[6], Bw[6];  // w det times the curl and mass coefficient tensors (tensor terms)
-  double C[3][kMaxDofs], P[3][kMaxDofs];
-  double Cs[2][3][kMaxDofs], Ps[2][3][kMaxDofs];  // tensor terms: (w det A) C, (w det B) P (real, imaginary)
-};
-
-template <int MAXENT, bool CPLX>
-__global__ void __launch_bounds__(32 * kWarpsPerBlockElem)
-    k_element_hcurl_fp64(const PlanDev p, const DevTerms *__restrict__ terms, double *__restrict__ ke) {
-  __shared__ HcurlWarpSmem smem[kWarpsPerBlockElem];
-  __shared__ uint8_t pairI[kMaxDofs * (kMaxDofs + 1) / 2], pairJ[kMaxDofs * (kMaxDofs + 1) / 2];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int n = p.nb;
-  const int nEnt = n * (n + 1) / 2;
-  for (int k = threadIdx.x; k < nEnt; k += blockDim.x) {
-    int i = 0, rem = k;
-    while (rem >= n - i) {
-      rem -= n - i;
-      ++i;
-    }
-    pairI[k] = (uint8_t)i;
-    pairJ[k] = (uint8_t)(i + rem);
-  }
-  __syncthreads();
-  HcurlWarpSmem &S = smem[warp];
-  const bool tensor = terms->tensorTerm >= 0 || terms->tensorMassTerm >= 0;
-  const int64_t stride = (int64_t)gridDim.x * kWarpsPerBlockElem;
-  for (int64_t e = (int64_t)blockIdx.x * kWarpsPerBlockElem + warp; e < p.E; e += stride) {
-    const int o = p.orient ? p.orient[e] : 0;
-    for (int t = lane; t < p.nn * 3; t += 32) S.X[t] = p.xyz[3 * (int64_t)p.enodes[e * p.nn + t / 3] + t % 3];
-    __syncwarp();
-    // the pairs in chunks of 32 MAXENT, the points once per chunk
-    for (int c0 = 0; c0 < nEnt; c0 += 32 * MAXENT) {
-    double accR[MAXENT], accI[MAXENT];
-#pragma unroll
-    for (int m = 0; m < MAXENT; ++m) accR[m] = accI[m] = 0.0;
-    const int nG = terms->nMod > 1 ? terms->nMod : 1;
-    for (int gq = 0; gq < nG * p.nq; ++gq) {
-      const int g = gq / p.nq, q = gq - g * p.nq;
-      if (lane == 0) {
-        double xq[3];
-        pointGeometry(p, terms, g, q, S.X, S.J0, S.det0, S.J, S.det, S.Jinv, xq);
-        double2 cc = make_double2(0.0, 0.0), cm = make_double2(0.0, 0.0);
-        for (int t = 0; t < terms->n; ++t) {
-          const DevTerm &T = terms->t[t];
-          if (T.mod != g) continue;
-          const double2 v = evalExpr(T.coef, e, xq, nullptr, 0, q, p.nq);
-          if (T.kind == FG_TERM_GRAD_GRAD) cc = cadd(cc, cmul(T.factor, v));
-          else if (T.kind == FG_TERM_MASS) cm = cadd(cm, cmul(T.factor, v));
-        }
-        const double wd = p.w[q] * S.det;
-        S.a = make_double2(wd * cc.x, wd * cc.y);
-        S.b = make_double2(wd * cm.x, wd * cm.y);
-        if (tensor) {
-          double2 A[6], B[6];
-          coefTensor(terms, terms->tensorTerm, terms->tensor, g, e, xq, cc, A, nullptr, 0, q, p.nq);
-          coefTensor(terms, terms->tensorMassTerm, terms->tensorMass, g, e, xq, cm, B, nullptr, 0, q, p.nq);
-          for (int k = 0; k < 6; ++k) {
-            S.Aw[k] = make_double2(wd * A[k].x, wd * A[k].y);
-            S.Bw[k] = make_double2(wd * B[k].x, wd * B[k].y);
+    for (int d0 = 0; d0 < p.nq; d0 += a.QD) {
+      const int dn = min(a.QD, p.nq - d0);
+      for (int t = tid; t < live * dn; t += kQuadThreads) {
+        const int el = t / dn, qd = t - el * dn, q = d0 + qd;
+        PointGeom P;
+        quadPoint<false>(p, terms, g, q, X + el * p.nn * 3, geom + el * kQuadGeom, a.needX != 0, P);
+        double *d = D + (size_t)(el * a.QD + qd) * ND;
+        const double wd = p.w[q] * P.det;
+        for (int k = 0; k < 9; ++k) d[k] = P.Ji[k];
+        d[9] = wd;
+        if (!UNIFORM) {
+          double2 c[3];
+          const CoefPoint cp = {e0 + el, P.x, p.bval + ((size_t)orient[2 * el] * p.nq + q) * ns, ns, q, p.nq};
+          scalarCoefs(terms, g, cp, c);
+          d[10] = wd * c[0].x;
+          d[11] = wd * c[2].x;
+          d[12] = wd * c[1].x;
+          if (NC == 2) {
+            d[ND - 3] = wd * c[0].y;
+            d[ND - 2] = wd * c[2].y;
+            d[ND - 1] = wd * c[1].y;
           }
         }
       }
-      __syncwarp();
-      const size_t base = ((size_t)o * p.nq + q) * p.nb;
-      for (int i = lane; i < n; i += 32) {
-        const double *cr = p.bgrad + 3 * (base + i), *vr = p.bval + 3 * (base + i);
-        double Ci[3], Pi[3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-          Ci[r] = (S.J[r] * cr[0] + S.J[3 + r] * cr[1] + S.J[6 + r] * cr[2]) / S.det;
-          Pi[r] = S.Jinv[r] * vr[0] + S.Jinv[3 + r] * vr[1] + S.Jinv[6 + r] * vr[2];
-          S.C[r][i] = Ci[r];
-          S.P[r][i] = Pi[r];
-        }
-        if (tensor) {
-          const int row[3][3] = {{0, 3, 4}, {3, 1, 5}, {4, 5, 2}};
+      __syncthreads();
+      for (int q0 = d0; q0 < d0 + dn; q0 += a.QC) {
+        const int qn = min(a.QC, d0 + dn - q0);
+        if (q0 > d0) __syncthreads();  // H has been read
+        for (int t = tid; t < live * qn * ns; t += kQuadThreads) {
+          const int ep = t / ns, j = t - ep * ns, el = ep / qn, qc = ep - el * qn;
+          const size_t row = ((size_t)orient[2 * el] * p.nq + q0 + qc) * ns + j;
+          const double *d = D + (size_t)(el * a.QD + q0 + qc - d0) * ND;
+          double *h = H + (size_t)(el * a.QC + qc) * NH * ns + j;
+          const double g0 = p.bgrad[3 * row], g1 = p.bgrad[3 * row + 1], g2 = p.bgrad[3 * row + 2], ph = p.bval[row];
 #pragma unroll
           for (int r = 0; r < 3; ++r) {
-            S.Cs[0][r][i] = S.Aw[row[r][0]].x * Ci[0] + S.Aw[row[r][1]].x * Ci[1] + S.Aw[row[r][2]].x * Ci[2];
-            S.Ps[0][r][i] = S.Bw[row[r][0]].x * Pi[0] + S.Bw[row[r][1]].x * Pi[1] + S.Bw[row[r][2]].x * Pi[2];
-            if (CPLX) {
-              S.Cs[1][r][i] = S.Aw[row[r][0]].y * Ci[0] + S.Aw[row[r][1]].y * Ci[1] + S.Aw[row[r][2]].y * Ci[2];
-              S.Ps[1][r][i] = S.Bw[row[r][0]].y * Pi[0] + S.Bw[row[r][1]].y * Pi[1] + S.Bw[row[r][2]].y * Pi[2];
+            if (!elastic) continue;
+            const double G = d[r] * g0 + d[3 + r] * g1 + d[6 + r] * g2;
+            h[r * ns] = G;
+            if (UNIFORM) {
+              h[(3 + r) * ns] = d[9] * G;
+            } else {
+#pragma unroll
+              for (int part = 0; part < NC; ++part) {
+                h[(3 + 7 * part + r) * ns] = d[10 + 3 * part] * G;
+                h[(6 + 7 * part + r) * ns] = d[11 + 3 * part] * G;
+              }
             }
           }
-        }
-      }
-      __syncwarp();
-#pragma unroll
-      for (int m = 0; m < MAXENT; ++m) {
-        const int k = c0 + lane + 32 * m;
-        if (k < nEnt) {
-          const int i = pairI[k], j = pairJ[k];
-          if (tensor) {
-            accR[m] += S.C[0][i] * S.Cs[0][0][j] + S.C[1][i] * S.Cs[0][1][j] + S.C[2][i] * S.Cs[0][2][j] +
-                       S.P[0][i] * S.Ps[0][0][j] + S.P[1][i] * S.Ps[0][1][j] + S.P[2][i] * S.Ps[0][2][j];
-            if (CPLX)
-              accI[m] += S.C[0][i] * S.Cs[1][0][j] + S.C[1][i] * S.Cs[1][1][j] + S.C[2][i] * S.Cs[1][2][j] +
-                         S.P[0][i] * S.Ps[1][0][j] + S.P[1][i] * S.Ps[1][1][j] + S.P[2][i] * S.Ps[1][2][j];
+          if (UNIFORM) {
+            h[6 * ns] = d[9] * ph;
           } else {
-            const double cc = S.C[0][i] * S.C[0][j] + S.C[1][i] * S.C[1][j] + S.C[2][i] * S.C[2][j];
-            const double pp = S.P[0][i] * S.P[0][j] + S.P[1][i] * S.P[1][j] + S.P[2][i] * S.P[2][j];
-            accR[m] += S.a.x * cc + S.b.x * pp;
-            if (CPLX) accI[m] += S.a.y * cc + S.b.y * pp;
+#pragma unroll
+            for (int part = 0; part < NC; ++part) h[(9 + 7 * part) * ns] = d[12 + 3 * part] * ph;
           }
         }
-      }
-      __syncwarp();
-    }
-    const int ncomp = CPLX ? 2 : 1;
-    double *K = ke + (size_t)e * ncomp * n * n;
+        __syncthreads();
+        for (int qc = 0; qc < qn; ++qc) {
+          const double *Hq = H + (size_t)qc * NH * ns;
+          const double *bv = p.bval + (size_t)(q0 + qc) * ns;
 #pragma unroll
-    for (int m = 0; m < MAXENT; ++m) {
-      const int k = c0 + lane + 32 * m;
-      if (k < nEnt) {
-        const int i = pairI[k], j = pairJ[k];
-        K[i * n + j] = K[j * n + i] = accR[m];
-        if (CPLX) K[n * n + i * n + j] = K[n * n + j * n + i] = accI[m];
+          for (int m = 0; m < MAXP; ++m)
+            if (m < mine) {
+              const double *hi = Hq + offI[m], *hj = Hq + offJ[m];
+              if (elastic) {
+                const double gi[3] = {hi[0], hi[ns], hi[2 * ns]};
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                  if (UNIFORM) {
+                    const double w = hj[(3 + b) * ns];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) acc[m][3 * c + b] = fma(gi[c], w, acc[m][3 * c + b]);
+                  } else {
+#pragma unroll
+                    for (int part = 0; part < NC; ++part) {
+                      const double l = hj[(3 + 7 * part + b) * ns], u = hj[(6 + 7 * part + b) * ns];
+#pragma unroll
+                      for (int c = 0; c < 3; ++c) {
+                        double &al = acc[m][(19 * part + 3 * c + b) % NS], &au = acc[m][(19 * part + 9 + 3 * c + b) % NS];
+                        al = fma(gi[c], l, al);
+                        au = fma(gi[c], u, au);
+                      }
+                    }
+                  }
+                }
+              }
+              if (mass) {
+                const double ph = bv[rowI[m]];
+                if (UNIFORM) {
+                  acc[m][9] = fma(ph, hj[6 * ns], acc[m][9]);
+                } else {
+#pragma unroll
+                  for (int part = 0; part < NC; ++part) {
+                    double &am = acc[m][(19 * part + 18) % NS];
+                    am = fma(ph, hj[(9 + 7 * part) * ns], am);
+                  }
+                }
+              }
+            }
+        }
       }
-    }
-    __syncwarp();
     }
   }
+  constexpr int ncomp = CPLX ? 2 : 1;
+#pragma unroll
+  for (int m = 0; m < MAXP; ++m)
+    if (m < mine) {
+      const int k = tid + kQuadThreads * m, el = k / a.nEnt, pr = pairs[k - el * a.nEnt], i = pr >> 8, j = pr & 255;
+      double *K = ke + (size_t)(e0 + el) * ncomp * n * n;
+#pragma unroll
+      for (int part = 0; part < ncomp; ++part) {
+        double lam = 1.0, mu = 1.0, cm = 1.0;
+        if (UNIFORM) {
+          lam = coef[6 * el + part];
+          cm = coef[6 * el + 2 + part];
+          mu = coef[6 * el + 4 + part];
+        }
+        // the lambda-, mu- and mass-weighted sums
+        const double *sl = acc[m] + (UNIFORM ? 0 : (19 * part) % NS), *su = UNIFORM ? sl : sl + 9;
+        const double diag = mu * (su[0] + su[4] + su[8]) + cm * (UNIFORM ? sl[9] : sl[(18) % NS]);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+          for (int b = 0; b < 3; ++b) {
+            double v = lam * sl[3 * c + b] + mu * su[3 * b + c];
+            if (c == b) v += diag;
+            const int ii = 3 * i + c, jj = 3 * j + b;  // test (i, c), unknown (j, b)
+            K[(size_t)part * n * n + ii * n + jj] = v;
+            K[(size_t)part * n * n + jj * n + ii] = v;
+          }
+      }
+    }
+  if (be)
+    for (int t = tid; t < live * n; t += kQuadThreads) be[(size_t)e0 * n + t] = make_double2(0.0, 0.0);
+}
+
+// Elements per block and points per chunk. An SM runs blocks / SMs of them
+// one after the other as far as its FP64 pipe goes, each as long as its
+// fullest warp has entries per thread (plus about half an entry for the other
+// phases): the number of elements with the least total, which is few for
+// small meshes (all SMs busy, short blocks) and the best filled block for
+// large ones: 82,944 tetrahedra of order 3 took 4.08 ms with the 6 elements
+// this picks, 4.34 with 5 or 4 and 4.89 with 2; order 2 with complex D, 1.51 ms
+// with 16 or more, 1.65 with 9, 2.41 with 3. D is formed for as many points as give every thread an
+// (element, point) pair, H for what the remaining shared memory holds.
+static bool quadShape(const PlanDev &p, int nEnt, int n, int nU, int nd, int nh, bool be, int nPairs, int maxItems, QuadArgs *a) {
+  const int64_t sms = smCount();
+  auto bytes = [&](int NE, int QD, int QC) { return (size_t)quadLayout(NE, QD, QC, p.nn, n, nU, nd, nh, be, nPairs).total * 8; };
+  double best = 0.0;
+  a->NE = 0;
+  for (int NE = 1; NE <= kQuadMaxElems && (int64_t)NE * nEnt <= (int64_t)kQuadThreads * maxItems; ++NE) {
+    if (bytes(NE, std::min(p.nq, 2), std::min(p.nq, 2)) > kQuadSmem && NE > 1) break;
+    const int64_t blocks = (p.E + NE - 1) / NE;
+    const double cost = (double)((blocks + sms - 1) / sms) * ((NE * nEnt + kQuadThreads - 1) / kQuadThreads + 0.5);
+    if (a->NE == 0 || cost < best) {
+      best = cost;
+      a->NE = NE;
+    }
+  }
+  if (a->NE == 0 || bytes(a->NE, 1, 1) > kQuadSmem) return false;
+  int QD = std::min(p.nq, (kQuadThreads + a->NE - 1) / a->NE);
+  while (QD > 1 && bytes(a->NE, QD, std::min(QD, 2)) > kQuadSmem) --QD;
+  int QC = std::min(QD, 16);
+  while (QC > 1 && bytes(a->NE, QD, QC) > kQuadSmem) --QC;
+  auto even = [](int count, int most) {  // chunks of nearly equal size
+    const int chunks = (count + most - 1) / most;
+    return (count + chunks - 1) / chunks;
+  };
+  a->QD = even(p.nq, QD);
+  a->QC = even(a->QD, std::min(QC, a->QD));
+  a->nEnt = nEnt;
+  return true;
+}
+
+// What the launch's switches need to know of the terms
+struct TermUse {
+  bool grad = false, mass = false, pointBilinear = false, pointSource = false;
+};
+static TermUse termUse(const DevTerms &terms) {
+  TermUse u;
+  auto scan = [](const DevExpr *ex, int count, bool &point) {
+    for (int k = 0; k < count; ++k) point = point || ex[k].cls == kExprPoint;
+  };
+  for (int t = 0; t < terms.n; ++t) {
+    const DevTerm &T = terms.t[t];
+    switch (T.kind) {
+      case FG_TERM_SOURCE: scan(&T.coef, 1, u.pointSource); continue;
+      case FG_TERM_SOURCE_GRAD:
+        scan(&T.coef, 1, u.pointSource);
+        scan(terms.srcGrad, 3, u.pointSource);
+        continue;
+      case FG_TERM_MASS:
+      case FG_TERM_MASS_TENSOR: u.mass = true; break;
+      case FG_TERM_ADVECTION: u.mass = true; break;  // tested by values
+      default: u.grad = true;
+    }
+    scan(&T.coef, 1, u.pointBilinear);
+    if (T.kind == FG_TERM_ELASTIC) scan(&T.coef2, 1, u.pointBilinear);
+    if (T.kind == FG_TERM_GRAD_GRAD_TENSOR) scan(terms.tensor, 6, u.pointBilinear);
+    if (T.kind == FG_TERM_MASS_TENSOR) scan(terms.tensorMass, 6, u.pointBilinear);
+    if (T.kind == FG_TERM_GRAD_GRAD_TENSOR_FULL) scan(terms.tensorFull, 9, u.pointBilinear);
+    if (T.kind == FG_TERM_ADVECTION) scan(terms.advect, 3, u.pointBilinear);
+    if (T.kind == FG_TERM_VECTOR_GRAD_TEST) scan(terms.vecGrad, 3, u.pointBilinear);
+  }
+  return u;
+}
+
+static int quadFail() {
+  setLastError("FP64 element kernel: more basis functions or nodes per element than a block's shared memory holds");
+  return FG_ERR_UNSUPPORTED;
+}
+
+template <int KIND, bool CPLX, bool SPLIT, bool MASKED, int MAXE>
+static int quadLaunch(const PlanDev &p, const DevTerms *dterms, QuadArgs a, int nEnt, double *ke, double2 *be, cudaStream_t s) {
+  constexpr int NC = CPLX ? 2 : 1;
+  const int nPairs = KIND == kQuadFull ? 0 : nEnt, nd = quadD(KIND) * NC, nh = quadComps(KIND) * NC;
+  if (!quadShape(p, nEnt, p.nb, p.nbU, nd, nh, be != nullptr, nPairs, MAXE, &a)) return quadFail();
+  const size_t smem = (size_t)quadLayout(a.NE, a.QD, a.QC, p.nn, p.nb, p.nbU, nd, nh, be != nullptr, nPairs).total * 8;
+  k_element_fp64<KIND, CPLX, SPLIT, MASKED, MAXE>
+      <<<(unsigned)((p.E + a.NE - 1) / a.NE), kQuadThreads, smem, s>>>(p, dterms, a, ke, be);
+  countLaunch();
+  FG_CUDA(cudaGetLastError());
+  return FG_OK;
+}
+
+// The kernel of one kind for these terms. ke null: the right-hand side alone.
+template <int KIND, int MAXE>
+static int quadKind(const PlanDev &p, const DevTerms &terms, const DevTerms *dterms, int nEnt, double *ke, double2 *be, cudaStream_t s) {
+  const TermUse u = termUse(terms);
+  QuadArgs a;
+  std::memset(&a, 0, sizeof(a));
+  const int full = (1 << quadComps(KIND)) - 1;
+  a.comps = p.tableComps & ((u.grad ? 7 : 0) | (u.mass ? full & ~7 : 0));
+  a.uniform = !u.pointBilinear;
+  a.needX = (ke && u.pointBilinear) || (be && u.pointSource) || terms.hasJacMod;
+  const bool masked = a.comps != full, cplx = terms.complexKe != 0;
+  // complex sums of real integrals: one group of terms, no tensors
+  const bool split = KIND != kQuadFull && cplx && a.uniform && terms.nMod <= 1 && terms.tensorTerm < 0 && terms.tensorMassTerm < 0;
+#define FG_QUAD(C, S)                                                                              \
+  (masked ? quadLaunch<KIND, C, S, true, MAXE>(p, dterms, a, nEnt, ke, be, s)                      \
+          : quadLaunch<KIND, C, S, false, MAXE>(p, dterms, a, nEnt, ke, be, s))
+  if constexpr (KIND != kQuadFull) {
+    if (split) return FG_QUAD(false, true);
+  }
+  return cplx ? FG_QUAD(true, false) : FG_QUAD(false, false);
+#undef FG_QUAD
+}
+
+template <bool UNIFORM, bool CPLX, int MAXP>
+static int quadElastic(const PlanDev &p, const DevTerms *dterms, QuadArgs a, int nEnt, double *ke, double2 *be, cudaStream_t s) {
+  constexpr int NC = (!UNIFORM && CPLX) ? 2 : 1, ND = 10 + (UNIFORM ? 0 : 3 * NC), NH = UNIFORM ? 7 : 3 + 7 * NC;
+  if (!quadShape(p, nEnt, 0, p.nb, ND, NH, false, nEnt, MAXP, &a)) return quadFail();
+  const size_t smem = (size_t)quadLayout(a.NE, a.QD, a.QC, p.nn, 0, p.nb, ND, NH, false, nEnt).total * 8;
+  k_element_elastic_fp64<UNIFORM, CPLX, MAXP><<<(unsigned)((p.E + a.NE - 1) / a.NE), kQuadThreads, smem, s>>>(p, dterms, a, ke, be);
+  countLaunch();
+  FG_CUDA(cudaGetLastError());
+  return FG_OK;
 }
 
 static int launchElementKernels(fg_plan *plan, const DevTerms &terms, const DevTerms *dterms, double *ke, double *be, cudaStream_t s) {
   const PlanDev &p = plan->d;
+  if (p.E == 0) return FG_OK;
+  double2 *be2 = (double2 *)be;
   if (terms.nonSym) {
-    const int perLane = (p.nb * p.nbU + 31) / 32;
-    int64_t blocks = std::min<int64_t>((p.E + kWarpsPerBlockElem - 1) / kWarpsPerBlockElem, (int64_t)smCount() * 64);
-    if (blocks < 1) blocks = 1;
-    const bool cplx = terms.complexKe != 0;
-    double2 *be2 = (double2 *)be;
-    ProfScope prof("k_element_full_fp64", s);
-#define FG_LAUNCH_FULL(M)                                                                                             \
-  do {                                                                                                                \
-    if (cplx) k_element_full_fp64<M, true><<<(unsigned)blocks, 32 * kWarpsPerBlockElem, 0, s>>>(p, dterms, ke, be2);  \
-    else k_element_full_fp64<M, false><<<(unsigned)blocks, 32 * kWarpsPerBlockElem, 0, s>>>(p, dterms, ke, be2);     \
-  } while (0)
-    if (perLane <= 2) FG_LAUNCH_FULL(2);
-    else if (perLane <= 8) FG_LAUNCH_FULL(8);
-    else if (perLane <= 13) FG_LAUNCH_FULL(13);
-    else if (perLane <= 39) FG_LAUNCH_FULL(39);
-    else {
+    const int nEnt = p.nb * p.nbU;
+    if (nEnt > 39 * 32) {
       setLastError("FP64 full element kernel: more than 35 basis functions per element");
       return FG_ERR_UNSUPPORTED;
     }
-#undef FG_LAUNCH_FULL
-    countLaunch();
-    FG_CUDA(cudaGetLastError());
-    return FG_OK;
+    ProfScope prof("k_element_full_fp64", s);
+    return quadKind<kQuadFull, 10>(p, terms, dterms, nEnt, ke, be2, s);
   }
-  if (p.E > 0 && factoredFp64Applies(plan, terms)) {
+  if (factoredFp64Applies(plan, terms)) {
     int st = launchFactoredFp64(plan, terms, dterms, ke, s);
     if (st) return st;
     if (be) {
@@ -634,83 +891,54 @@ static int launchElementKernels(fg_plan *plan, const DevTerms &terms, const DevT
         setLastError("HCurl fields take no source terms");
         return FG_ERR_UNSUPPORTED;
       }
-      return launchRhsFp64(plan, dterms, be, s);
+      return launchRhsFp64(plan, terms, dterms, be, s);
     }
     return FG_OK;
   }
+  const int nEnt = p.nb * (p.nb + 1) / 2;
   if (p.form == FG_FORM_1) {
-    const int nEnt = p.nb * (p.nb + 1) / 2;
-    const int perLane = (nEnt + 31) / 32;
-    int64_t blocks = std::min<int64_t>((p.E + kWarpsPerBlockElem - 1) / kWarpsPerBlockElem, (int64_t)smCount() * 64);
-    if (blocks < 1) blocks = 1;
-    const bool cplx = terms.complexKe != 0;
     ProfScope prof("k_element_hcurl_fp64", s);
-#define FG_LAUNCH_HC(M)                                                                                              \
-  do {                                                                                                               \
-    if (cplx) k_element_hcurl_fp64<M, true><<<(unsigned)blocks, 32 * kWarpsPerBlockElem, 0, s>>>(p, dterms, ke);     \
-    else k_element_hcurl_fp64<M, false><<<(unsigned)blocks, 32 * kWarpsPerBlockElem, 0, s>>>(p, dterms, ke);        \
-  } while (0)
-    if (perLane <= 1) FG_LAUNCH_HC(1);
-    else FG_LAUNCH_HC(8);  // 256 pairs per chunk: one chunk up to 22 functions, more chunks beyond
-#undef FG_LAUNCH_HC
-    (void)be;
-    countLaunch();
-    FG_CUDA(cudaGetLastError());
-    return FG_OK;
+    // one thread's entries: 10 reach 50 functions, 17 the limit of 64
+    if (nEnt <= 10 * kQuadThreads) return quadKind<kQuadHcurl, 10>(p, terms, dterms, nEnt, ke, nullptr, s);
+    return quadKind<kQuadHcurl, 17>(p, terms, dterms, nEnt, ke, nullptr, s);
   }
   if (p.mult != 1 || terms.hasElastic) {
     if (p.mult != 3 || terms.hasSource) {
       setLastError("FP64 element kernel: compound fields take the elastic and mass terms only");
       return FG_ERR_UNSUPPORTED;
     }
-    const int nPairs = p.nb * (p.nb + 1) / 2;
-    const int perLane = (nPairs + 31) / 32;
-    int64_t blocks = std::min<int64_t>((p.E + kWarpsPerBlockElem - 1) / kWarpsPerBlockElem, (int64_t)smCount() * 64);
-    if (blocks < 1) blocks = 1;
-    const bool cplx = terms.complexKe != 0;
-    ProfScope prof("k_element_elastic_fp64", s);
-#define FG_LAUNCH_EL(M)                                                                                                    \
-  do {                                                                                                                     \
-    if (cplx) k_element_elastic_fp64<M, true><<<(unsigned)blocks, 32 * kWarpsPerBlockElem, 0, s>>>(p, dterms, ke, (double2 *)be); \
-    else k_element_elastic_fp64<M, false><<<(unsigned)blocks, 32 * kWarpsPerBlockElem, 0, s>>>(p, dterms, ke, (double2 *)be); \
-  } while (0)
-    if (perLane <= 2) FG_LAUNCH_EL(2);
-    else if (perLane <= 4) FG_LAUNCH_EL(4);
-    else if (perLane <= 8) FG_LAUNCH_EL(8);
-    else {
+    if (nEnt > 8 * 32) {
       setLastError("FP64 elastic kernel: more than 21 scalar basis functions per element");
       return FG_ERR_UNSUPPORTED;
     }
-#undef FG_LAUNCH_EL
-    countLaunch();
-    FG_CUDA(cudaGetLastError());
-    return FG_OK;
+    const TermUse u = termUse(terms);
+    QuadArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.comps = (u.grad ? 1 : 0) | (u.mass ? 2 : 0);
+    a.needX = u.pointBilinear || terms.hasJacMod;
+    // the element's sums are scaled once at the end: one group of terms
+    a.uniform = !u.pointBilinear && terms.nMod <= 1;
+    const bool cplx = terms.complexKe != 0;
+    ProfScope prof("k_element_elastic_fp64", s);
+    if (a.uniform)
+      return cplx ? quadElastic<true, true, 4>(p, dterms, a, nEnt, ke, be2, s) : quadElastic<true, false, 4>(p, dterms, a, nEnt, ke, be2, s);
+    return cplx ? quadElastic<false, true, 2>(p, dterms, a, nEnt, ke, be2, s) : quadElastic<false, false, 2>(p, dterms, a, nEnt, ke, be2, s);
   }
-  const int nEnt = p.nb * (p.nb + 1) / 2;
-  const int perLane = (nEnt + 31) / 32;
-  const int sms = smCount();
-  int64_t blocks = (p.E + kWarpsPerBlockElem - 1) / kWarpsPerBlockElem;
-  blocks = std::min<int64_t>(blocks, (int64_t)sms * 64);
-  if (blocks < 1) blocks = 1;
-  const bool cplx = terms.complexKe != 0;
-  double2 *be2 = (double2 *)be;
-#define FG_LAUNCH_ELEM(M)                                                                                   \
-  do {                                                                                                      \
-    if (cplx) k_element_fp64<M, true><<<(unsigned)blocks, 32 * kWarpsPerBlockElem, 0, s>>>(p, dterms, ke, be2); \
-    else k_element_fp64<M, false><<<(unsigned)blocks, 32 * kWarpsPerBlockElem, 0, s>>>(p, dterms, ke, be2);  \
-  } while (0)
-  ProfScope prof("k_element_fp64", s);
-  if (perLane <= 1) FG_LAUNCH_ELEM(1);
-  else if (perLane <= 8) FG_LAUNCH_ELEM(8);
-  else if (perLane <= 20) FG_LAUNCH_ELEM(20);
-  else {
+  if (nEnt > 20 * 32) {
     setLastError("FP64 element kernel: more than 35 basis functions per element");
     return FG_ERR_UNSUPPORTED;
   }
-#undef FG_LAUNCH_ELEM
-  countLaunch();
-  FG_CUDA(cudaGetLastError());
-  return FG_OK;
+  ProfScope prof("k_element_fp64", s);
+  return quadKind<kQuadSym, 10>(p, terms, dterms, nEnt, ke, be2, s);
+}
+
+// FP64 element right-hand sides of the source terms into be ([E][n] complex):
+// the quadrature kernel without its element matrices
+int launchRhsFp64(fg_plan *plan, const DevTerms &terms, const DevTerms *dterms, double *be, cudaStream_t s) {
+  const PlanDev &p = plan->d;
+  if (p.E == 0) return FG_OK;
+  ProfScope prof("k_rhs_fp64", s);
+  return quadKind<kQuadSym, 10>(p, terms, dterms, p.nb, nullptr, (double2 *)be, s);
 }
 
 // With Jacobian modificators the kernels flag integration points outside a

@@ -705,44 +705,6 @@ __global__ void __launch_bounds__(kThreadsGemm, 2)
   if (warp == 0) tmemDealloc(tmem, (uint32_t)tmemCols);
 }
 
-// ---------------------------------------------------- FP64 RHS (mixed)
-
-// b_e[i] = sum_q w det conj(phi_i) f(x_q)  (LinearTerm::evaluate), warp per element
-__global__ void k_rhs_fp64(const PlanDev p, const DevTerms *__restrict__ terms, double2 *__restrict__ be) {
-  const int lane = threadIdx.x & 31;
-  const int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (e >= p.E) return;
-  const int o = p.orient ? p.orient[e] : 0;
-  double X[kMaxNodes * 3];
-  for (int k = 0; k < p.nn; ++k)
-    for (int c = 0; c < 3; ++c) X[3 * k + c] = p.xyz[3 * (int64_t)p.enodes[e * p.nn + k] + c];
-  double2 acc[2] = {make_double2(0, 0), make_double2(0, 0)};
-  for (int q = 0; q < p.nq; ++q) {
-    double2 s = make_double2(0.0, 0.0);
-    if (lane == 0) {
-      double J[9];
-      const double det = jacobian(p.dim, p.nn, X, p.geoGrad + (size_t)q * p.nn * 3, J);
-      double xq[3] = {0, 0, 0};
-      for (int k = 0; k < p.nn; ++k)
-        for (int c = 0; c < 3; ++c) xq[c] += p.geoVal[q * p.nn + k] * X[3 * k + c];
-      double2 f = make_double2(0.0, 0.0);
-      for (int t = 0; t < terms->n; ++t)
-        if (terms->t[t].kind == FG_TERM_SOURCE)
-          f = cadd(f, evalExpr(terms->t[t].coef, e, xq, p.bval + ((size_t)o * p.nq + q) * p.nb, p.nb, q, p.nq));
-      s = make_double2(p.w[q] * det * f.x, p.w[q] * det * f.y);
-    }
-    s.x = __shfl_sync(0xffffffffu, s.x, 0);
-    s.y = __shfl_sync(0xffffffffu, s.y, 0);
-    const size_t base = ((size_t)o * p.nq + q) * p.nb;
-    for (int i = lane; i < p.nb; i += 32) {
-      const double ph = p.bval[base + i];
-      acc[i >> 5].x += s.x * ph;
-      acc[i >> 5].y += s.y * ph;
-    }
-  }
-  for (int i = lane; i < p.nb; i += 32) be[(size_t)e * p.nb + i] = acc[i >> 5];
-}
-
 // -------------------------------------------- error report (device side)
 
 // per element ||Ke32 - Ke64||_F^2 and ||Ke64||_F^2; the FP64 matrices are
@@ -1136,18 +1098,6 @@ FactorJob mixedFactorJob(fg_plan *plan, const DevTerms *dterms, bool tensor, int
   return j;
 }
 
-// FP64 element right-hand sides of the source terms into be ([E][n] complex)
-int launchRhsFp64(fg_plan *plan, const DevTerms *dterms, double *be, cudaStream_t s) {
-  const PlanDev &p = plan->d;
-  if (p.E == 0) return FG_OK;
-  ProfScope prof("k_rhs_fp64", s);
-  const int64_t threads = p.E * 32;
-  k_rhs_fp64<<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(p, dterms, (double2 *)be);
-  countLaunch();
-  FG_CUDA(cudaGetLastError());
-  return FG_OK;
-}
-
 // Accessors for the multi-frequency path
 float *mixedKe(fg_plan *plan, KeLayout *lay) {
   MixedState *m = state(plan);
@@ -1240,7 +1190,7 @@ extern "C" int fg_assemble_mixed(fg_plan *plan, const fg_term_desc *terms, int32
     if (dt.hasSource && rhs) {
       if ((st = ensureDevice((void **)&plan->be, &plan->beBytes, (size_t)p.E * p.n * 16))) return st;
       be = plan->be;
-      if ((st = launchRhsFp64(plan, dterms, be, s))) return st;
+      if ((st = launchRhsFp64(plan, dt, dterms, be, s))) return st;
     }
     if ((st = launchFused(plan, dt, dterms, (const double2 *)be, (double2 *)o.values, (double2 *)o.rhs, s))) return st;
     if ((st = finishOutputs(plan, o, csr_values, rhs, s))) return st;
@@ -1259,11 +1209,7 @@ extern "C" int fg_assemble_mixed(fg_plan *plan, const fg_term_desc *terms, int32
   if (dt.hasSource && rhs) {
     if ((st = ensureDevice((void **)&plan->be, &plan->beBytes, (size_t)p.E * p.n * 16))) return st;
     be = plan->be;
-    ProfScope prof("k_rhs_fp64", s);
-    const int64_t threads = p.E * 32;
-    k_rhs_fp64<<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(p, dterms, (double2 *)be);
-    countLaunch();
-    FG_CUDA(cudaGetLastError());
+    if ((st = launchRhsFp64(plan, dt, dterms, be, s))) return st;
   }
   if (p.E > 0)
     if ((st = launchMixedElement(plan, &dterms, 1, dt.tensorTerm >= 0 ? 1u : 0u, s))) return st;

@@ -170,7 +170,7 @@ int runElements(fg_batch *b, cudaStream_t s) {
   if (b->mixed) {
     for (int q = 0; q < b->n; ++q)
       if (b->source[q])
-        if ((st = launchRhsFp64(b->plans[q], b->termsDev[q], b->plans[q]->be, s))) return st;
+        if ((st = launchRhsFp64(b->plans[q], b->terms[q], b->termsDev[q], b->plans[q]->be, s))) return st;
     if ((st = launchFactorsBatch(b->factorJobs, b->n, b->totalElems, s))) return st;
     if (!b->tilesHost.empty())
       if ((st = launchContract(b->gemmDev, b->tiles, b->ctaStart, b->nCta, b->err, b->maxK3, b->smem, s, 512, nullptr,

@@ -145,6 +145,8 @@ struct PlanDev {
   int32_t slotBytes;
   int32_t slotLd;         // slot row stride (entries)
   int32_t maxRowLen;
+  int32_t tableComps;     // components of the basis tables that are not zero everywhere: bits 0-2 the reference gradient
+                          // (curl), then the value (H1: bit 3; HCurl: bits 3-5)
   int32_t plainSlots;     // 1: no element row has two columns in one slot (plain shared adds are race-free)
   int *jmErr;             // set by the FP64 element kernels: an integration point outside a shell
   const double2 *lscale;  // [E][n] linked DOF coefficient (1 for other DOFs), or null without linked DOFs
@@ -330,7 +332,7 @@ int launchFactoredFp64(fg_plan *plan, const DevTerms &terms, const DevTerms *dte
 // mixed path pieces shared with the multi-frequency path (assemble_mixed.cu)
 int prepareMixed(fg_plan *plan, int ncomp, int groups);
 int launchMixedElement(fg_plan *plan, const DevTerms *const *dterms, int groups, uint32_t tensorMask, cudaStream_t s);
-int launchRhsFp64(fg_plan *plan, const DevTerms *dterms, double *be, cudaStream_t s);
+int launchRhsFp64(fg_plan *plan, const DevTerms &terms, const DevTerms *dterms, double *be, cudaStream_t s);
 float *mixedKe(fg_plan *plan, KeLayout *lay);
 int mixedCheckTimeout(fg_plan *plan, bool wait);
 int mixedRecordError(fg_plan *plan, cudaStream_t s);
@@ -715,28 +717,5 @@ __host__ __device__ inline bool applyJacMod(const DevJacMod &m, const double *x,
   for (int k = 0; k < 9; ++k) J[k] = J2[k];
   return true;
 }
-
-// Lane-0 geometry of integration point q for the terms of modificator group
-// g: J0/det0 hold the unmodified Jacobian (formed once for affine elements),
-// J/det/Jinv the one the group's terms use, xq the physical point.
-__device__ inline void pointGeometry(const PlanDev &p, const DevTerms *terms, int g, int q, const double *X, double *J0, double &det0,
-                                     double *J, double &det, double *Jinv, double *xq) {
-  if (q == 0 || !p.affine) det0 = jacobian(p.dim, p.nn, X, p.geoGrad + (size_t)q * p.nn * 3, J0);
-  xq[0] = xq[1] = xq[2] = 0.0;
-  for (int k = 0; k < p.nn; ++k) {
-    const double v = p.geoVal[q * p.nn + k];
-    xq[0] += v * X[3 * k];
-    xq[1] += v * X[3 * k + 1];
-    xq[2] += v * X[3 * k + 2];
-  }
-  const DevJacMod &m = terms->mods[g];
-  if (m.kind != FG_JACMOD_NONE || q == 0 || !p.affine || terms->nMod > 1) {
-    for (int k = 0; k < 9; ++k) J[k] = J0[k];
-    det = det0;
-    if (m.kind != FG_JACMOD_NONE && !applyJacMod(m, xq, J, det)) atomicOr(p.jmErr, 1);
-    jacobianInverse(J, det, Jinv);
-  }
-}
-
 
 }  // namespace femg

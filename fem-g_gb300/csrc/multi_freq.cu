@@ -411,7 +411,7 @@ int runGroups(fg_plan *plan, const fg_term_desc *terms, int32_t n_terms, int32_t
     if ((st = prepareMixed(plan, ncomp, G))) return st;
     if ((st = mixedCheckTimeout(plan, false))) return st;
     if (source)
-      if ((st = launchRhsFp64(plan, m->dev[0], be, s))) return st;
+      if ((st = launchRhsFp64(plan, m->terms[0], m->dev[0], be, s))) return st;
     if (p.E > 0) {
       const DevTerms *devs[kMaxGroups] = {m->dev[0], m->dev[1], m->dev[2]};
       uint32_t tensorMask = 0;

@@ -465,6 +465,16 @@ static int createPlan(const fg_mesh_desc *mesh, const fg_rule_desc *rule, const 
     for (size_t r = 0; r < (size_t)E * n; ++r)
       std::fill(slot8.begin() + (int64_t)(r * nS + nc), slot8.begin() + (int64_t)((r + 1) * nS), (uint8_t)0xFE);
 
+  // table components that vanish everywhere (the third one on triangles, say)
+  {
+    const size_t rows = (size_t)space->n_orientations * rule->nq * space->n_basis;
+    const int nv = d.form == FG_FORM_1 ? 3 : 1;
+    for (size_t k = 0; k < rows; ++k) {
+      for (int c = 0; c < 3; ++c) d.tableComps |= space->basis_grad[3 * k + c] != 0.0 ? 1 << c : 0;
+      for (int c = 0; c < nv; ++c) d.tableComps |= space->basis_val[nv * k + c] != 0.0 ? 8 << c : 0;
+    }
+  }
+
   int st;
   if ((st = upload(plan, mesh->node_xyz, (size_t)mesh->n_nodes * 3, &d.xyz))) return st;
   if ((st = upload(plan, en.data(), en.size(), &d.enodes))) return st;
