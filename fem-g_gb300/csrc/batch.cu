@@ -142,7 +142,7 @@ int checkBatchError(fg_batch *b, bool wait) {
 void layoutClass(fg_batch *b, GatherClass &c) {
   int64_t rows = 0;
   for (int q : c.probs) rows += (int64_t)b->plans[q]->d.nRows;
-  const int64_t cap = (int64_t)smCount() * 16;
+  const int64_t cap = (int64_t)smCount() * kGatherWarpsPerSm / c.shape.wpb;
   int64_t start = 0;
   for (size_t k = 0; k < c.probs.size(); ++k) {
     const int64_t r = (int64_t)b->plans[c.probs[k]]->d.nRows;
@@ -162,7 +162,9 @@ int uploadJobs(GatherClass &c, cudaStream_t s) {
 }
 
 int runGatherClass(fg_batch *b, GatherClass &c, cudaStream_t s) {
-  return launchGatherBatch(c.jobsDev, (int)c.probs.size(), c.blocks, c.slotBytes, c.kcplx, b->mixed ? 1 : 0, c.shape, s);
+  bool simple = true;
+  for (size_t k = 0; k < c.probs.size(); ++k) simple = simple && gatherSimple(c.jobsHost[k].p, c.jobsHost[k].be);
+  return launchGatherBatch(c.jobsDev, (int)c.probs.size(), c.blocks, c.slotBytes, c.kcplx, b->mixed ? 1 : 0, c.shape, simple, s);
 }
 
 int runElements(fg_batch *b, cudaStream_t s) {
@@ -292,20 +294,13 @@ int tune(fg_batch *b, cudaStream_t s) {
   if ((st = runElements(b, s))) return st;
   for (size_t ci = 0; ci < b->classes.size(); ++ci) {
     GatherClass &c = b->classes[ci];
-    const GatherShape base = gatherShape(c.n, c.maxRowLen, c.kcplx, b->mixed, 0, 0);
+    const GatherJob &J0 = c.jobsHost[0];
+    const GatherShape base = gatherShape(J0.p, c.maxRowLen, c.kcplx, b->mixed, J0.lay, 0);
     std::vector<GatherShape> cands;
-    for (int L : {base.L, base.L * 2})
-      for (int w : {4, 8}) {
-        if (L > 32) continue;
-        GatherShape g = gatherShape(c.n, c.maxRowLen, c.kcplx, b->mixed, L, w);
-        if (g.ok) cands.push_back(g);
-      }
-    // the vector-load kernel for real FP32 element matrices with n = 4k
-    if (b->mixed && !c.kcplx && c.slotBytes == 1 && c.n % 4 == 0 && c.n <= 32)
-      for (int w : {4, 8}) {
-        GatherShape g = gatherShapeV4(c.n, c.maxRowLen, w);
-        if (g.ok) cands.push_back(g);
-      }
+    for (int w : {4, 8}) {
+      GatherShape g = gatherShape(J0.p, c.maxRowLen, c.kcplx, b->mixed, J0.lay, w);
+      if (g.ok) cands.push_back(g);
+    }
     if (cands.empty()) cands.push_back(base);
     float best = 1e30f;
     GatherShape bestShape = cands[0];
@@ -325,8 +320,8 @@ int tune(fg_batch *b, cudaStream_t s) {
     if ((st = uploadJobs(c, s))) return st;
     js += std::string(ci ? ", " : "") + "{\"dim\": " + std::to_string(c.dim) + ", \"n\": " + std::to_string(c.n) +
           ", \"nq\": " + std::to_string(c.nq) + ", \"problems\": " + std::to_string(c.probs.size()) +
-          ", \"lanes\": " + std::to_string(c.shape.L) + ", \"columns\": " + std::to_string(c.shape.J) +
-          ", \"vector_loads\": " + std::string(c.shape.v4 ? "true" : "false") +
+          ", \"lanes\": " + std::to_string(c.shape.lanes.L) + ", \"columns\": " + std::to_string(c.shape.J * c.shape.VW) +
+          ", \"vector_loads\": " + std::string(c.shape.VW == 4 && !c.shape.blocks3 ? "true" : "false") +
           ", \"warps\": " + std::to_string(c.shape.wpb) +
           ", \"ms\": " + std::to_string(best) + "}";
   }
@@ -487,11 +482,6 @@ extern "C" int fg_batch_create(fg_plan *const *plans, const fg_term_desc *const 
     c.maxRowLen = std::max(c.maxRowLen, p.maxRowLen);
   }
   for (auto &c : b->classes) {
-    c.shape = gatherShape(c.n, c.maxRowLen, c.kcplx, b->mixed, 0, 0);
-    if (!c.shape.ok) {
-      setLastError("fg_batch_create: CSR row too long for the shared-memory accumulator");
-      return fail(FG_ERR_UNSUPPORTED);
-    }
     if (cudaMalloc(&c.jobsDev, c.probs.size() * sizeof(GatherJob)) != cudaSuccess) return fail(FG_ERR_OOM);
     if (cudaMallocHost(&c.jobsHost, c.probs.size() * sizeof(GatherJob)) != cudaSuccess) return fail(FG_ERR_OOM);
     std::memset(c.jobsHost, 0, c.probs.size() * sizeof(GatherJob));
@@ -504,6 +494,11 @@ extern "C" int fg_batch_create(fg_plan *const *plans, const fg_term_desc *const 
       J.ke = b->mixed ? (const void *)mixedKe(pl, &J.lay) : (const void *)pl->ke;
       J.be = b->source[q] ? (const double2 *)pl->be : nullptr;
       J.uD = nullptr;
+    }
+    c.shape = gatherShape(c.jobsHost[0].p, c.maxRowLen, c.kcplx, b->mixed, c.jobsHost[0].lay, 0);
+    if (!c.shape.ok) {
+      setLastError("fg_batch_create: CSR row too long for the shared-memory accumulator");
+      return fail(FG_ERR_UNSUPPORTED);
     }
     layoutClass(b, c);
   }

@@ -140,7 +140,9 @@ struct PlanDev {
   const uint64_t *rowPtr; // [nRows+1] into rowElem
   const uint32_t *rowElem;// (e << 6) | i : element and local test index
   const uint4 *visit;      // per visited row: row, CSR start, element-list start, len | count << 16
-  const uint32_t *visitElem;// element lists in visiting order
+  const uint8_t *rec;       // records of the element lists in visiting order: (e << 6) | i, then the slots
+  int32_t recLd;            // bytes of a record
+  int32_t cleanSlots;       // 1: every slot is a column of the row (none fixed, none ignored)
   const void *slot;       // [E][n][slotLd] uint8 or uint16 position in the row
   int32_t slotBytes;
   int32_t slotLd;         // slot row stride (entries)
@@ -173,8 +175,6 @@ struct fg_plan {
   // row ranges of the gather's visiting order ([k] .. [k + 1]), copied out
   // one by one when the CSR values go to the host
   std::vector<uint64_t> outChunkRow;
-  const uint4 *visitRanged = nullptr;         // the visit tables in range-major order
-  const uint32_t *visitElemRanged = nullptr;
   cudaStream_t copyStream = nullptr;
   std::vector<cudaEvent_t> copyEvents;
   // owned device allocations
@@ -290,18 +290,29 @@ struct GatherJob {
   KeLayout lay;
   int64_t blockStart, nBlocks;
 };
+// Lanes of the reduction: L per CSR row, R rows per warp (R * L <= 32), OL =
+// 2^lgOL lanes writing a finished row
+struct GatherLanes {
+  int32_t L = 0, R = 0, OL = 0, lgOL = 0;
+};
+constexpr int kGatherWarpsPerSm = 64;  // of a reduction's grid
 struct GatherShape {
-  int L = 0, J = 3, wpb = 0, rowsPerBlock = 0;  // lanes per row, columns per lane
+  GatherLanes lanes;
+  int VW = 1, J = 3;  // columns per load, loads per lane and element row
+  bool blocks3 = false;  // 3x3 component blocks (kKeBlocks3)
+  int wpb = 0, rowsPerBlock = 0;
   size_t smem = 0;
   bool ok = false;
-  bool v4 = false;  // k_gather_batch_v4: L = n / 4 lanes, 4 columns each by vector loads
 };
-// L, wpb <= 0: the defaults of the single-plan gather
-GatherShape gatherShape(int n, int maxRowLen, int kcplx, int keIsFloat, int L, int wpb);
-// the vector-load shape (real FP32 element matrices, n a multiple of 4 up to 32)
-GatherShape gatherShapeV4(int n, int maxRowLen, int wpb);
+// wpb (warps per block) <= 0: the default
+GatherShape gatherShape(const PlanDev &p, int maxRowLen, int kcplx, int keIsFloat, KeLayout lay, int wpb);
+// whether the reduction's hot kernel (gather.cuh, SIMPLE) applies to real element matrices
+inline bool gatherSimple(const PlanDev &p, const void *be) { return p.cleanSlots && p.plainSlots && !p.lscale && !be; }
+// the records of the visiting order, from its (element, local row) list
+int buildRecords(const PlanDev &p, const uint32_t *visitElem, int64_t entries, uint32_t *rec);
+// simple: gatherSimple() of every job
 int launchGatherBatch(const GatherJob *jobsDev, int nJobs, int64_t blocks, int slotBytes, int kcplx, int keIsFloat,
-                      const GatherShape &g, cudaStream_t s);
+                      const GatherShape &g, bool simple, cudaStream_t s);
 
 // One problem (element bucket) of a tensor-core contraction launch
 struct GemmProblem {
@@ -366,26 +377,25 @@ __device__ inline double2 cdiv(double2 a, double2 b) {
 
 // Exact FP32 -> FP64 widening with integer operations. The F2F instruction
 // runs on the FP64 pipe, which is narrow on GB300; the bit manipulation runs
-// on the integer pipes. Handles zeros, subnormals, infinities and NaNs.
+// on the integer pipes. A normal number takes a shift and an add (1023 - 127
+// = 896 more in the exponent); zeros, subnormals, infinities and NaNs (an
+// exponent of all zeros or ones) go the long way.
+static __device__ __noinline__ double widenSpecial(uint32_t b) {
+  const uint64_t sign = (uint64_t)(b & 0x80000000u) << 32;
+  uint32_t man = b & 0x7FFFFFu;
+  const uint32_t ex = b >> 23 & 0xFFu;
+  if (ex != 0 && ex != 0xFFu) return __longlong_as_double((long long)(sign | ((uint64_t)(ex + 896u) << 52) | ((uint64_t)man << 29)));
+  if (ex == 0xFFu) return __longlong_as_double((long long)(sign | (0x7FFull << 52) | ((uint64_t)man << 29)));
+  if (man == 0) return __longlong_as_double((long long)sign);
+  // subnormal: value = man * 2^-149; normalise the leading one to bit 23
+  const int lz = __clz(man) - 8;  // shift that brings the leading one to bit 23
+  man = (man << lz) & 0x7FFFFFu;
+  return __longlong_as_double((long long)(sign | ((uint64_t)(897 - lz) << 52) | ((uint64_t)man << 29)));
+}
 __device__ inline double widen(float x) {
   const uint32_t b = __float_as_uint(x);
-  const uint64_t sign = (uint64_t)(b & 0x80000000u) << 32;
-  const uint32_t ex = (b >> 23) & 0xFFu;
-  uint32_t man = b & 0x7FFFFFu;
-  uint64_t bits;
-  if (ex == 0xFFu) {
-    bits = sign | (0x7FFull << 52) | ((uint64_t)man << 29);
-  } else if (ex != 0) {
-    bits = sign | ((uint64_t)(ex + 896u) << 52) | ((uint64_t)man << 29);  // 1023 - 127 = 896
-  } else if (man == 0) {
-    bits = sign;
-  } else {
-    // subnormal: value = man * 2^-149; normalise the leading one to bit 23
-    const int lz = __clz(man) - 8;  // shift that brings the leading one to bit 23
-    man = (man << lz) & 0x7FFFFFu;
-    bits = sign | ((uint64_t)(897 - lz) << 52) | ((uint64_t)man << 29);
-  }
-  return __longlong_as_double((long long)bits);
+  if (((b + 0x00800000u) & 0x7F000000u) == 0) return widenSpecial(b);
+  return __hiloint2double((int)((((int)b >> 3) & 0x8FFFFFFF) + 0x38000000), (int)(b << 29));
 }
 __device__ inline double widen(double x) { return x; }
 

@@ -1,0 +1,19 @@
+// Instances of the CSR reduction for FP64 element matrices.
+#include "gather.cuh"
+
+namespace femg {
+
+template <typename SlotT, bool KCPLX>
+static int pick(const GatherLaunch &a) {
+  const GatherShape &g = a.g;
+  if (g.VW == 2)
+    return g.J == 1 ? launchGatherShape<SlotT, KCPLX, double, 2, 1, false>(a) : launchGatherShape<SlotT, KCPLX, double, 2, 3, false>(a);
+  return g.J == 3 ? launchGatherShape<SlotT, KCPLX, double, 1, 3, false>(a) : launchGatherShape<SlotT, KCPLX, double, 1, 5, false>(a);
+}
+
+int launchGatherF64(const GatherLaunch &a) {
+  if (a.slotBytes == 1) return a.kcplx ? pick<uint8_t, true>(a) : pick<uint8_t, false>(a);
+  return a.kcplx ? pick<uint16_t, true>(a) : pick<uint16_t, false>(a);
+}
+
+}  // namespace femg

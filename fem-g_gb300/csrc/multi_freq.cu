@@ -15,229 +15,57 @@
 // and right-hand side (sources, plus the Dirichlet lifting of each group
 // scaled the same way). The reduction visits the element rows in the order
 // of the single-frequency gather, so each group sum is deterministic.
+#include <algorithm>
 #include <cstring>
 #include <functional>
 
-#include "common.cuh"
+#include "multi_gather.cuh"
 
 namespace femg {
-
-constexpr int kMaxGroups = 3;
-constexpr int kMaxFreq = 64;
-
-struct MultiIn {
-  const void *ke[kMaxGroups];    // element matrices of group g (KT)
-  int64_t stride[kMaxGroups];    // KT entries from one element to the next
-  int cplx[kMaxGroups];          // group g has an imaginary part (at +n*n)
-  int realFactor[kMaxGroups];    // the factors of group g are real for every output
-  int imagFactor[kMaxGroups];    // ... purely imaginary for every output
-  int G, F, R;
-  int anyCplx;                   // some group has an imaginary part: two accumulators per group and slot, else one
-  KeLayout lay;                  // element-matrix layout (ld entries per component)
-  const double2 *coef;           // [F][G] factors of the value arrays
-  const double2 *rcoef;          // [R][G] factors of the liftings in the right-hand sides
-  const double2 *be;             // [E][n] element right-hand sides or null
-  const double2 *uD;             // Dirichlet values or null
-  double2 *const *values;        // F value arrays [nnz] (device table)
-  double2 *const *rhs;           // R right-hand sides [nRows] (device table), or null
-};
-
-template <typename SlotT, typename KT, int L, int J>
-__global__ void __launch_bounds__(256)
-    k_gather_multi(const PlanDev p, const MultiIn in, int rowsPerBlock) {
-  using AT = KT;
-  constexpr int R = 32 / L;  // rows per warp; J columns per lane (L * J >= n)
-  const int G = in.G, F = in.F;
-  auto keOff = [&](int ii, int jj) -> int { return keOffset(in.lay, p.n, ii, jj); };
-  extern __shared__ __align__(16) unsigned char smraw[];
-  AT *cf = reinterpret_cast<AT *>(smraw);  // [F][G][2] factors in the accumulation type
-  for (int k = threadIdx.x; k < F * G; k += blockDim.x) {
-    cf[2 * k] = (AT)in.coef[k].x;
-    cf[2 * k + 1] = (AT)in.coef[k].y;
-  }
-  __syncthreads();
-  const size_t cfBytes = ((size_t)F * G * 2 * sizeof(AT) + 15) / 16 * 16;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int sub = lane / L, lt = lane % L;
-  // accumulators per slot: (re, im) per group when some group is complex,
-  // else one real sum per group
-  const int perSlot = in.anyCplx ? 2 * G : G;
-  const int gStep = in.anyCplx ? 2 : 1;
-  AT *A = reinterpret_cast<AT *>(smraw + cfBytes) + (size_t)(warp * R + sub) * p.maxRowLen * perSlot;
-  const SlotT *slot = (const SlotT *)p.slot;
-  const SlotT kFixed = (SlotT)(sizeof(SlotT) == 1 ? 0xFF : kSlotFixed);
-  const SlotT kIgnore = (SlotT)(sizeof(SlotT) == 1 ? 0xFE : kSlotIgnore);
-  const int n = p.n;
-  const int nn2 = in.lay.ld;  // entries per component
-  const int64_t nRows = (int64_t)p.nRows;
-  const int64_t stride = (int64_t)gridDim.x * rowsPerBlock;
-  for (int64_t base = (int64_t)blockIdx.x * rowsPerBlock + warp * R; base < nRows; base += stride) {
-    const int64_t idx = base + sub;
-    const bool live = idx < nRows;
-    const uint4 v = live ? p.visit[idx] : make_uint4(0, 0, 0, 0);
-    const int64_t row = v.x;
-    const uint64_t start = v.y;
-    const int len = live ? (int)(v.w & 0xFFFFu) : 0;
-    const uint64_t r0 = v.z;
-    const int cnt = live ? (int)(v.w >> 16) : 0;
-    for (int s = lt; s < len * perSlot; s += L) A[s] = (AT)0;
-    int maxCnt = cnt;
-#pragma unroll
-    for (int off = L; off < 32; off <<= 1) maxCnt = max(maxCnt, __shfl_xor_sync(0xffffffffu, maxCnt, off));
-    __syncwarp();
-    double2 dc[kMaxGroups];
-#pragma unroll
-    for (int g = 0; g < kMaxGroups; ++g) dc[g] = make_double2(0.0, 0.0);
-    double2 bsum = make_double2(0.0, 0.0);
-    for (int k = 0; k < maxCnt; ++k) {
-      if (k < cnt) {
-        const uint32_t packed = p.visitElem[r0 + k];
-        const int64_t e = packed >> 6;
-        const int i = packed & 63;
-        const SlotT *S = slot + ((size_t)e * n + i) * p.slotLd;
-        if (in.be && lt == 0) bsum = cadd(bsum, in.be[e * n + i]);
-#pragma unroll
-        for (int jj = 0; jj < J; ++jj) {
-          const int j = lt + L * jj;
-          if (j >= n) continue;
-          const SlotT s = S[j];
-          if (s == kIgnore) continue;
-          if (s != kFixed) {
-            const int o = keOff(i, j);
-#pragma unroll
-            for (int g = 0; g < kMaxGroups; ++g) {
-              if (g >= G) break;
-              const KT *K = (const KT *)in.ke[g] + e * in.stride[g];
-              // distinct slots per lane within an element row; rows are
-              // separated by the __syncwarp below, so the adds are ordered
-              atomicAdd(&A[(int)s * perSlot + gStep * g], (AT)K[o]);
-              if (in.cplx[g]) atomicAdd(&A[(int)s * perSlot + gStep * g + 1], (AT)K[nn2 + o]);
-            }
-          } else {
-            // lifting with the transposed entry (VectorFactory::addValuesDC)
-            const int o = keOff(j, i);
-            const double2 u = in.uD[p.edof[e * n + j]];
-#pragma unroll
-            for (int g = 0; g < kMaxGroups; ++g) {
-              if (g >= G) break;
-              const KT *K = (const KT *)in.ke[g] + e * in.stride[g];
-              const double2 kv = make_double2((double)K[o], in.cplx[g] ? (double)K[nn2 + o] : 0.0);
-              dc[g] = cadd(dc[g], cmul(kv, u));
-            }
-          }
-        }
-      }
-      __syncwarp();
-    }
-    for (int s = lt; s < len; s += L) {
-      AT ar[kMaxGroups], ai[kMaxGroups];
-#pragma unroll
-      for (int g = 0; g < kMaxGroups; ++g) {
-        ar[g] = g < G ? A[s * perSlot + gStep * g] : (AT)0;
-        ai[g] = (g < G && in.cplx[g]) ? A[s * perSlot + gStep * g + 1] : (AT)0;
-      }
-      for (int f = 0; f < F; ++f) {
-        AT re = (AT)0, im = (AT)0;
-#pragma unroll
-        for (int g = 0; g < kMaxGroups; ++g) {
-          if (g >= G) break;
-          const AT cr = cf[2 * (f * G + g)], ci = cf[2 * (f * G + g) + 1];
-          // real sums and real or imaginary factors (the usual case) skip the
-          // zero products: they cost FP64 issue slots on the FP64 path
-          if (in.realFactor[g]) re += cr * ar[g];
-          else if (in.imagFactor[g]) im += ci * ar[g];
-          else {
-            re += cr * ar[g];
-            im += ci * ar[g];
-          }
-          if (in.cplx[g]) {
-            re -= ci * ai[g];
-            im += cr * ai[g];
-          }
-        }
-        in.values[f][start + s] = make_double2(widen(re), widen(im));
-      }
-    }
-    if (in.rhs) {
-      if (in.uD) {
-#pragma unroll
-        for (int g = 0; g < kMaxGroups; ++g)
-#pragma unroll
-          for (int off = L / 2; off > 0; off >>= 1) {
-            dc[g].x += __shfl_down_sync(0xffffffffu, dc[g].x, off, L);
-            dc[g].y += __shfl_down_sync(0xffffffffu, dc[g].y, off, L);
-          }
-      }
-      if (live && lt == 0)
-        for (int r = 0; r < in.R; ++r) {
-          double2 v = bsum;
-#pragma unroll
-          for (int g = 0; g < kMaxGroups; ++g)
-            if (g < G) v = cadd(v, cmul(in.rcoef[r * G + g], dc[g]));
-          in.rhs[r][row] = v;
-        }
-    }
-    __syncwarp();
-  }
-}
-
-template <typename SlotT, typename KT>
-static int launchMultiTyped(const PlanDev &p, const MultiIn &in, cudaStream_t s) {
-  // three columns per lane: the 8 x 5 shape of the single-frequency
-  // reduction measured 43% slower here (complex accumulators per group, and
-  // 16 frequencies written per row)
-  const int n = p.n;
-  int L = 32;
-  if (n <= 6) L = 2;
-  else if (n <= 12) L = 4;
-  else if (n <= 24) L = 8;
-  else if (n <= 48) L = 16;
-  const int J = 3;
-  const int R = 32 / L;
-  const size_t cfBytes = ((size_t)in.F * in.G * 2 * sizeof(KT) + 15) / 16 * 16;
-  const size_t rowBytes = (size_t)std::max(p.maxRowLen, 1) * (in.anyCplx ? 2 : 1) * in.G * sizeof(KT);
-  int wpb = 8;
-  while (wpb > 1 && cfBytes + rowBytes * R * wpb > 200 * 1024) wpb >>= 1;
-  const size_t smem = cfBytes + rowBytes * R * wpb;
-  if (smem > 200 * 1024) {
-    setLastError("multi-frequency gather: CSR row too long for shared memory");
-    return FG_ERR_UNSUPPORTED;
-  }
-  const int rowsPerBlock = wpb * R;
-  int64_t blocks = ((int64_t)p.nRows + rowsPerBlock - 1) / rowsPerBlock;
-  blocks = std::min<int64_t>(blocks, (int64_t)smCount() * 16);
-  bool launched = false;
-#define FG_MULTI_L(LL, JJ)                                                                         \
-  if (L == LL && J == JJ) {                                                                        \
-    launched = true;                                                                               \
-    auto kern = k_gather_multi<SlotT, KT, LL, JJ>;                                                 \
-    static SmemAllowance allowed;                                                                                \
-    FG_CUDA(allowSmem(kern, smem, allowed));                                                                      \
-    kern<<<(unsigned)blocks, 32 * wpb, smem, s>>>(p, in, rowsPerBlock);                            \
-  }
-  FG_MULTI_L(2, 3)
-  FG_MULTI_L(4, 3)
-  FG_MULTI_L(8, 3)
-  FG_MULTI_L(8, 5)
-  FG_MULTI_L(16, 3)
-  FG_MULTI_L(32, 3)
-#undef FG_MULTI_L
-  if (!launched) {
-    setLastError("multi-frequency gather: no kernel for this (lanes, columns) shape");
-    return FG_ERR_UNSUPPORTED;
-  }
-  FG_CUDA(cudaGetLastError());
-  return FG_OK;
-}
 
 static int launchGatherMulti(fg_plan *plan, const MultiIn &in, bool isFloat, cudaStream_t s) {
   const PlanDev &p = plan->d;
   if (p.nRows == 0) return FG_OK;
+  MultiLaunch a;
+  a.in = in;
+  a.p = &p;
+  a.s = s;
+  // the single-frequency shape of one group; several groups' sums take as
+  // many times the shared memory, and complex groups come column by column
+  // (VW = 1), which keeps the rare kernels few
+  a.g = gatherShape(p, p.maxRowLen, 0, isFloat, in.lay, 8);
+  GatherShape &g = a.g;
+  if (in.anyCplx) {
+    const int nb = g.blocks3 ? p.nc / 3 : p.nc;
+    g.VW = 1;
+    g.J = g.blocks3 || nb <= 24 ? 3 : 5;
+    g.lanes.L = g.blocks3 ? nb : (nb + g.J - 1) / g.J;
+    g.lanes.R = 32 / g.lanes.L;
+  }
+  const size_t size = isFloat ? 4 : 8;
+  const size_t cfBytes = (size_t)multiHeadBytes(in.F, in.G, (int)size);
+  const size_t rowBytes = (size_t)std::max(p.maxRowLen, 1) * (in.anyCplx ? 2 : 1) * in.G * size;
+  // a row of the visiting order has to fit with this many rows per warp
+  const int limit = p.n <= 6 ? 16 : p.n <= 12 ? 8 : p.n <= 24 ? 4 : p.n <= 48 ? 2 : 1;
+  if ((size_t)multiFactorBytes(in.F, in.G, (int)size) + rowBytes * limit > 200 * 1024) {
+    setLastError("multi-frequency gather: CSR row too long for shared memory");
+    return FG_ERR_UNSUPPORTED;
+  }
+  // measured on 48,000 order-2 Navier tetrahedra at 8 frequencies: 0.599 ms
+  // with 4 warps and 32 lanes writing a row, 0.608 with 8 warps, 0.631 with 16
+  // lanes, 0.678 and 0.794 with 4 and 2 rows per warp in place of 6
+  g.wpb = 4;
+  g.lanes.lgOL = 5;
+  g.lanes.OL = 32;
+  while (g.lanes.R > 1 && cfBytes + rowBytes * g.lanes.R * g.wpb > 100 * 1024) --g.lanes.R;
+  while (g.wpb > 1 && cfBytes + rowBytes * g.lanes.R * g.wpb > 200 * 1024) g.wpb >>= 1;  // (a block may hold 227 KB)
+  g.smem = cfBytes + rowBytes * g.lanes.R * g.wpb;
+  g.rowsPerBlock = g.wpb * g.lanes.R;
+  const int64_t groups = ((int64_t)p.nRows + g.rowsPerBlock - 1) / g.rowsPerBlock;
+  a.blocks = std::min<int64_t>(groups, (int64_t)smCount() * kGatherWarpsPerSm / g.wpb);
   ProfScope prof("k_gather_multi", s);
   countLaunch();
-  if (p.slotBytes == 1)
-    return isFloat ? launchMultiTyped<uint8_t, float>(p, in, s) : launchMultiTyped<uint8_t, double>(p, in, s);
-  return isFloat ? launchMultiTyped<uint16_t, float>(p, in, s) : launchMultiTyped<uint16_t, double>(p, in, s);
+  return isFloat ? launchMultiF32(a) : launchMultiF64(a);
 }
 
 struct MultiState {
@@ -377,6 +205,8 @@ int runGroups(fg_plan *plan, const fg_term_desc *terms, int32_t n_terms, int32_t
     in.realFactor[g] = re;
     in.imagFactor[g] = im && !re;
   }
+  in.allReal = 1;
+  for (int g = 0; g < G; ++g) in.allReal = in.allReal && in.realFactor[g];
   in.R = anyRhs ? R : 0;
   in.coef = m->coef;
   in.rcoef = m->coef + (size_t)kMaxFreq * kMaxGroups;

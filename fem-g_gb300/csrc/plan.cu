@@ -333,13 +333,11 @@ static int createPlan(const fg_mesh_desc *mesh, const fg_rule_desc *rule, const 
       }
   }
 
-  // gather visiting orders, rows grouped by contribution count (stable):
-  // over all rows (rowOrder, for device outputs), and within kOutChunks
-  // consecutive row ranges (rowOrderRanged, for host outputs: the visit
-  // indices of a range are its rows' indices, so the CSR slice of a range is
-  // complete once its part of the order has run, and can be copied out while
-  // the next range reduces)
-  std::vector<uint32_t> rowOrder(sys->n_rows), rowOrderRanged;
+  // gather visiting order: rows grouped by contribution count (stable) within
+  // kOutChunks consecutive row ranges. The visit indices of a range are its
+  // rows' indices, so the CSR slice of a range is complete once its part of
+  // the order has run, and can be copied to the host while the next reduces.
+  std::vector<uint32_t> rowOrder(sys->n_rows);
   const int nChunks = sys->n_rows >= (uint64_t)kOutChunks * 4096 ? kOutChunks : 1;
   {
     plan->outChunkRow.assign((size_t)nChunks + 1, 0);
@@ -347,18 +345,14 @@ static int createPlan(const fg_mesh_desc *mesh, const fg_rule_desc *rule, const 
     uint64_t maxCnt = 0;
     for (uint64_t r = 0; r < sys->n_rows; ++r) maxCnt = std::max(maxCnt, rowPtr[r + 1] - rowPtr[r]);
     std::vector<uint64_t> bucket(maxCnt + 2);
-    auto countSort = [&](uint64_t ra, uint64_t rb, std::vector<uint32_t> &order) {
+    auto countSort = [&](uint64_t ra, uint64_t rb) {
       std::fill(bucket.begin(), bucket.end(), 0);
       bucket[0] = ra;
       for (uint64_t r = ra; r < rb; ++r) bucket[rowPtr[r + 1] - rowPtr[r] + 1]++;
       for (uint64_t k = 0; k <= maxCnt; ++k) bucket[k + 1] += bucket[k];
-      for (uint64_t r = ra; r < rb; ++r) order[bucket[rowPtr[r + 1] - rowPtr[r]]++] = (uint32_t)r;
+      for (uint64_t r = ra; r < rb; ++r) rowOrder[bucket[rowPtr[r + 1] - rowPtr[r]]++] = (uint32_t)r;
     };
-    countSort(0, sys->n_rows, rowOrder);
-    if (nChunks > 1) {
-      rowOrderRanged.resize(sys->n_rows);
-      for (int c = 0; c < nChunks; ++c) countSort(plan->outChunkRow[(size_t)c], plan->outChunkRow[(size_t)c + 1], rowOrderRanged);
-    }
+    for (int c = 0; c < nChunks; ++c) countSort(plan->outChunkRow[(size_t)c], plan->outChunkRow[(size_t)c + 1]);
   }
   if (sys->n_rows >= (uint64_t(1) << 32) || d.nnz >= (uint64_t(1) << 32) || rowElem.size() >= (uint64_t(1) << 32)) {
     setLastError("fg_plan_create: more than 2^32 rows, nonzeros or element rows in one plan");
@@ -367,29 +361,22 @@ static int createPlan(const fg_mesh_desc *mesh, const fg_rule_desc *rule, const 
   // visit table: one 16-byte record per row in visiting order (row, CSR
   // start, start of its element list, length | count << 16), the element
   // lists stored contiguously in that order
-  std::vector<uint4> visit(sys->n_rows), visitRanged;
-  std::vector<uint32_t> visitElem(rowElem.size()), visitElemRanged;
-  auto buildVisit = [&](const std::vector<uint32_t> &order, std::vector<uint4> &vis, std::vector<uint32_t> &visElem) -> int {
+  std::vector<uint4> visit(sys->n_rows);
+  std::vector<uint32_t> visitElem(rowElem.size());
+  {
     uint64_t pos = 0;
     for (uint64_t v = 0; v < sys->n_rows; ++v) {
-      const uint32_t r = order[v];
+      const uint32_t r = rowOrder[v];
       const uint64_t cnt = rowPtr[r + 1] - rowPtr[r];
       const uint64_t len = sys->ai[r + 1] - sys->ai[r];
       if (cnt > 0xFFFF || len > 0xFFFF) {
         setLastError("fg_plan_create: row with more than 65535 entries or contributions");
         return FG_ERR_UNSUPPORTED;
       }
-      std::copy(rowElem.begin() + (int64_t)rowPtr[r], rowElem.begin() + (int64_t)rowPtr[r + 1], visElem.begin() + (int64_t)pos);
-      vis[v] = make_uint4(r, (uint32_t)sys->ai[r], (uint32_t)pos, (uint32_t)(len | (cnt << 16)));
+      std::copy(rowElem.begin() + (int64_t)rowPtr[r], rowElem.begin() + (int64_t)rowPtr[r + 1], visitElem.begin() + (int64_t)pos);
+      visit[v] = make_uint4(r, (uint32_t)sys->ai[r], (uint32_t)pos, (uint32_t)(len | (cnt << 16)));
       pos += cnt;
     }
-    return FG_OK;
-  };
-  if (int st0 = buildVisit(rowOrder, visit, visitElem)) return st0;
-  if (nChunks > 1) {
-    visitRanged.resize(sys->n_rows);
-    visitElemRanged.resize(rowElem.size());
-    if (int st0 = buildVisit(rowOrderRanged, visitRanged, visitElemRanged)) return st0;
   }
 
   // slots: position of each column inside its row
@@ -411,8 +398,9 @@ static int createPlan(const fg_mesh_desc *mesh, const fg_rule_desc *rule, const 
   std::vector<uint8_t> slot8;
   std::vector<uint16_t> slot16;
   if (narrow) slot8.assign(nSlots, 0xFF); else slot16.assign(nSlots, kSlotIgnore);
+  int open = 0;  // some column of an element row is fixed or not stored
   int dup = 0;  // elements with two row columns on one DOF, or slots taken from the upper-storage lower_bound
-#pragma omp parallel for schedule(dynamic, 256) reduction(+ : bad, dup)
+#pragma omp parallel for schedule(dynamic, 256) reduction(+ : bad, dup) reduction(| : open)
   for (int64_t e = 0; e < E; ++e) {
     {
       uint32_t cols[64];
@@ -450,6 +438,7 @@ static int createPlan(const fg_mesh_desc *mesh, const fg_rule_desc *rule, const 
             s = kSlotIgnore;
           }
         }
+        open |= s == kSlotFixed || s == kSlotIgnore;
         const size_t ks = ki * nS + j;
         if (narrow) slot8[ks] = s == kSlotFixed ? 0xFF : (s == kSlotIgnore ? 0xFE : (uint8_t)s);
         else slot16[ks] = s;
@@ -461,6 +450,7 @@ static int createPlan(const fg_mesh_desc *mesh, const fg_rule_desc *rule, const 
     return FG_ERR_INDEX;
   }
   d.plainSlots = dup == 0;
+  d.cleanSlots = open == 0;
   if (nS > nc)
     for (size_t r = 0; r < (size_t)E * n; ++r)
       std::fill(slot8.begin() + (int64_t)(r * nS + nc), slot8.begin() + (int64_t)((r + 1) * nS), (uint8_t)0xFE);
@@ -510,13 +500,6 @@ static int createPlan(const fg_mesh_desc *mesh, const fg_rule_desc *rule, const 
   if ((st = upload(plan, rowPtr.data(), rowPtr.size(), &d.rowPtr))) return st;
   if ((st = upload(plan, rowElem.data(), rowElem.size(), &d.rowElem))) return st;
   if ((st = upload(plan, visit.data(), visit.size(), &d.visit))) return st;
-  if ((st = upload(plan, visitElem.data(), visitElem.size(), &d.visitElem))) return st;
-  plan->visitRanged = d.visit;
-  plan->visitElemRanged = d.visitElem;
-  if (nChunks > 1) {
-    if ((st = upload(plan, visitRanged.data(), visitRanged.size(), &plan->visitRanged))) return st;
-    if ((st = upload(plan, visitElemRanged.data(), visitElemRanged.size(), &plan->visitElemRanged))) return st;
-  }
   if (narrow) {
     const uint8_t *p;
     if ((st = upload(plan, slot8.data(), slot8.size(), &p))) return st;
@@ -525,6 +508,32 @@ static int createPlan(const fg_mesh_desc *mesh, const fg_rule_desc *rule, const 
     const uint16_t *p;
     if ((st = upload(plan, slot16.data(), slot16.size(), &p))) return st;
     d.slot = p;
+  }
+  // the slots once more, per list entry in visiting order
+  d.recLd = (nc * d.slotBytes + 3) / 4 * 4 + 4;
+  if (!visitElem.empty()) {
+    uint32_t *list = nullptr;
+    void *rec = nullptr;
+    if (cudaMalloc(&rec, visitElem.size() * (size_t)d.recLd) != cudaSuccess) {
+      cudaGetLastError();
+      setLastError("fg_plan_create: device allocation of the reduction records failed");
+      return FG_ERR_OOM;
+    }
+    plan->allocs.push_back(rec);
+    d.rec = (const uint8_t *)rec;
+    if (cudaMalloc(&list, visitElem.size() * 4) != cudaSuccess) {
+      cudaGetLastError();
+      setLastError("fg_plan_create: device allocation of the element lists failed");
+      return FG_ERR_OOM;
+    }
+    st = cudaMemcpy(list, visitElem.data(), visitElem.size() * 4, cudaMemcpyHostToDevice) == cudaSuccess
+             ? buildRecords(d, list, (int64_t)visitElem.size(), (uint32_t *)rec)
+             : FG_ERR_CUDA;
+    cudaFree(list);
+    if (st) {
+      if (st == FG_ERR_CUDA) setLastError("fg_plan_create: building the reduction records failed");
+      return st;
+    }
   }
   if (linked) {
     std::vector<double2> ls((size_t)E * n, make_double2(1.0, 0.0));
