@@ -34,7 +34,7 @@ namespace femg {
 
 constexpr int kQuadThreads = 128;
 constexpr int kQuadMaxElems = 64;             // elements per block
-constexpr size_t kQuadSmem = 47 * 1024;       // shared memory of a block: no opt-in, room for the tables in L1 at three blocks per SM
+constexpr size_t kQuadSmem = 30 * 1024;       // shared memory of a block: seven blocks per SM
 constexpr int kQuadGeom = 31;                 // per element: J, J^-1, det, det J^-1 J^-T, J^T J / det (HCurl)
 
 // Shape and switches of one launch
@@ -44,6 +44,7 @@ struct QuadArgs {
   int nEnt;        // entries accumulated per element: the upper triangle, or all n x nc
   int comps;       // mask of the table components that contribute (see tableComps)
   int uniform;     // the scalar bilinear coefficients are constant on each element
+  int realSource;  // the scalar sources are real
   int needX;       // some coefficient or modificator reads the physical point
 };
 
@@ -91,6 +92,9 @@ __host__ __device__ inline QuadLayout quadLayout(int NE, int QD, int QC, int nn,
 __device__ __noinline__ double2 evalExprCall(const DevExpr *ex, int64_t e, const double *x, const double *phi, int nb, int q, int nq) {
   return evalExpr(*ex, e, x, phi, nb, q, nq);
 }
+__device__ __noinline__ double evalRealCall(const DevExpr *ex, int64_t e, const double *x, const double *phi, int nb, int q, int nq) {
+  return evalExprReal(*ex, e, x, phi, nb, q, nq);
+}
 struct CoefPoint {
   int64_t e;
   const double *x, *phi;
@@ -98,7 +102,15 @@ struct CoefPoint {
 };
 __device__ __forceinline__ double2 evalAt(const DevExpr &ex, const CoefPoint &c) {
   if (ex.cls == kExprConst) return ex.cval;
+  if (ex.real) return make_double2(evalRealCall(&ex, c.e, c.x, c.phi, c.nb, c.q, c.nq), 0.0);
   return evalExprCall(&ex, c.e, c.x, c.phi, c.nb, c.q, c.nq);
+}
+// a coefficient times its module factor; real ones, which are told apart by
+// their bits (a comparison of doubles would take the FP64 pipe), by one product
+__device__ __forceinline__ bool zeroBits(double x) { return (__double_as_longlong(x) << 1) == 0; }
+__device__ __forceinline__ double2 scaled(double2 factor, double2 v) {
+  if (zeroBits(factor.y) && zeroBits(v.y)) return make_double2(factor.x * v.x, 0.0);
+  return cmul(factor, v);
 }
 // A = c0 I + factor c D of tensor term `term` (coefTensor of common.cuh with
 // the shared interpreter)
@@ -115,9 +127,9 @@ __device__ inline void scalarCoefs(const DevTerms *terms, int g, const CoefPoint
   for (int t = 0; t < terms->n; ++t) {
     const DevTerm &T = terms->t[t];
     if (T.mod != g) continue;
-    if (T.kind == FG_TERM_GRAD_GRAD || T.kind == FG_TERM_ELASTIC) c[0] = cadd(c[0], cmul(T.factor, evalAt(T.coef, cp)));
-    else if (T.kind == FG_TERM_MASS) c[1] = cadd(c[1], cmul(T.factor, evalAt(T.coef, cp)));
-    if (T.kind == FG_TERM_ELASTIC) c[2] = cadd(c[2], cmul(T.factor, evalAt(T.coef2, cp)));
+    if (T.kind == FG_TERM_GRAD_GRAD || T.kind == FG_TERM_ELASTIC) c[0] = cadd(c[0], scaled(T.factor, evalAt(T.coef, cp)));
+    else if (T.kind == FG_TERM_MASS) c[1] = cadd(c[1], scaled(T.factor, evalAt(T.coef, cp)));
+    if (T.kind == FG_TERM_ELASTIC) c[2] = cadd(c[2], scaled(T.factor, evalAt(T.coef2, cp)));
   }
 }
 
@@ -148,6 +160,52 @@ __device__ inline void geomMaps(const double *J, double det, double *Ji, double 
   }
 }
 
+// The same from the nodes of a planar 2D element: J is [[a b 0], [c d 0],
+// [0 0 s]] with s = +-1 the normal, so no square root, and one division
+template <bool HCURL>
+__device__ inline double planarMaps(int nn, bool p1, const double *X, const double *dN, double *J, double *Ji, double *K6, double *M6) {
+  double a = 0.0, b = 0.0, c = 0.0, d = 0.0;  // dx/du dy/du dx/dv dy/dv
+  if (p1) {
+    a = X[3] - X[0];
+    b = X[4] - X[1];
+    c = X[6] - X[0];
+    d = X[7] - X[1];
+  } else {
+    for (int k = 0; k < nn; ++k) {
+      a += X[3 * k] * dN[3 * k];
+      b += X[3 * k + 1] * dN[3 * k];
+      c += X[3 * k] * dN[3 * k + 1];
+      d += X[3 * k + 1] * dN[3 * k + 1];
+    }
+  }
+  const double nz = a * d - b * c, s = copysign(1.0, nz), det = fabs(nz), id = 1.0 / det, sid = s * id;
+  for (int k = 0; k < 9; ++k) J[k] = Ji[k] = 0.0;
+  J[0] = a;
+  J[1] = b;
+  J[3] = c;
+  J[4] = d;
+  J[8] = s;
+  Ji[0] = d * sid;
+  Ji[1] = -c * sid;
+  Ji[3] = -b * sid;
+  Ji[4] = a * sid;
+  Ji[8] = s;
+  const double aa = a * a + b * b, cc = c * c + d * d, ac = a * c + b * d;  // J^T J
+  K6[0] = cc * id;
+  K6[1] = aa * id;
+  K6[2] = det;
+  K6[3] = -ac * id;
+  K6[4] = K6[5] = 0.0;
+  if (HCURL) {
+    M6[0] = aa * id;
+    M6[1] = cc * id;
+    M6[2] = id;
+    M6[3] = ac * id;
+    M6[4] = M6[5] = 0.0;
+  }
+  return det;
+}
+
 // Nodes and, for affine elements, the geometry of the block's elements
 // (J, J^-1, det, det J^-1 J^-T and J^T J / det)
 template <bool HCURL>
@@ -167,8 +225,13 @@ __device__ inline void quadElements(const PlanDev &p, const DevTerms *terms, int
     for (int t = threadIdx.x; t < live; t += kQuadThreads) {
       double *g = geom + t * kQuadGeom;
       double J[9], Ji[9];
-      const double det = p.p1geom ? jacobianP1(p.dim, X + t * p.nn * 3, J) : jacobian(p.dim, p.nn, X + t * p.nn * 3, p.geoGrad, J);
-      geomMaps<HCURL>(J, det, Ji, g + 19, g + 25);
+      double det;
+      if (p.planar) {
+        det = planarMaps<HCURL>(p.nn, p.p1geom != 0, X + t * p.nn * 3, p.geoGrad, J, Ji, g + 19, g + 25);
+      } else {
+        det = p.p1geom ? jacobianP1(p.dim, X + t * p.nn * 3, J) : jacobian(p.dim, p.nn, X + t * p.nn * 3, p.geoGrad, J);
+        geomMaps<HCURL>(J, det, Ji, g + 19, g + 25);
+      }
       for (int k = 0; k < 9; ++k) {
         g[k] = J[k];
         g[9 + k] = Ji[k];
@@ -179,45 +242,34 @@ __device__ inline void quadElements(const PlanDev &p, const DevTerms *terms, int
   }
 }
 
-// Geometry of one (element, point) for the terms of modificator group g:
-// from the element's where the Jacobian is constant, else formed here
-struct PointGeom {
-  double J[9], Ji[9], det;
-  double K6[6], M6[6];  // det J^-1 J^-T, J^T J / det
-  double x[3];
-};
+// Geometry of one (element, point) for the terms of modificator group g, laid
+// out as an element's: that one where the Jacobian is constant and
+// unmodified, else formed in `own`. x: the physical point.
+constexpr int kGeomJ = 0, kGeomJi = 9, kGeomDet = 18, kGeomK = 19, kGeomM = 25;
 template <bool HCURL>
-__device__ inline void quadPoint(const PlanDev &p, const DevTerms *terms, int g, int q, const double *X, const double *geom, bool needX,
-                                 PointGeom &P) {
-  P.x[0] = P.x[1] = P.x[2] = 0.0;
+__device__ inline const double *quadPoint(const PlanDev &p, const DevTerms *terms, int g, int q, const double *X, const double *geom,
+                                          bool needX, double *own, double *x) {
+  x[0] = x[1] = x[2] = 0.0;
   const DevJacMod &m = terms->mods[g];
   if (needX)
     for (int k = 0; k < p.nn; ++k) {
       const double v = p.geoVal[q * p.nn + k];
-      P.x[0] += v * X[3 * k];
-      P.x[1] += v * X[3 * k + 1];
-      P.x[2] += v * X[3 * k + 2];
+      x[0] += v * X[3 * k];
+      x[1] += v * X[3 * k + 1];
+      if (!p.planar || !zeroBits(X[2])) x[2] += v * X[3 * k + 2];
     }
-  if (p.affine && m.kind == FG_JACMOD_NONE) {
-    for (int k = 0; k < 9; ++k) {
-      P.J[k] = geom[k];
-      P.Ji[k] = geom[9 + k];
-    }
-    P.det = geom[18];
-    for (int k = 0; k < 6; ++k) {
-      P.K6[k] = geom[19 + k];
-      if (HCURL) P.M6[k] = geom[25 + k];
-    }
-    return;
-  }
+  if (p.affine && m.kind == FG_JACMOD_NONE) return geom;
+  double det;
   if (p.affine) {
-    for (int k = 0; k < 9; ++k) P.J[k] = geom[k];
-    P.det = geom[18];
+    for (int k = 0; k < 9; ++k) own[k] = geom[k];
+    det = geom[kGeomDet];
   } else {
-    P.det = jacobian(p.dim, p.nn, X, p.geoGrad + (size_t)q * p.nn * 3, P.J);
+    det = jacobian(p.dim, p.nn, X, p.geoGrad + (size_t)q * p.nn * 3, own);
   }
-  if (m.kind != FG_JACMOD_NONE && !applyJacMod(m, P.x, P.J, P.det)) atomicOr(p.jmErr, 1);
-  geomMaps<HCURL>(P.J, P.det, P.Ji, P.K6, P.M6);
+  if (m.kind != FG_JACMOD_NONE && !applyJacMod(m, x, own, det)) atomicOr(p.jmErr, 1);
+  geomMaps<HCURL>(own, det, own + kGeomJi, own + kGeomK, own + kGeomM);
+  own[kGeomDet] = det;
+  return own;
 }
 
 // Upper-triangle entry k -> (i << 8 | j), i <= j, row-major
@@ -233,7 +285,13 @@ __device__ inline void fillPairs(uint16_t *pairs, int n) {
   }
 }
 
-__device__ __forceinline__ void sym3(const double *S, double g0, double g1, double g2, double *h) {
+// h = S g; flat: g2 vanishes and h[2] is not wanted (triangles)
+__device__ __forceinline__ void sym3(const double *S, double g0, double g1, double g2, double *h, bool flat) {
+  if (flat) {
+    h[0] = S[0] * g0 + S[3] * g1;
+    h[1] = S[3] * g0 + S[1] * g1;
+    return;
+  }
   h[0] = S[0] * g0 + S[3] * g1 + S[4] * g2;
   h[1] = S[3] * g0 + S[1] * g1 + S[5] * g2;
   h[2] = S[4] * g0 + S[5] * g1 + S[2] * g2;
@@ -256,14 +314,18 @@ __device__ __forceinline__ void sym3(const double *S, double g0, double g1, doub
 // combined at the end, half the FP64 work of complex D. MASKED: some table
 // components vanish or have no term (a.comps); otherwise all contribute.
 // Bound by the FP64 pipe: 82,944 tetrahedra of order 3 (24 points, real,
-// constant on each element) take 3.98 ms, of which the entries' products
+// constant on each element) take 3.72 ms, of which the entries' products
 // alone are 2.7 ms at one warp instruction per 64 cycles and scheduler; a warp
 // per element, with the geometry and coefficients on its first lane, took
 // 9.93 ms. Order 2 with complex coefficients that vary inside the elements
-// (55,566 tetrahedra): 1.47 ms, before 7.93. HCurl of order 1 (34,992
-// tetrahedra): 1.64 ms, before 5.32.
+// (55,566 tetrahedra): 1.32 ms, before 7.93. HCurl of order 1 (34,992
+// tetrahedra): 1.57 ms, before 5.32. Seven blocks per SM in 72 registers: the
+// phases of one block fill the barriers of the others, and the spills, which
+// are around the (element, point) phase, cost less than that. Three blocks in
+// 168 registers took 4.06, 1.49 and 1.67 ms, five 3.82, 1.40 and 1.58, eight
+// 3.71, 1.42 and 1.58.
 template <int KIND, bool CPLX, bool SPLIT, bool MASKED, int MAXE>
-__global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 3)
+__global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 7)
     k_element_fp64(const PlanDev p, const DevTerms *__restrict__ terms, const QuadArgs a, double *__restrict__ ke, double2 *__restrict__ be) {
   constexpr int R = quadComps(KIND), ND = quadD(KIND);
   constexpr int NC = CPLX ? 2 : 1;           // parts of D and H
@@ -319,10 +381,10 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 3)
       // D (and the source) of every (element, point)
       for (int t = tid; t < live * dn; t += kQuadThreads) {
         const int el = t / dn, qd = t - el * dn, q = d0 + qd;
-        PointGeom P;
-        quadPoint<KIND == kQuadHcurl>(p, terms, g, q, X + el * p.nn * 3, geom + el * kQuadGeom, a.needX != 0, P);
-        const double w = p.w[q];
-        CoefPoint cp = {e0 + el, P.x, nullptr, 0, q, p.nq};
+        double own[kQuadGeom], x[3];
+        const double *P = quadPoint<KIND == kQuadHcurl>(p, terms, g, q, X + el * p.nn * 3, geom + el * kQuadGeom, a.needX != 0, own, x);
+        const double w = p.w[q], wd = w * P[kGeomDet];
+        CoefPoint cp = {e0 + el, x, nullptr, 0, q, p.nq};
         if (KIND != kQuadHcurl) {  // field-node coefficients read the point's row of the basis table
           cp.phi = p.bval + ((size_t)orient[2 * el] * p.nq + q) * n;
           cp.nb = n;
@@ -352,26 +414,27 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 3)
             if (tensor) {
               double F[6];
               if (KIND == kQuadSym) {
-                congruence6(P.Ji, A, part, F);
-                for (int k = 0; k < 6; ++k) dp[k] = w * P.det * F[k];
-                dp[6] = cm * P.det;
+                congruence6(P + kGeomJi, A, part, F);
+                for (int k = 0; k < 6; ++k) dp[k] = wd * F[k];
+                dp[6] = cm * P[kGeomDet];
               } else {
-                congruence6(P.J, A, part, F);
-                for (int k = 0; k < 6; ++k) dp[k] = w * F[k] / P.det;
-                congruence6(P.Ji, B, part, F);
-                for (int k = 0; k < 6; ++k) dp[6 + k] = w * P.det * F[k];
+                congruence6(P + kGeomJ, A, part, F);
+                for (int k = 0; k < 6; ++k) dp[k] = w * F[k] / P[kGeomDet];
+                congruence6(P + kGeomJi, B, part, F);
+                for (int k = 0; k < 6; ++k) dp[6 + k] = wd * F[k];
               }
             } else if (KIND == kQuadSym) {
-              for (int k = 0; k < 6; ++k) dp[k] = cg * P.K6[k];
-              dp[6] = cm * P.det;
+              for (int k = 0; k < 6; ++k) dp[k] = cg * P[kGeomK + k];
+              dp[6] = cm * P[kGeomDet];
             } else {
               for (int k = 0; k < 6; ++k) {
-                dp[k] = cg * P.M6[k];
-                dp[6 + k] = cm * P.K6[k];
+                dp[k] = cg * P[kGeomM + k];
+                dp[6 + k] = cm * P[kGeomK + k];
               }
             }
           }
         } else {
+          const double *Ji = P + kGeomJi;
           double2 A6[6], M[9], v[3], vb[3];
           tensorAt(terms, terms->tensorTerm, terms->tensor, g, cp, c[0], A6);  // c_gg I (+ the symmetric tensor term)
           const int sym[9] = {0, 3, 4, 3, 1, 5, 4, 5, 2};
@@ -392,7 +455,6 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 3)
             const double2 fc = cmul(T.factor, evalAt(T.coef, cp));
             for (int k = 0; k < 3; ++k) vb[k] = cmul(fc, evalAt(terms->vecGrad[k], cp));
           }
-          const double wd = w * P.det;
 #pragma unroll
           for (int part = 0; part < NC; ++part) {
             double *dp = d + part * ND;
@@ -400,11 +462,11 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 3)
             for (int r = 0; r < 3; ++r) {
               double QM[3];  // row r of J^-1 M
               for (int s = 0; s < 3; ++s)
-                QM[s] = P.Ji[3 * r] * re(M[s]) + P.Ji[3 * r + 1] * re(M[3 + s]) + P.Ji[3 * r + 2] * re(M[6 + s]);
+                QM[s] = Ji[3 * r] * re(M[s]) + Ji[3 * r + 1] * re(M[3 + s]) + Ji[3 * r + 2] * re(M[6 + s]);
               for (int s = 0; s < 3; ++s)
-                dp[4 * r + s] = wd * (QM[0] * P.Ji[3 * s] + QM[1] * P.Ji[3 * s + 1] + QM[2] * P.Ji[3 * s + 2]);
-              dp[4 * r + 3] = wd * (P.Ji[3 * r] * re(vb[0]) + P.Ji[3 * r + 1] * re(vb[1]) + P.Ji[3 * r + 2] * re(vb[2]));
-              dp[12 + r] = wd * (P.Ji[3 * r] * re(v[0]) + P.Ji[3 * r + 1] * re(v[1]) + P.Ji[3 * r + 2] * re(v[2]));
+                dp[4 * r + s] = wd * (QM[0] * Ji[3 * s] + QM[1] * Ji[3 * s + 1] + QM[2] * Ji[3 * s + 2]);
+              dp[4 * r + 3] = wd * (Ji[3 * r] * re(vb[0]) + Ji[3 * r + 1] * re(vb[1]) + Ji[3 * r + 2] * re(vb[2]));
+              dp[12 + r] = wd * (Ji[3 * r] * re(v[0]) + Ji[3 * r + 1] * re(v[1]) + Ji[3 * r + 2] * re(v[2]));
             }
             dp[15] = wd * re(c[1]);
           }
@@ -414,18 +476,18 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 3)
           for (int k = 0; k < terms->n; ++k)
             if (terms->t[k].kind == FG_TERM_SOURCE && terms->t[k].mod == g) f = cadd(f, evalAt(terms->t[k].coef, cp));
           double *s = src + (size_t)(el * a.QD + qd) * 8;
-          const double wd = w * P.det;
           s[0] = wd * f.x;
           s[1] = wd * f.y;
           if (KIND == kQuadFull) {
+            const double *Ji = P + kGeomJi;
             double2 sg[3] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
             if (terms->srcGradTerm >= 0 && terms->t[terms->srcGradTerm].mod == g) {
               const double2 fc = evalAt(terms->t[terms->srcGradTerm].coef, cp);
               for (int k = 0; k < 3; ++k) sg[k] = cmul(fc, evalAt(terms->srcGrad[k], cp));
             }
             for (int r = 0; r < 3; ++r) {
-              s[2 + r] = wd * (P.Ji[3 * r] * sg[0].x + P.Ji[3 * r + 1] * sg[1].x + P.Ji[3 * r + 2] * sg[2].x);
-              s[5 + r] = wd * (P.Ji[3 * r] * sg[0].y + P.Ji[3 * r + 1] * sg[1].y + P.Ji[3 * r + 2] * sg[2].y);
+              s[2 + r] = wd * (Ji[3 * r] * sg[0].x + Ji[3 * r + 1] * sg[1].x + Ji[3 * r + 2] * sg[2].x);
+              s[5 + r] = wd * (Ji[3 * r] * sg[0].y + Ji[3 * r + 1] * sg[1].y + Ji[3 * r + 2] * sg[2].y);
             }
           }
         }
@@ -441,7 +503,7 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 3)
             const double *s = src + (size_t)(el * a.QD + qd) * 8;
             const double ph = p.bval[row];
             b.x += s[0] * ph;
-            b.y += s[1] * ph;
+            if (!a.realSource) b.y += s[1] * ph;
             if (KIND == kQuadFull && terms->srcGradTerm >= 0) {
               const double *gr = p.bgrad + 3 * row;
               b.x += s[2] * gr[0] + s[3] * gr[1] + s[4] * gr[2];
@@ -478,9 +540,9 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 3)
 #pragma unroll
               for (int r = 0; r < 4; ++r) o[r] = dp[4 * r] * g0 + dp[4 * r + 1] * g1 + dp[4 * r + 2] * g2 + dp[4 * r + 3] * v[0];
             } else {
-              if (!MASKED || (a.comps & 7)) sym3(dp, g0, g1, g2, o);
+              if (!MASKED || (a.comps & 7)) sym3(dp, g0, g1, g2, o, MASKED && KIND == kQuadSym && !(a.comps & 4));
               if (KIND == kQuadSym) o[3] = dp[6] * v[0];
-              else if (!MASKED || (a.comps & 56)) sym3(dp + 6, v[0], v[1], v[2], o + 3);
+              else if (!MASKED || (a.comps & 56)) sym3(dp + 6, v[0], v[1], v[2], o + 3, false);
             }
 #pragma unroll
             for (int r = 0; r < R; ++r)
@@ -560,10 +622,11 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 3)
 // is formed once; otherwise the lambda- and mu-weighted sums are kept apart
 // (19 products, twice for complex coefficients). a.comps: 1 the elastic
 // term, 2 the mass term. Bound by the FP64 pipe: order 2, 20,250 tetrahedra,
-// Lame coefficients per element: 0.468 ms (with the weighted terms formed for
-// every entry, a warp per element, it took 3.15 ms).
+// Lame coefficients per element: 0.475 ms (with the weighted terms formed for
+// every entry, a warp per element, it took 3.15 ms); three blocks per SM in
+// place of four took 0.492.
 template <bool UNIFORM, bool CPLX, int MAXP>
-__global__ void __launch_bounds__(kQuadThreads, UNIFORM ? 3 : 2)
+__global__ void __launch_bounds__(kQuadThreads, UNIFORM ? 4 : 2)
     k_element_elastic_fp64(const PlanDev p, const DevTerms *__restrict__ terms, const QuadArgs a, double *__restrict__ ke,
                            double2 *__restrict__ be) {
   constexpr int NC = (!UNIFORM && CPLX) ? 2 : 1;
@@ -615,15 +678,15 @@ __global__ void __launch_bounds__(kQuadThreads, UNIFORM ? 3 : 2)
       const int dn = min(a.QD, p.nq - d0);
       for (int t = tid; t < live * dn; t += kQuadThreads) {
         const int el = t / dn, qd = t - el * dn, q = d0 + qd;
-        PointGeom P;
-        quadPoint<false>(p, terms, g, q, X + el * p.nn * 3, geom + el * kQuadGeom, a.needX != 0, P);
+        double own[kQuadGeom], x[3];
+        const double *P = quadPoint<false>(p, terms, g, q, X + el * p.nn * 3, geom + el * kQuadGeom, a.needX != 0, own, x);
         double *d = D + (size_t)(el * a.QD + qd) * ND;
-        const double wd = p.w[q] * P.det;
-        for (int k = 0; k < 9; ++k) d[k] = P.Ji[k];
+        const double wd = p.w[q] * P[kGeomDet];
+        for (int k = 0; k < 9; ++k) d[k] = P[kGeomJi + k];
         d[9] = wd;
         if (!UNIFORM) {
           double2 c[3];
-          const CoefPoint cp = {e0 + el, P.x, p.bval + ((size_t)orient[2 * el] * p.nq + q) * ns, ns, q, p.nq};
+          const CoefPoint cp = {e0 + el, x, p.bval + ((size_t)orient[2 * el] * p.nq + q) * ns, ns, q, p.nq};
           scalarCoefs(terms, g, cp, c);
           d[10] = wd * c[0].x;
           d[11] = wd * c[2].x;
@@ -747,47 +810,58 @@ __global__ void __launch_bounds__(kQuadThreads, UNIFORM ? 3 : 2)
     for (int t = tid; t < live * n; t += kQuadThreads) be[(size_t)e0 * n + t] = make_double2(0.0, 0.0);
 }
 
-// Elements per block and points per chunk. An SM runs blocks / SMs of them
-// one after the other as far as its FP64 pipe goes, each as long as its
-// fullest warp has entries per thread (plus about half an entry for the other
-// phases): the number of elements with the least total, which is few for
-// small meshes (all SMs busy, short blocks) and the best filled block for
-// large ones: 82,944 tetrahedra of order 3 took 4.08 ms with the 6 elements
-// this picks, 4.34 with 5 or 4 and 4.89 with 2; order 2 with complex D, 1.51 ms
-// with 16 or more, 1.65 with 9, 2.41 with 3. D is formed for as many points as give every thread an
-// (element, point) pair, H for what the remaining shared memory holds.
-static bool quadShape(const PlanDev &p, int nEnt, int n, int nU, int nd, int nh, bool be, int nPairs, int maxItems, QuadArgs *a) {
+// Elements per block and points per chunk: the fewest FP64 instructions that
+// an SM's fullest warps run one after the other. A block takes, per point,
+// one product per table component for every entry of a thread (comps), hCost
+// instructions per round of (element, point, function) triples, dCost per
+// round of (element, point) pairs, and about 60 for the elements' geometry; an
+// SM runs blocks / SMs of them. So small meshes get few elements per block
+// (all SMs busy), large ones what fills the rounds best. D is formed for QD
+// points at a time, H for what the remaining shared memory holds.
+// Measured: 55,566 order-2 tetrahedra, complex D inside the elements, 1.31 to
+// 1.33 ms with 6, 9 or 24 elements, whose rounds are full, 1.43 with 12 and
+// 1.74 with 18.
+static bool quadShape(const PlanDev &p, int nEnt, int n, int nU, int nd, int nh, bool be, int nPairs, int maxItems, int comps,
+                      int hCost, int dCost, QuadArgs *a) {
   const int64_t sms = smCount();
   auto bytes = [&](int NE, int QD, int QC) { return (size_t)quadLayout(NE, QD, QC, p.nn, n, nU, nd, nh, be, nPairs).total * 8; };
+  auto rounds = [](int64_t items) { return (items + kQuadThreads - 1) / kQuadThreads; };
+  auto even = [&](int chunks) { return (p.nq + chunks - 1) / chunks; };
   double best = 0.0;
   a->NE = 0;
   for (int NE = 1; NE <= kQuadMaxElems && (int64_t)NE * nEnt <= (int64_t)kQuadThreads * maxItems; ++NE) {
-    if (bytes(NE, std::min(p.nq, 2), std::min(p.nq, 2)) > kQuadSmem && NE > 1) break;
+    // the fewest chunks of D that fit beside two points of H, or one or two more
+    int chunks = 1;
+    while (chunks < p.nq && bytes(NE, even(chunks), std::min(2, even(chunks))) > kQuadSmem) ++chunks;
+    if (bytes(NE, even(chunks), 1) > kQuadSmem && NE > 1) break;
     const int64_t blocks = (p.E + NE - 1) / NE;
-    const double cost = (double)((blocks + sms - 1) / sms) * ((NE * nEnt + kQuadThreads - 1) / kQuadThreads + 0.5);
-    if (a->NE == 0 || cost < best) {
-      best = cost;
-      a->NE = NE;
+    for (int c = chunks; c <= chunks + 2 && c <= p.nq; ++c) {
+      const int64_t d = (int64_t)((p.nq + even(c) - 1) / even(c)) * rounds((int64_t)NE * even(c)) * dCost;
+      const int64_t block = rounds((int64_t)NE * nEnt) * p.nq * comps + rounds((int64_t)NE * p.nq * nU) * hCost + d + 60;
+      const double cost = (double)((blocks + sms - 1) / sms) * (double)block;
+      if (a->NE == 0 || cost < best) {
+        best = cost;
+        a->NE = NE;
+        a->QD = even(c);
+      }
     }
   }
-  if (a->NE == 0 || bytes(a->NE, 1, 1) > kQuadSmem) return false;
-  int QD = std::min(p.nq, (kQuadThreads + a->NE - 1) / a->NE);
-  while (QD > 1 && bytes(a->NE, QD, std::min(QD, 2)) > kQuadSmem) --QD;
-  int QC = std::min(QD, 16);
-  while (QC > 1 && bytes(a->NE, QD, QC) > kQuadSmem) --QC;
-  auto even = [](int count, int most) {  // chunks of nearly equal size
-    const int chunks = (count + most - 1) / most;
-    return (count + chunks - 1) / chunks;
-  };
-  a->QD = even(p.nq, QD);
-  a->QC = even(a->QD, std::min(QC, a->QD));
+  if (a->NE == 0 || bytes(a->NE, a->QD, 1) > kQuadSmem) {
+    // the widest element matrices: one element and one point at a time
+    a->NE = a->QD = 1;
+    if (nEnt > kQuadThreads * maxItems || bytes(1, 1, 1) > 48 * 1024) return false;
+  }
+  int QC = std::min(a->QD, 16);
+  while (QC > 1 && bytes(a->NE, a->QD, QC) > kQuadSmem) --QC;
+  const int parts = (a->QD + QC - 1) / QC;
+  a->QC = (a->QD + parts - 1) / parts;
   a->nEnt = nEnt;
   return true;
 }
 
 // What the launch's switches need to know of the terms
 struct TermUse {
-  bool grad = false, mass = false, pointBilinear = false, pointSource = false;
+  bool grad = false, mass = false, pointBilinear = false, pointSource = false, realSource = true;
 };
 static TermUse termUse(const DevTerms &terms) {
   TermUse u;
@@ -797,7 +871,10 @@ static TermUse termUse(const DevTerms &terms) {
   for (int t = 0; t < terms.n; ++t) {
     const DevTerm &T = terms.t[t];
     switch (T.kind) {
-      case FG_TERM_SOURCE: scan(&T.coef, 1, u.pointSource); continue;
+      case FG_TERM_SOURCE:
+        scan(&T.coef, 1, u.pointSource);
+        u.realSource = u.realSource && T.coef.real;
+        continue;
       case FG_TERM_SOURCE_GRAD:
         scan(&T.coef, 1, u.pointSource);
         scan(terms.srcGrad, 3, u.pointSource);
@@ -824,10 +901,12 @@ static int quadFail() {
 }
 
 template <int KIND, bool CPLX, bool SPLIT, bool MASKED, int MAXE>
-static int quadLaunch(const PlanDev &p, const DevTerms *dterms, QuadArgs a, int nEnt, double *ke, double2 *be, cudaStream_t s) {
+static int quadLaunch(const PlanDev &p, const DevTerms *dterms, QuadArgs a, int nEnt, int coefCost, double *ke, double2 *be, cudaStream_t s) {
   constexpr int NC = CPLX ? 2 : 1;
   const int nPairs = KIND == kQuadFull ? 0 : nEnt, nd = quadD(KIND) * NC, nh = quadComps(KIND) * NC;
-  if (!quadShape(p, nEnt, p.nb, p.nbU, nd, nh, be != nullptr, nPairs, MAXE, &a)) return quadFail();
+  const int hCost = (KIND == kQuadSym ? 10 : KIND == kQuadHcurl ? 18 : 16) * NC;
+  if (!quadShape(p, nEnt, p.nb, p.nbU, nd, nh, be != nullptr, nPairs, MAXE, quadComps(KIND) * NC, hCost, nd + coefCost, &a))
+    return quadFail();
   const size_t smem = (size_t)quadLayout(a.NE, a.QD, a.QC, p.nn, p.nb, p.nbU, nd, nh, be != nullptr, nPairs).total * 8;
   k_element_fp64<KIND, CPLX, SPLIT, MASKED, MAXE>
       <<<(unsigned)((p.E + a.NE - 1) / a.NE), kQuadThreads, smem, s>>>(p, dterms, a, ke, be);
@@ -845,13 +924,16 @@ static int quadKind(const PlanDev &p, const DevTerms &terms, const DevTerms *dte
   const int full = (1 << quadComps(KIND)) - 1;
   a.comps = p.tableComps & ((u.grad ? 7 : 0) | (u.mass ? full & ~7 : 0));
   a.uniform = !u.pointBilinear;
+  a.realSource = u.realSource;
   a.needX = (ke && u.pointBilinear) || (be && u.pointSource) || terms.hasJacMod;
   const bool masked = a.comps != full, cplx = terms.complexKe != 0;
+  // about what a point's coefficients take
+  const int coefCost = (ke && u.pointBilinear ? 80 : 10) + (be ? (u.realSource ? 40 : 100) : 0);
   // complex sums of real integrals: one group of terms, no tensors
   const bool split = KIND != kQuadFull && cplx && a.uniform && terms.nMod <= 1 && terms.tensorTerm < 0 && terms.tensorMassTerm < 0;
 #define FG_QUAD(C, S)                                                                              \
-  (masked ? quadLaunch<KIND, C, S, true, MAXE>(p, dterms, a, nEnt, ke, be, s)                      \
-          : quadLaunch<KIND, C, S, false, MAXE>(p, dterms, a, nEnt, ke, be, s))
+  (masked ? quadLaunch<KIND, C, S, true, MAXE>(p, dterms, a, nEnt, coefCost, ke, be, s)                      \
+          : quadLaunch<KIND, C, S, false, MAXE>(p, dterms, a, nEnt, coefCost, ke, be, s))
   if constexpr (KIND != kQuadFull) {
     if (split) return FG_QUAD(false, true);
   }
@@ -862,7 +944,8 @@ static int quadKind(const PlanDev &p, const DevTerms &terms, const DevTerms *dte
 template <bool UNIFORM, bool CPLX, int MAXP>
 static int quadElastic(const PlanDev &p, const DevTerms *dterms, QuadArgs a, int nEnt, double *ke, double2 *be, cudaStream_t s) {
   constexpr int NC = (!UNIFORM && CPLX) ? 2 : 1, ND = 10 + (UNIFORM ? 0 : 3 * NC), NH = UNIFORM ? 7 : 3 + 7 * NC;
-  if (!quadShape(p, nEnt, 0, p.nb, ND, NH, false, nEnt, MAXP, &a)) return quadFail();
+  const int sums = UNIFORM ? 10 : 19 * NC;
+  if (!quadShape(p, nEnt, 0, p.nb, ND, NH, false, nEnt, MAXP, sums, 9 + NH, ND + (UNIFORM ? 0 : 80), &a)) return quadFail();
   const size_t smem = (size_t)quadLayout(a.NE, a.QD, a.QC, p.nn, 0, p.nb, ND, NH, false, nEnt).total * 8;
   k_element_elastic_fp64<UNIFORM, CPLX, MAXP><<<(unsigned)((p.E + a.NE - 1) / a.NE), kQuadThreads, smem, s>>>(p, dterms, a, ke, be);
   countLaunch();

@@ -71,7 +71,8 @@ constexpr uint16_t kSlotIgnore = 0xFFFE;  // column does not assemble (undefined
 enum ExprClass { kExprConst = 0, kExprElem = 1, kExprPoint = 2 };
 struct DevExpr {
   int32_t n_code;
-  int32_t cls;
+  int16_t cls;
+  int16_t real;  // 1: its value is real for real points and arrays (no imaginary constant or array, no operator that leaves the reals)
   double2 cval;  // value when cls == kExprConst
   fg_instr code[FG_EXPR_MAX_CODE];
   const double2 *arr[FG_EXPR_MAX_ARRAYS];
@@ -123,6 +124,7 @@ struct DevTerms {
 struct PlanDev {
   int32_t dim, nn, nq, nb, mult, n, nOrient, affine;
   int32_t p1geom;         // first-order simplex geometry with the standard node order
+  int32_t planar;         // 2D elements whose nodes share one z: the unit normal is (0, 0, +-1)
   int32_t form;           // FG_FORM_0 (H1) or FG_FORM_1 (HCurl: vector values, curls)
   int64_t E, nNodes;
   uint64_t nRows, nnz, nFixed;
@@ -561,6 +563,45 @@ __device__ inline double2 evalExpr(const DevExpr &ex, int64_t e, const double *x
         break;
       }
       default: st[sp - 1] = cUnary(in.op, in.arg, st[sp - 1]);
+    }
+  }
+  return st[0];
+}
+
+// The same for an expression of real value (DevExpr::real): one product or
+// sum per operator instead of a complex one's two to six, on a pipe that takes
+// 64 cycles for each
+__device__ inline double evalExprReal(const DevExpr &ex, int64_t e, const double *x, const double *phi, int nb, int q, int nq) {
+  double st[16];
+  int sp = 0;
+  for (int k = 0; k < ex.n_code; ++k) {
+    const fg_instr in = ex.code[k];
+    switch (in.op) {
+      case FG_OP_CONST: st[sp++] = in.re; break;
+      case FG_OP_X: st[sp++] = x[0]; break;
+      case FG_OP_Y: st[sp++] = x[1]; break;
+      case FG_OP_Z: st[sp++] = x[2]; break;
+      case FG_OP_ELEM: st[sp++] = ex.arr[in.arg][e].x; break;
+      case FG_OP_POINT: st[sp++] = ex.arr[in.arg][e * nq + q].x; break;
+      case FG_OP_FIELD: {
+        const double2 *u = ex.arr[in.arg] + (size_t)e * nb;
+        double s = 0.0;
+        for (int j = 0; phi && j < nb; ++j) s += phi[j] * u[j].x;
+        st[sp++] = s;
+        break;
+      }
+      case FG_OP_ADD: --sp; st[sp - 1] += st[sp]; break;
+      case FG_OP_SUB: --sp; st[sp - 1] -= st[sp]; break;
+      case FG_OP_MUL: --sp; st[sp - 1] *= st[sp]; break;
+      case FG_OP_NEG: st[sp - 1] = -st[sp - 1]; break;
+      case FG_OP_HEAVISIDE: st[sp - 1] = st[sp - 1] > 0.0 ? 1.0 : (st[sp - 1] < 0.0 ? 0.0 : 0.5); break;
+      case FG_OP_DIV:
+      case FG_OP_ATAN2: {
+        const double2 b = make_double2(st[--sp], 0.0), a = make_double2(st[sp - 1], 0.0);
+        st[sp - 1] = in.op == FG_OP_DIV ? cdiv(a, b).x : atan2(a.x, b.x);
+        break;
+      }
+      default: st[sp - 1] = cUnary(in.op, in.arg, make_double2(st[sp - 1], 0.0)).x;
     }
   }
   return st[0];

@@ -136,7 +136,7 @@ __device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *__restric
       }
     }
   };
-  auto loadKe = [&](const Step &s, KT (&vr)[U][J * VW], KT (&vi)[U][KCPLX ? J * VW : 1]) {
+  auto loadKe = [&](const Step &s, KT (&vr)[U][J * VW], KT (&vi)[U][KCPLX ? J * VW : 1], double2 (&vb)[U]) {
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (s.packed[u] != kRecNone) {
@@ -146,6 +146,7 @@ __device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *__restric
           const uint32_t ib = i / 3, a = i - 3 * ib;
           row = (a * 3 * nb + ib) * nb;
         }
+        if (!SIMPLE && be && lt == 0) vb[u] = __ldg(&be[(size_t)e * n + i]);
         const KT *K = ke + ((uint64_t)e * (SS * ld) + row);
 #pragma unroll
         for (int c = 0; c < J; ++c)
@@ -164,8 +165,9 @@ __device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *__restric
   uint4 v = visitAt(first), vN = visitAt(first + stride);
   Step cur, nxt;
   KT vr[U][J * VW], vi[U][KCPLX ? J * VW : 1];
+  double2 vb[U];  // the element vectors' entries (first lane of a row)
   loadRec(v.z, 0, (int)(v.w >> 16), cur);
-  loadKe(cur, vr, vi);
+  loadKe(cur, vr, vi, vb);
   loadRec(v.z, U, (int)(v.w >> 16), nxt);
   __syncwarp();
   for (int64_t base = v0 + (blk * wpb + warp) * R; base < v1; base += stride) {
@@ -183,7 +185,8 @@ __device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *__restric
       const bool last = st + 1 == steps;
       if (last) nxt = nextRow;
       KT vrN[U][J * VW], viN[U][KCPLX ? J * VW : 1];
-      loadKe(nxt, vrN, viN);
+      double2 vbN[U];
+      loadKe(nxt, vrN, viN, vbN);
       Step after;
       if (last) loadRec(vN.z, U, cntN, after);
       else loadRec(v.z, (st + 2) * U, cnt, after);
@@ -200,8 +203,7 @@ __device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *__restric
             cI.y = -cI.y;
           }
           if (!SIMPLE && be && lt == 0) {
-            const double2 b = be[(size_t)e * n + i];
-            bsum = cadd(bsum, linked ? cmul(cI, b) : b);
+            bsum = cadd(bsum, linked ? cmul(cI, vb[u]) : vb[u]);
           }
 #pragma unroll
           for (int c = 0; c < J; ++c) {
@@ -247,6 +249,7 @@ __device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *__restric
       nxt = after;
 #pragma unroll
       for (int u = 0; u < U; ++u) {
+        if (!SIMPLE) vb[u] = vbN[u];
 #pragma unroll
         for (int k = 0; k < J * VW; ++k) {
           vr[u][k] = vrN[u][k];

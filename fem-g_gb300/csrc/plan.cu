@@ -455,6 +455,8 @@ static int createPlan(const fg_mesh_desc *mesh, const fg_rule_desc *rule, const 
     for (size_t r = 0; r < (size_t)E * n; ++r)
       std::fill(slot8.begin() + (int64_t)(r * nS + nc), slot8.begin() + (int64_t)((r + 1) * nS), (uint8_t)0xFE);
 
+  d.planar = mesh->dim == 2 && mesh->n_nodes > 0;
+  for (int64_t k = 1; k < mesh->n_nodes && d.planar; ++k) d.planar = mesh->node_xyz[3 * k + 2] == mesh->node_xyz[2];
   // table components that vanish everywhere (the third one on triangles, say)
   {
     const size_t rows = (size_t)space->n_orientations * rule->nq * space->n_basis;
@@ -681,7 +683,7 @@ static int validateExpr(const fg_expr &ex) {
 // tables of FG_OP_POINT); the first `used` are
 // this upload's, later ones are reused from the previous upload instead of
 // freed and allocated again (a buffer too small for its new array is replaced).
-static int devExpr(fg_plan *plan, const fg_expr &ex, DevExpr *out, bool *complexOut, std::vector<void *> &arrays, size_t &used) {
+static int devExprParts(fg_plan *plan, const fg_expr &ex, DevExpr *out, bool *complexOut, std::vector<void *> &arrays, size_t &used) {
   if (validateExpr(ex)) {
     setLastError("invalid coefficient expression");
     return FG_ERR_ARG;
@@ -756,6 +758,15 @@ static int devExpr(fg_plan *plan, const fg_expr &ex, DevExpr *out, bool *complex
     }
     out->arr[a] = (const double2 *)p;
   }
+  return FG_OK;
+}
+
+static int devExpr(fg_plan *plan, const fg_expr &ex, DevExpr *out, bool *complexOut, std::vector<void *> &arrays, size_t &used) {
+  bool cplx = false;
+  const int st = devExprParts(plan, ex, out, &cplx, arrays, used);
+  if (st) return st;
+  out->real = cplx ? 0 : 1;
+  if (cplx) *complexOut = true;
   return FG_OK;
 }
 
