@@ -5,10 +5,11 @@
 // Keys: float coordinates scaled into the box exactly as the host does it,
 // an unfused float multiply then add (__fmul_rn, __fadd_rn) truncated to an
 // integer per axis, walked through the Hilbert state tables (2D: 32 bits
-// per axis, 3D: 21). The order is the stable order of the keys; sorting the
-// composite (key, input index), which is unique, with a bitonic network
-// gives it exactly, whatever sort is used. Strides of 2048 and more run as
-// global compare-exchange passes, the smaller ones in shared memory.
+// per axis, 3D: 21). The order is the stable order of the keys: a radix sort
+// of (key, input index) by eight bits a pass, least first, each pass stable.
+// The numbering sorts every DOF by one more pass over its class (Unknown,
+// Unknown bubble, other), so that the host neither picks out nor spreads the
+// DOFs: on 195,112 DOFs, 0.63 ms a call in place of 2.4.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -18,25 +19,23 @@
 
 namespace femg {
 
-constexpr int kBitonicTile = 2048;
+constexpr int kRadixThreads = 256, kRadixWarps = 8, kRadixTile = 4096;  // 512 consecutive items per warp
 
 struct HilbertDev {
   uint8_t code[24][8];
   uint8_t next[24][8];
 };
 
-__global__ void k_hilbert_keys(int dim, uint64_t n, uint64_t padded, const float *__restrict__ pts, float3 scale, float3 scaleMin,
-                               const HilbertDev tab, uint64_t *__restrict__ keys, uint32_t *__restrict__ idx) {
+// Keys of the points pts [n][stride], index i beside each. cls (may be null):
+// the class of DOF i by its assemble type
+__global__ void k_hilbert_keys(int dim, uint64_t n, const float *__restrict__ pts, int stride, float3 scale, float3 scaleMin,
+                               const HilbertDev tab, uint64_t *__restrict__ keys, uint32_t *__restrict__ idx,
+                               const int32_t *__restrict__ type, uint8_t *__restrict__ cls) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= padded) return;
-  if (i >= n) {  // padding sorts after every point
-    keys[i] = ~0ull;
-    idx[i] = 0xFFFFFFFFu;
-    return;
-  }
+  if (i >= n) return;
   const float sc[3] = {scale.x, scale.y, scale.z}, sm[3] = {scaleMin.x, scaleMin.y, scaleMin.z};
   uint32_t u[3] = {0, 0, 0};
-  for (int j = 0; j < dim; ++j) u[j] = __float2uint_rz(__fadd_rn(__fmul_rn(pts[i * dim + j], sc[j]), sm[j]));
+  for (int j = 0; j < dim; ++j) u[j] = __float2uint_rz(__fadd_rn(__fmul_rn(pts[i * stride + j], sc[j]), sm[j]));
   const int begBit = (64 / dim) - 1;
   uint64_t h = 0;
   unsigned ed = 0;
@@ -49,68 +48,117 @@ __global__ void k_hilbert_keys(int dim, uint64_t n, uint64_t padded, const float
   }
   keys[i] = h;
   idx[i] = (uint32_t)i;
+  if (cls) cls[i] = type[i] == FG_AT_UNKNOWN ? 0 : type[i] == FG_AT_UNKNOWN_BUBBLE ? 1 : 2;
 }
 
-__device__ __forceinline__ bool pairLess(uint64_t ka, uint32_t ia, uint64_t kb, uint32_t ib) {
-  return ka < kb || (ka == kb && ia < ib);
+// The digit of item k in a pass: eight bits of its key, or its DOF's class
+struct RadixDigit {
+  const uint64_t *keys;
+  const uint32_t *idx;
+  const uint8_t *cls;  // not null: the pass over the classes
+  int shift;
+  __device__ __forceinline__ uint32_t at(uint64_t k) const { return cls ? cls[idx[k]] : (uint32_t)(keys[k] >> shift) & 0xFFu; }
+};
+
+// Digit counts of a tile into hist[digit][tile]
+__global__ void __launch_bounds__(kRadixThreads) k_radix_count(const RadixDigit d, uint64_t n, uint32_t tiles, uint32_t *__restrict__ hist) {
+  __shared__ uint32_t h[256];
+  h[threadIdx.x] = 0;
+  __syncthreads();
+  const uint64_t end = min(n, ((uint64_t)blockIdx.x + 1) * kRadixTile);
+  for (uint64_t k = (uint64_t)blockIdx.x * kRadixTile + threadIdx.x; k < end; k += kRadixThreads) atomicAdd(&h[d.at(k)], 1u);
+  __syncthreads();
+  hist[(uint64_t)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
 
-// one compare-exchange pass of stride j in bitonic blocks of size k
-__global__ void k_bitonic_global(uint64_t *__restrict__ keys, uint32_t *__restrict__ idx, uint64_t padded, uint64_t k, uint64_t j) {
-  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= padded / 2) return;
-  const uint64_t lo = 2 * j * (t / j) + (t % j), hi = lo + j;
-  const bool up = (lo & k) == 0;
-  const uint64_t ka = keys[lo], kb = keys[hi];
-  const uint32_t ia = idx[lo], ib = idx[hi];
-  if (pairLess(kb, ib, ka, ia) == up) {
-    keys[lo] = kb;
-    keys[hi] = ka;
-    idx[lo] = ib;
-    idx[hi] = ia;
+// Exclusive scan of each digit's counts over the tiles, in place; totals[digit]
+__global__ void __launch_bounds__(kRadixThreads) k_radix_scan(uint32_t *__restrict__ hist, uint32_t tiles, uint32_t *__restrict__ totals) {
+  __shared__ uint32_t warpSum[kRadixWarps];
+  uint32_t *row = hist + (uint64_t)blockIdx.x * tiles;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t carry = 0;
+  for (uint32_t b = 0; b < tiles; b += kRadixThreads) {
+    const uint32_t k = b + threadIdx.x, v = k < tiles ? row[k] : 0u;
+    uint32_t inc = v;
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t o = __shfl_up_sync(0xffffffffu, inc, off);
+      if (lane >= off) inc += o;
+    }
+    if (lane == 31) warpSum[warp] = inc;
+    __syncthreads();
+    uint32_t before = carry, all = 0;
+    for (int w = 0; w < kRadixWarps; ++w) {
+      if (w < warp) before += warpSum[w];
+      all += warpSum[w];
+    }
+    if (k < tiles) row[k] = before + inc - v;
+    carry += all;
+    __syncthreads();
   }
+  if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
 
-// strides jStart, jStart/2, ..., 1 of blocks of size k inside one tile (k <= tile: the whole
-// sort of the tile up to k)
-__global__ void __launch_bounds__(kBitonicTile / 2) k_bitonic_tile(uint64_t *__restrict__ keys, uint32_t *__restrict__ idx, uint64_t k,
-                                                                  uint64_t jStart, int full) {
-  __shared__ uint64_t sk[kBitonicTile];
-  __shared__ uint32_t si[kBitonicTile];
-  const uint64_t base = (uint64_t)blockIdx.x * kBitonicTile;
-  for (int t = threadIdx.x; t < kBitonicTile; t += blockDim.x) {
-    sk[t] = keys[base + t];
-    si[t] = idx[base + t];
+// The items of a tile to their places: after all items of smaller digits,
+// those of the digit in earlier tiles, in earlier warps of this one (a warp
+// has 512 consecutive items) and earlier in the warp (32 at a time, the equal
+// digits of which are matched)
+__global__ void __launch_bounds__(kRadixThreads)
+    k_radix_scatter(const RadixDigit d, uint64_t n, uint32_t tiles, const uint32_t *__restrict__ hist, const uint32_t *__restrict__ totals,
+                    uint64_t *__restrict__ keysOut, uint32_t *__restrict__ idxOut) {
+  __shared__ uint32_t place[kRadixWarps][256];
+  __shared__ uint32_t warpSum[kRadixWarps];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int w = 0; w < kRadixWarps; ++w) place[w][tid] = 0;
+  __syncthreads();
+  constexpr int kPer = kRadixTile / kRadixWarps;
+  const uint64_t w0 = (uint64_t)blockIdx.x * kRadixTile + (uint64_t)warp * kPer;
+  for (int r = 0; r < kPer; r += 32)
+    if (w0 + r + lane < n) atomicAdd(&place[warp][d.at(w0 + r + lane)], 1u);
+  // exclusive scan of the digits' totals, one digit per thread
+  const uint32_t total = totals[tid];
+  uint32_t inc = total;
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t o = __shfl_up_sync(0xffffffffu, inc, off);
+    if (lane >= off) inc += o;
+  }
+  if (lane == 31) warpSum[warp] = inc;
+  __syncthreads();
+  uint32_t at = inc - total + hist[(uint64_t)tid * tiles + blockIdx.x];
+  for (int w = 0; w < warp; ++w) at += warpSum[w];
+  for (int w = 0; w < kRadixWarps; ++w) {
+    const uint32_t c = place[w][tid];
+    place[w][tid] = at;
+    at += c;
   }
   __syncthreads();
-  const uint64_t kFirst = full ? 2 : k;
-  for (uint64_t kk = kFirst; kk <= k; kk <<= 1) {
-    for (uint64_t j = full ? kk / 2 : jStart; j > 0; j >>= 1) {
-      const int t = threadIdx.x;
-      const uint64_t lo = 2 * j * (t / j) + (t % j), hi = lo + j;
-      const bool up = ((base + lo) & kk) == 0;
-      const uint64_t ka = sk[lo], kb = sk[hi];
-      const uint32_t ia = si[lo], ib = si[hi];
-      if (pairLess(kb, ib, ka, ia) == up) {
-        sk[lo] = kb;
-        sk[hi] = ka;
-        si[lo] = ib;
-        si[hi] = ia;
-      }
-      __syncthreads();
+  for (int r = 0; r < kPer; r += 32) {
+    const uint64_t k = w0 + r + lane;
+    const bool live = k < n;
+    const uint32_t digit = live ? d.at(k) : 256u;
+    const uint32_t same = __match_any_sync(0xffffffffu, digit);
+    if (live) {
+      const uint32_t to = place[warp][digit] + __popc(same & ((1u << lane) - 1u));
+      keysOut[to] = d.keys[k];
+      idxOut[to] = d.idx[k];
     }
-  }
-  for (int t = threadIdx.x; t < kBitonicTile; t += blockDim.x) {
-    keys[base + t] = sk[t];
-    idx[base + t] = si[t];
+    __syncwarp();
+    if (live && lane == __ffs(same) - 1) place[warp][digit] += __popc(same);
+    __syncwarp();
   }
 }
 
-// Stable Hilbert order of n points (float [n][dim]) in the box [mn, mx].
-static int hilbertOrderGpu(int dim, uint64_t n, const float *pts, const float *mn, const float *mx, uint32_t *perm) {
+// DOF idx[k] gets number k + 1, k < count (Unknown DOFs, then bubbles)
+__global__ void k_number(const uint32_t *__restrict__ idx, uint64_t n, const uint8_t *__restrict__ cls, uint64_t *__restrict__ num) {
+  const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n && cls[idx[k]] < 2) num[idx[k]] = k + 1;
+}
+
+// Stable Hilbert order of n points (float [n][stride], in host memory) in the
+// box [mn, mx]: into perm; or, with the assemble types, the DOFs' numbers
+// into num.
+static int hilbertOrderGpu(int dim, uint64_t n, const float *pts, int stride, const float *mn, const float *mx, uint32_t *perm,
+                           const int32_t *type, uint64_t *num) {
   if (n == 0) return FG_OK;
-  uint64_t padded = kBitonicTile;
-  while (padded < n) padded <<= 1;
   // scale as the host sort computes it (float)
   const unsigned nbrBits = 64 / dim;
   const unsigned twoPow = 1u << (nbrBits - 1);
@@ -121,46 +169,52 @@ static int hilbertOrderGpu(int dim, uint64_t n, const float *pts, const float *m
   }
   HilbertDev tab;
   hilbertTableData(dim, &tab.code[0][0], &tab.next[0][0]);
-  float *dPts = nullptr;
-  uint64_t *keys = nullptr;
-  uint32_t *idx = nullptr;
-  auto release = [&]() {
-    cudaFree(dPts);
-    cudaFree(keys);
-    cudaFree(idx);
+  const uint32_t tiles = (uint32_t)((n + kRadixTile - 1) / kRadixTile);
+  size_t bytes = 0;
+  auto part = [&](size_t b) {
+    const size_t at = bytes;
+    bytes += (b + 255) / 256 * 256;
+    return at;
   };
-  if (cudaMalloc(&dPts, n * dim * sizeof(float)) != cudaSuccess || cudaMalloc(&keys, padded * 8) != cudaSuccess ||
-      cudaMalloc(&idx, padded * 4) != cudaSuccess) {
+  const size_t oPts = part(n * stride * sizeof(float)), oType = part(type ? n * 4 : 0), oCls = part(type ? n : 0),
+               oNum = part(type ? n * 8 : 0), oK0 = part(n * 8), oK1 = part(n * 8), oI0 = part(n * 4), oI1 = part(n * 4),
+               oHist = part((size_t)256 * tiles * 4), oTotals = part(256 * 4);
+  uint8_t *base = nullptr;
+  if (cudaMalloc(&base, bytes) != cudaSuccess) {
     cudaGetLastError();
-    release();
     setLastError("hilbert order: device allocation failed");
     return FG_ERR_OOM;
   }
-  int st = FG_OK;
-  do {
-    if (cudaMemcpy(dPts, pts, n * dim * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) break;
-    k_hilbert_keys<<<(unsigned)((padded + 255) / 256), 256>>>(dim, n, padded, dPts, make_float3(sc[0], sc[1], sc[2]),
-                                                              make_float3(sm[0], sm[1], sm[2]), tab, keys, idx);
-    const unsigned tiles = (unsigned)(padded / kBitonicTile);
-    k_bitonic_tile<<<tiles, kBitonicTile / 2>>>(keys, idx, kBitonicTile, 0, 1);  // every tile sorted in alternating directions
-    int launches = 2;
-    for (uint64_t k = 2 * kBitonicTile; k <= padded; k <<= 1) {
-      for (uint64_t j = k / 2; j >= kBitonicTile; j >>= 1) {
-        k_bitonic_global<<<(unsigned)((padded / 2 + 255) / 256), 256>>>(keys, idx, padded, k, j);
-        ++launches;
-      }
-      k_bitonic_tile<<<tiles, kBitonicTile / 2>>>(keys, idx, k, kBitonicTile / 2, 0);
-      ++launches;
+  uint64_t *keys[2] = {(uint64_t *)(base + oK0), (uint64_t *)(base + oK1)};
+  uint32_t *idx[2] = {(uint32_t *)(base + oI0), (uint32_t *)(base + oI1)};
+  uint32_t *hist = (uint32_t *)(base + oHist), *totals = (uint32_t *)(base + oTotals);
+  uint8_t *cls = type ? base + oCls : nullptr;
+  auto run = [&]() -> cudaError_t {
+    cudaError_t e = cudaMemcpyAsync(base + oPts, pts, n * stride * sizeof(float), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && type) e = cudaMemcpyAsync(base + oType, type, n * 4, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && type) e = cudaMemcpyAsync(base + oNum, num, n * 8, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return e;
+    const unsigned nb = (unsigned)((n + 255) / 256);
+    k_hilbert_keys<<<nb, 256>>>(dim, n, (const float *)(base + oPts), stride, make_float3(sc[0], sc[1], sc[2]),
+                                make_float3(sm[0], sm[1], sm[2]), tab, keys[0], idx[0], (const int32_t *)(base + oType), cls);
+    const int passes = 8 + (type ? 1 : 0);
+    for (int q = 0; q < passes; ++q) {
+      const int a = q & 1;
+      const RadixDigit d = {keys[a], idx[a], q == 8 ? cls : nullptr, 8 * q};
+      k_radix_count<<<tiles, kRadixThreads>>>(d, n, tiles, hist);
+      k_radix_scan<<<256, kRadixThreads>>>(hist, tiles, totals);
+      k_radix_scatter<<<tiles, kRadixThreads>>>(d, n, tiles, hist, totals, keys[a ^ 1], idx[a ^ 1]);
     }
-    countLaunch(launches);
-    if (cudaGetLastError() != cudaSuccess) break;
-    if (cudaMemcpy(perm, idx, n * 4, cudaMemcpyDeviceToHost) != cudaSuccess) break;
-    st = FG_OK;
-    release();
-    return st;
-  } while (false);
-  const cudaError_t e = cudaGetLastError();
-  release();
+    const uint32_t *order = idx[passes & 1];
+    if (type) k_number<<<nb, 256>>>(order, n, cls, (uint64_t *)(base + oNum));
+    countLaunch(1 + 3 * passes + (type ? 1 : 0));
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    return type ? cudaMemcpy(num, base + oNum, n * 8, cudaMemcpyDeviceToHost) : cudaMemcpy(perm, order, n * 4, cudaMemcpyDeviceToHost);
+  };
+  const cudaError_t e = run();
+  cudaFree(base);
+  if (e == cudaSuccess) return FG_OK;
+  cudaGetLastError();
   setLastError(std::string("hilbert order: ") + cudaGetErrorString(e));
   return FG_ERR_CUDA;
 }
@@ -180,7 +234,7 @@ extern "C" int fg_hilbert_order(int32_t dim, uint64_t n, const float *pts, const
     setLastError("fg_hilbert_order: no CUDA device");
     return FG_ERR_NO_DEVICE;
   }
-  return hilbertOrderGpu(dim, n, pts, mn, mx, perm);
+  return hilbertOrderGpu(dim, n, pts, dim, mn, mx, perm, nullptr, nullptr);
 }
 
 extern "C" int fg_hilbert_numbering(int32_t dim, const double *bbox, uint64_t n_dofs, const float *xyz, const int32_t *assemble_type,
@@ -189,16 +243,9 @@ extern "C" int fg_hilbert_numbering(int32_t dim, const double *bbox, uint64_t n_
     setLastError("fg_hilbert_numbering: invalid arguments");
     return FG_ERR_ARG;
   }
-  std::vector<float> pts, bpts;
-  std::vector<uint64_t> ids, bids;
-  for (uint64_t i = 0; i < n_dofs; ++i) {
-    const int t = assemble_type[i];
-    if (t != FG_AT_UNKNOWN && t != FG_AT_UNKNOWN_BUBBLE) continue;
-    auto &P = t == FG_AT_UNKNOWN_BUBBLE ? bpts : pts;
-    (t == FG_AT_UNKNOWN_BUBBLE ? bids : ids).push_back(i);
-    for (int c = 0; c < dim; ++c) P.push_back(xyz[3 * i + c]);
-  }
-  const uint64_t nUnknown = ids.size() + bids.size(), nBubble = bids.size();
+  uint64_t nUnknown = 0;  // without any, nothing is numbered and no device is needed
+  for (uint64_t i = 0; i < n_dofs && !nUnknown; ++i)
+    nUnknown += assemble_type[i] == FG_AT_UNKNOWN || assemble_type[i] == FG_AT_UNKNOWN_BUBBLE;
   if (nUnknown == 0) return FG_OK;
   // the box widened by a relative 1e-6, as the reference does (DofsManager.cpp)
   float mn[3], mx[3];
@@ -206,11 +253,15 @@ extern "C" int fg_hilbert_numbering(int32_t dim, const double *bbox, uint64_t n_
     mn[c] = (float)(bbox[c] - 0.000001 * std::fabs(bbox[c]));
     mx[c] = (float)(bbox[3 + c] + 0.000001 * std::fabs(bbox[3 + c]));
   }
-  std::vector<uint32_t> perm(ids.size()), bperm(bids.size());
-  int st = fg_hilbert_order(dim, ids.size(), pts.data(), mn, mx, perm.data());
-  if (st) return st;
-  if ((st = fg_hilbert_order(dim, bids.size(), bpts.data(), mn, mx, bperm.data()))) return st;
-  for (size_t i = 0; i < perm.size(); ++i) num_dof[ids[perm[i]]] = i + 1;
-  for (size_t i = 0; i < bperm.size(); ++i) num_dof[bids[bperm[i]]] = nUnknown - nBubble + i + 1;
-  return FG_OK;
+  if (n_dofs >= (uint64_t(1) << 32) - 1) {
+    setLastError("fg_hilbert_numbering: more than 2^32 - 2 DOFs");
+    return FG_ERR_ARG;
+  }
+  int dev = 0;
+  if (cudaGetDeviceCount(&dev) != cudaSuccess || dev == 0) {
+    cudaGetLastError();
+    setLastError("fg_hilbert_numbering: no CUDA device");
+    return FG_ERR_NO_DEVICE;
+  }
+  return hilbertOrderGpu(dim, n_dofs, xyz, 3, mn, mx, nullptr, assemble_type, num_dof);
 }

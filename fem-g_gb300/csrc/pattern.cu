@@ -16,7 +16,18 @@
 // bitonic network and keeps the first of every run, once to count and once
 // to write. The result does not depend on the order of the entries, so it
 // is the reference's pattern bit for bit.
+//
+// The element DOF map is converted and checked on the device, and the row
+// starts and row pointers come from device scans; the host reads five words
+// and the two results. The columns go to plain host memory: page-locking 73 MB
+// (9.2 M nonzeros) and giving it back took 4.7 ms of 7.0, and its pages are
+// instead touched by all cores while the device writes the columns. 41,154
+// order-3 tetrahedra: 2.0 ms a call.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
+#include <cstdlib>
 #include <vector>
 
 #include "common.cuh"
@@ -26,6 +37,112 @@ namespace femg {
 constexpr uint32_t kPatNone = 0xFFFFFFFFu;
 
 __device__ __forceinline__ bool patRow(uint8_t t) { return t == FG_AT_UNKNOWN || t == FG_AT_UNKNOWN_BUBBLE || t == FG_AT_UNKNOWN_GLOBAL; }
+
+// What the host needs of the device's passes
+struct PatInfo {
+  unsigned long long total;  // of the last scan
+  uint32_t maxCount;         // largest value scanned
+  int bad;                   // an index out of range
+  int linkedBubbles;         // some linked bubble
+  int pad;
+};
+
+// The element DOF map as the passes below read it: rows' indices in 32 bits
+// (0 for other types) and the assemble types in bytes. A linked DOF is a row
+// and a column of its master (MatrixFactory.cpp:468-470, :481-483); a linked
+// bubble is a bubble row of its master's (:505).
+__global__ void k_pat_convert(const uint64_t *__restrict__ idx, const int32_t *__restrict__ type, int64_t count, uint64_t nRows,
+                              const uint64_t *__restrict__ linkedRow, uint64_t nLinked, uint32_t *__restrict__ ed,
+                              uint8_t *__restrict__ et, PatInfo *__restrict__ info) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= count) return;
+  // an entry out of range is marked and takes no part in what follows
+  et[k] = FG_AT_UNDEFINED;
+  ed[k] = 0u;
+  int t = type[k];
+  uint64_t v = idx[k];
+  if (t == FG_AT_LINKED || t == FG_AT_LINKED_BUBBLE) {
+    if (!linkedRow || v >= nLinked) {
+      atomicOr(&info->bad, 1);
+      return;
+    }
+    v = linkedRow[v];
+    if (t == FG_AT_LINKED_BUBBLE) atomicOr(&info->linkedBubbles, 1);
+    t = t == FG_AT_LINKED ? FG_AT_UNKNOWN : FG_AT_UNKNOWN_BUBBLE;
+  }
+  const bool row = t == FG_AT_UNKNOWN || t == FG_AT_UNKNOWN_BUBBLE || t == FG_AT_UNKNOWN_GLOBAL;
+  if (row && v >= nRows) {
+    atomicOr(&info->bad, 1);
+    return;
+  }
+  // (a value outside the enumeration is no row, whatever its low byte)
+  et[k] = t >= FG_AT_UNDEFINED && t <= FG_AT_LINKED_BUBBLE ? (uint8_t)t : (uint8_t)FG_AT_UNDEFINED;
+  if (row) ed[k] = (uint32_t)v;
+}
+
+// Exclusive scan of in[n] into out[n + 1] (64 bits), the total and the largest
+// value into info: sums of tiles, a scan of those by one block, and the tiles.
+constexpr int kScanThreads = 256, kScanTile = 2048;
+__device__ __forceinline__ uint64_t blockExclusive(uint64_t v, uint64_t *total) {  // over kScanThreads threads
+  __shared__ uint64_t warpSum[kScanThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t inc = v;
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint64_t o = __shfl_up_sync(0xffffffffu, inc, off);
+    if (lane >= off) inc += o;
+  }
+  __syncthreads();  // an earlier call's sums have been read
+  if (lane == 31) warpSum[warp] = inc;
+  __syncthreads();
+  uint64_t before = 0, all = 0;
+  for (int w = 0; w < kScanThreads / 32; ++w) {
+    if (w < warp) before += warpSum[w];
+    all += warpSum[w];
+  }
+  *total = all;
+  return before + inc - v;
+}
+__global__ void __launch_bounds__(kScanThreads) k_scan_sums(const uint32_t *__restrict__ in, uint64_t n, uint64_t *__restrict__ sums,
+                                                           PatInfo *__restrict__ info) {
+  uint64_t sum = 0, all;
+  uint32_t top = 0;
+  for (uint64_t k = (uint64_t)blockIdx.x * kScanTile + threadIdx.x; k < min(n, ((uint64_t)blockIdx.x + 1) * kScanTile); k += kScanThreads) {
+    sum += in[k];
+    top = max(top, in[k]);
+  }
+  blockExclusive(sum, &all);
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0 && top) atomicMax(&info->maxCount, top);
+  if (threadIdx.x == 0) sums[blockIdx.x] = all;
+}
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(uint64_t *__restrict__ sums, uint64_t tiles, PatInfo *__restrict__ info) {
+  uint64_t carry = 0;
+  for (uint64_t b = 0; b < tiles; b += kScanThreads) {
+    const uint64_t k = b + threadIdx.x;
+    uint64_t all;
+    const uint64_t ex = blockExclusive(k < tiles ? sums[k] : 0, &all);
+    if (k < tiles) sums[k] = carry + ex;
+    carry += all;
+  }
+  if (threadIdx.x == 0) info->total = carry;
+}
+__global__ void __launch_bounds__(kScanThreads) k_scan_write(const uint32_t *__restrict__ in, uint64_t n, const uint64_t *__restrict__ sums,
+                                                            uint64_t *__restrict__ out) {
+  constexpr int kPer = kScanTile / kScanThreads;  // consecutive values per thread
+  const uint64_t k0 = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kPer;
+  uint32_t v[kPer];
+  uint64_t sum = 0, all;
+  for (int i = 0; i < kPer; ++i) {
+    v[i] = k0 + i < n ? in[k0 + i] : 0u;
+    sum += v[i];
+  }
+  uint64_t at = sums[blockIdx.x] + blockExclusive(sum, &all);
+  for (int i = 0; i < kPer; ++i) {
+    if (k0 + i < n) out[k0 + i] = at;
+    at += v[i];
+    if (k0 + i + 1 == n) out[n] = at;
+  }
+}
 
 // Row counts and bubble aliases, thread per element. preAliased: the
 // aliases came from the host (linked bubbles: the bubble rows of a master
@@ -168,6 +285,69 @@ int devAlloc(DevBuf &b, size_t bytes) {
   return FG_OK;
 }
 
+int scanCounts(const uint32_t *in, uint64_t n, uint64_t *sums, uint64_t *out, PatInfo *info) {
+  FG_CUDA(cudaMemsetAsync(&info->maxCount, 0, sizeof(uint32_t)));
+  if (n == 0) {
+    FG_CUDA(cudaMemsetAsync(&info->total, 0, sizeof(info->total)));
+    FG_CUDA(cudaMemsetAsync(out, 0, sizeof(uint64_t)));
+    return FG_OK;
+  }
+  const uint64_t tiles = (n + kScanTile - 1) / kScanTile;
+  k_scan_sums<<<(unsigned)tiles, kScanThreads>>>(in, n, sums, info);
+  k_scan_tiles<<<1, kScanThreads>>>(sums, tiles, info);
+  k_scan_write<<<(unsigned)tiles, kScanThreads>>>(in, n, sums, out);
+  countLaunch(3);
+  FG_CUDA(cudaGetLastError());
+  return FG_OK;
+}
+
+// With linked bubbles, the rows that share one list: the reference's element
+// after element pointer assignment (MatrixFactory.cpp:505-535) puts every
+// bubble row of a master element and of the element linked to it on the list
+// of whichever bubble row was taken first; connecting the bubble rows of each
+// element gives the same groups in any element order. Each group's list is
+// kept on its smallest row.
+std::vector<uint32_t> bubbleAliases(const std::vector<uint32_t> &ed, const std::vector<uint8_t> &et, int64_t E, int n, uint64_t nRows) {
+  std::vector<uint32_t> root(nRows);
+  for (uint64_t r = 0; r < nRows; ++r) root[r] = (uint32_t)r;
+  auto find = [&](uint32_t r) {
+    while (root[r] != r) r = root[r] = root[root[r]];
+    return r;
+  };
+  for (int64_t e = 0; e < E; ++e) {
+    uint32_t first = kPatNone;
+    for (int i = 0; i < n; ++i) {
+      const size_t k = (size_t)e * n + i;
+      if (et[k] != FG_AT_UNKNOWN_BUBBLE) continue;
+      if (first == kPatNone) {
+        first = ed[k];
+        continue;
+      }
+      const uint32_t a = find(first), b = find(ed[k]);
+      if (a != b) root[std::max(a, b)] = std::min(a, b);
+    }
+  }
+  std::vector<uint32_t> al(nRows, kPatNone);
+  for (uint64_t r = 0; r < nRows; ++r)
+    if (find((uint32_t)r) != r) al[r] = find((uint32_t)r);
+  return al;
+}
+
+// Plain host memory for the columns (freed by fg_host_free), its pages made
+// present by all cores
+void *hostColumns(size_t bytes) {
+  constexpr size_t kHuge = size_t(2) << 20;
+  void *p = nullptr;
+  if (bytes < 2 * kHuge) return std::malloc(std::max<size_t>(bytes, 8));
+  if (posix_memalign(&p, kHuge, bytes) != 0) return nullptr;
+  madvise(p, bytes, MADV_HUGEPAGE);  // a hint
+  const size_t page = (size_t)std::max<long>(sysconf(_SC_PAGESIZE), 4096);
+  const int64_t pages = (int64_t)((bytes + page - 1) / page);
+#pragma omp parallel for schedule(static)
+  for (int64_t k = 0; k < pages; ++k) static_cast<volatile char *>(p)[(size_t)k * page] = 0;
+  return p;
+}
+
 }  // namespace
 
 extern "C" int fg_pattern_build(const uint64_t *elem_dof_idx, const int32_t *elem_dof_type, int64_t n_elements, int32_t n_dofs,
@@ -191,103 +371,80 @@ extern "C" int fg_pattern_build(const uint64_t *elem_dof_idx, const int32_t *ele
   const int n = n_dofs;
   const int64_t E = n_elements;
   const size_t en = (size_t)E * n;
-  std::vector<uint32_t> ed(en);
-  std::vector<uint8_t> et(en);
-  int bad = 0;
-  int64_t linkedBubbles = 0;
-  for (size_t k = 0; k < en; ++k) {
-    int t = elem_dof_type[k];
-    uint64_t v = elem_dof_idx[k];
-    if (t == FG_AT_LINKED || t == FG_AT_LINKED_BUBBLE) {
-      // a linked DOF is a row and a column of its master (MatrixFactory.cpp:468-470, :481-483);
-      // a linked bubble is a bubble row of its master's (:505)
-      if (!linked_row || v >= n_linked) {
-        ++bad;
-        continue;
-      }
-      v = linked_row[v];
-      if (t == FG_AT_LINKED_BUBBLE) ++linkedBubbles;
-      t = t == FG_AT_LINKED ? FG_AT_UNKNOWN : FG_AT_UNKNOWN_BUBBLE;
-    }
-    et[k] = (uint8_t)t;
-    const bool row = t == FG_AT_UNKNOWN || t == FG_AT_UNKNOWN_BUBBLE || t == FG_AT_UNKNOWN_GLOBAL;
-    if (row && v >= n_rows) ++bad;
-    ed[k] = row ? (uint32_t)v : 0u;
-  }
-  if (bad) {
-    setLastError("fg_pattern_build: a DOF index is not below n_rows (or a linked index not below n_linked)");
-    return FG_ERR_INDEX;
-  }
-  DevBuf dEd, dEt, dCnt, dAlias, dStart, dFill, dElem, dLen, dAi, dAj;
+  if (!linked_row) n_linked = 0;
+  // one device allocation for everything whose size is known here
+  const uint64_t scanTiles = (n_rows + kScanTile - 1) / kScanTile;
+  size_t bytes = 0;
+  auto part = [&](size_t b) {
+    const size_t at = bytes;
+    bytes += (b + 255) / 256 * 256;
+    return at;
+  };
+  const size_t oInfo = part(sizeof(PatInfo)), oIdx = part(en * 8), oType = part(en * 4), oLinked = part(n_linked * 8), oEd = part(en * 4),
+               oEt = part(en), oCnt = part(n_rows * 4), oFill = part(n_rows * 4), oAlias = part(n_rows * 4), oLen = part(n_rows * 4),
+               oStart = part((n_rows + 1) * 8), oAi = part((n_rows + 1) * 8), oSums = part(scanTiles * 8);
+  DevBuf arena, dElem, dAj;
   int st;
-  if ((st = devAlloc(dEd, en * 4)) || (st = devAlloc(dEt, en)) || (st = devAlloc(dCnt, n_rows * 4)) ||
-      (st = devAlloc(dAlias, n_rows * 4)) || (st = devAlloc(dStart, (n_rows + 1) * 8)) || (st = devAlloc(dFill, n_rows * 4)) ||
-      (st = devAlloc(dLen, n_rows * 4)) || (st = devAlloc(dAi, (n_rows + 1) * 8)))
-    return st;
-  uint32_t *cnt = (uint32_t *)dCnt.p, *alias = (uint32_t *)dAlias.p, *fill = (uint32_t *)dFill.p, *len = (uint32_t *)dLen.p;
-  uint64_t *rowStart = (uint64_t *)dStart.p, *dai = (uint64_t *)dAi.p;
-  FG_CUDA(cudaMemcpy(dEd.p, ed.data(), en * 4, cudaMemcpyHostToDevice));
-  FG_CUDA(cudaMemcpy(dEt.p, et.data(), en, cudaMemcpyHostToDevice));
-  FG_CUDA(cudaMemset(cnt, 0, n_rows * 4));
-  FG_CUDA(cudaMemset(fill, 0, n_rows * 4));
-  // With linked bubbles, the rows that share one list: the reference's
-  // element after element pointer assignment (MatrixFactory.cpp:505-535)
-  // puts every bubble row of a master element and of the element linked to
-  // it on the list of whichever bubble row was taken first; connecting the
-  // bubble rows of each element gives the same groups in any element order.
-  // Each group's list is kept on its smallest row.
-  const bool preAliased = linkedBubbles > 0;
-  if (preAliased) {
-    std::vector<uint32_t> root(n_rows);
-    for (uint64_t r = 0; r < n_rows; ++r) root[r] = (uint32_t)r;
-    auto find = [&](uint32_t r) {
-      while (root[r] != r) r = root[r] = root[root[r]];
-      return r;
-    };
-    for (int64_t e = 0; e < E; ++e) {
-      uint32_t first = kPatNone;
-      for (int i = 0; i < n; ++i) {
-        const size_t k = (size_t)e * n + i;
-        if (et[k] != FG_AT_UNKNOWN_BUBBLE) continue;
-        if (first == kPatNone) {
-          first = ed[k];
-          continue;
-        }
-        const uint32_t a = find(first), b = find(ed[k]);
-        if (a != b) root[std::max(a, b)] = std::min(a, b);
-      }
-    }
-    std::vector<uint32_t> al(n_rows, kPatNone);
-    for (uint64_t r = 0; r < n_rows; ++r)
-      if (find((uint32_t)r) != r) al[r] = find((uint32_t)r);
-    FG_CUDA(cudaMemcpy(alias, al.data(), n_rows * 4, cudaMemcpyHostToDevice));
-  } else {
-    FG_CUDA(cudaMemset(alias, 0xFF, n_rows * 4));
+  if ((st = devAlloc(arena, bytes))) return st;
+  uint8_t *base = (uint8_t *)arena.p;
+  PatInfo *info = (PatInfo *)(base + oInfo);
+  uint32_t *ed = (uint32_t *)(base + oEd), *cnt = (uint32_t *)(base + oCnt), *fill = (uint32_t *)(base + oFill),
+           *alias = (uint32_t *)(base + oAlias), *len = (uint32_t *)(base + oLen);
+  uint8_t *et = base + oEt;
+  uint64_t *rowStart = (uint64_t *)(base + oStart), *dai = (uint64_t *)(base + oAi), *sums = (uint64_t *)(base + oSums);
+  PatInfo host;
+  FG_CUDA(cudaMemsetAsync(info, 0, sizeof(PatInfo)));
+  if (n_rows) {
+    FG_CUDA(cudaMemsetAsync(cnt, 0, oAlias - oCnt));  // the counts and the fill positions
+    FG_CUDA(cudaMemsetAsync(alias, 0xFF, n_rows * 4));
   }
   const unsigned eb = (unsigned)std::max<int64_t>(1, (E + 255) / 256);
   if (E > 0) {
-    k_pat_count<<<eb, 256>>>((const uint32_t *)dEd.p, (const uint8_t *)dEt.p, E, n, cnt, alias, preAliased);
+    FG_CUDA(cudaMemcpyAsync(base + oIdx, elem_dof_idx, en * 8, cudaMemcpyHostToDevice));
+    FG_CUDA(cudaMemcpyAsync(base + oType, elem_dof_type, en * 4, cudaMemcpyHostToDevice));
+    if (n_linked) FG_CUDA(cudaMemcpyAsync(base + oLinked, linked_row, n_linked * 8, cudaMemcpyHostToDevice));
+    k_pat_convert<<<(unsigned)((en + 255) / 256), 256>>>((const uint64_t *)(base + oIdx), (const int32_t *)(base + oType), (int64_t)en,
+                                                         n_rows, n_linked ? (const uint64_t *)(base + oLinked) : nullptr, n_linked, ed,
+                                                         et, info);
     countLaunch();
+    FG_CUDA(cudaGetLastError());
   }
-  // row starts of the entry lists (host scan)
-  std::vector<uint32_t> h32(n_rows);
-  std::vector<uint64_t> h64(n_rows + 1, 0);
-  FG_CUDA(cudaMemcpy(h32.data(), cnt, n_rows * 4, cudaMemcpyDeviceToHost));
-  uint32_t maxCnt = 0;
-  for (uint64_t r = 0; r < n_rows; ++r) {
-    h64[r + 1] = h64[r] + h32[r];
-    maxCnt = std::max(maxCnt, h32[r]);
+  bool preAliased = false;
+  auto count = [&]() -> int {
+    if (E > 0) {
+      k_pat_count<<<eb, 256>>>(ed, et, E, n, cnt, alias, preAliased);
+      countLaunch();
+    }
+    int s2 = scanCounts(cnt, n_rows, sums, rowStart, info);
+    if (s2) return s2;
+    FG_CUDA(cudaMemcpy(&host, info, sizeof(PatInfo), cudaMemcpyDeviceToHost));
+    return FG_OK;
+  };
+  if ((st = count())) return st;
+  if (host.bad) {
+    setLastError("fg_pattern_build: a DOF index is not below n_rows (or a linked index not below n_linked)");
+    return FG_ERR_INDEX;
   }
-  FG_CUDA(cudaMemcpy(rowStart, h64.data(), (n_rows + 1) * 8, cudaMemcpyHostToDevice));
-  if ((st = devAlloc(dElem, h64[n_rows] * 4))) return st;
+  if (host.linkedBubbles) {
+    // rare: the groups on the host, and the counts again on the grouped rows
+    std::vector<uint32_t> hEd(en);
+    std::vector<uint8_t> hEt(en);
+    FG_CUDA(cudaMemcpy(hEd.data(), ed, en * 4, cudaMemcpyDeviceToHost));
+    FG_CUDA(cudaMemcpy(hEt.data(), et, en, cudaMemcpyDeviceToHost));
+    const std::vector<uint32_t> al = bubbleAliases(hEd, hEt, E, n, n_rows);
+    FG_CUDA(cudaMemcpy(alias, al.data(), n_rows * 4, cudaMemcpyHostToDevice));
+    FG_CUDA(cudaMemsetAsync(cnt, 0, n_rows * 4));
+    preAliased = true;
+    if ((st = count())) return st;
+  }
+  if ((st = devAlloc(dElem, host.total * 4))) return st;
   if (E > 0) {
-    k_pat_fill<<<eb, 256>>>((const uint32_t *)dEd.p, (const uint8_t *)dEt.p, E, n, rowStart, fill, (uint32_t *)dElem.p, alias,
-                            preAliased);
+    k_pat_fill<<<eb, 256>>>(ed, et, E, n, rowStart, fill, (uint32_t *)dElem.p, alias, preAliased);
     countLaunch();
   }
   // shared memory per warp: the largest candidate list, rounded to a power of two
   int cap = 1;
-  while ((uint64_t)cap < (uint64_t)maxCnt * n) cap <<= 1;
+  while ((uint64_t)cap < (uint64_t)host.maxCount * n) cap <<= 1;
   int wpb = 8;
   while (wpb > 1 && (size_t)cap * 4 * wpb > 96 * 1024) wpb >>= 1;
   const size_t smem = (size_t)cap * 4 * wpb;
@@ -299,35 +456,33 @@ extern "C" int fg_pattern_build(const uint64_t *elem_dof_idx, const int32_t *ele
   FG_CUDA(cudaFuncSetAttribute(k_pat_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const unsigned rb = (unsigned)std::min<uint64_t>(std::max<uint64_t>(1, (n_rows + wpb - 1) / wpb), (uint64_t)smCount() * 64);
   if (n_rows > 0) {
-    k_pat_rows<false><<<rb, 32 * wpb, smem>>>((const uint32_t *)dEd.p, (const uint8_t *)dEt.p, n, rowStart,
-                                               (const uint32_t *)dElem.p, alias, n_rows, cap, upper ? 1 : 0, len, nullptr, nullptr);
+    k_pat_rows<false><<<rb, 32 * wpb, smem>>>(ed, et, n, rowStart, (const uint32_t *)dElem.p, alias, n_rows, cap, upper ? 1 : 0, len,
+                                               nullptr, nullptr);
     k_pat_alias_len<<<(unsigned)((n_rows + 255) / 256), 256>>>(alias, n_rows, len);
     countLaunch(2);
     FG_CUDA(cudaGetLastError());
   }
-  FG_CUDA(cudaMemcpy(h32.data(), len, n_rows * 4, cudaMemcpyDeviceToHost));
-  ai[0] = 0;
-  for (uint64_t r = 0; r < n_rows; ++r) ai[r + 1] = ai[r] + h32[r];
-  const uint64_t nnz = ai[n_rows];
-  FG_CUDA(cudaMemcpy(dai, ai, (n_rows + 1) * 8, cudaMemcpyHostToDevice));
+  if ((st = scanCounts(len, n_rows, sums, dai, info))) return st;
+  FG_CUDA(cudaMemcpy(&host, info, sizeof(PatInfo), cudaMemcpyDeviceToHost));
+  const uint64_t nnz = host.total;
   if ((st = devAlloc(dAj, nnz * 8))) return st;
   if (n_rows > 0) {
-    k_pat_rows<true><<<rb, 32 * wpb, smem>>>((const uint32_t *)dEd.p, (const uint8_t *)dEt.p, n, rowStart,
-                                              (const uint32_t *)dElem.p, alias, n_rows, cap, upper ? 1 : 0, len, dai, (uint64_t *)dAj.p);
+    k_pat_rows<true><<<rb, 32 * wpb, smem>>>(ed, et, n, rowStart, (const uint32_t *)dElem.p, alias, n_rows, cap, upper ? 1 : 0, len, dai,
+                                              (uint64_t *)dAj.p);
     k_pat_alias_copy<<<(unsigned)((n_rows + 7) / 8), 256>>>(alias, n_rows, dai, (uint64_t *)dAj.p);
     countLaunch(2);
     FG_CUDA(cudaGetLastError());
   }
-  void *out = nullptr;
-  if (cudaMallocHost(&out, std::max<uint64_t>(nnz, 1) * 8) != cudaSuccess) {
-    cudaGetLastError();
+  void *out = hostColumns(nnz * 8);  // while the device writes the columns
+  if (!out) {
     setLastError("fg_pattern_build: host allocation failed");
     return FG_ERR_OOM;
   }
-  if (cudaMemcpy(out, dAj.p, nnz * 8, cudaMemcpyDeviceToHost) != cudaSuccess) {
+  if (cudaMemcpy(ai, dai, (n_rows + 1) * 8, cudaMemcpyDeviceToHost) != cudaSuccess ||
+      cudaMemcpy(out, dAj.p, nnz * 8, cudaMemcpyDeviceToHost) != cudaSuccess) {
     cudaGetLastError();
-    cudaFreeHost(out);
-    setLastError("fg_pattern_build: copy of the columns failed");
+    std::free(out);
+    setLastError("fg_pattern_build: copy of the pattern failed");
     return FG_ERR_CUDA;
   }
   *aj = (uint64_t *)out;

@@ -8,6 +8,7 @@ the library is missing or was not built.
 """
 import ctypes as C
 import os
+import weakref
 
 import numpy as np
 
@@ -637,10 +638,11 @@ def pattern_build(edof, etype, n_rows, upper=False, linked_row=None):
     check(L.fg_pattern_build(edof.ctypes.data, etype.ctypes.data, E, n, int(n_rows), ai.ctypes.data, C.byref(ajp),
                              1 if upper else 0, lrow.ctypes.data if lrow is not None and lrow.size else None,
                              0 if lrow is None else len(lrow)))
+    # the library's buffer itself, freed with the last array on it
     nnz = int(ai[-1])
-    aj = np.ctypeslib.as_array(C.cast(ajp, C.POINTER(C.c_uint64)), shape=(max(nnz, 1),))[:nnz].copy()
-    L.fg_host_free(ajp)
-    return ai, aj
+    buf = (C.c_uint64 * max(nnz, 1)).from_address(ajp.value)
+    weakref.finalize(buf, L.fg_host_free, ajp.value).atexit = False
+    return ai, np.frombuffer(buf, np.uint64)[:nnz]
 
 
 def hilbert_order(dim, pts, mn, mx):
