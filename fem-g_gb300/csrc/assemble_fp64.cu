@@ -340,6 +340,7 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 7)
   int *orient = reinterpret_cast<int *>(qsm + L.orient);
   const int64_t e0 = (int64_t)blockIdx.x * a.NE;
   const int live = (int)min((int64_t)a.NE, p.E - e0);
+  gridTrigger();
   if (KIND != kQuadFull && ke) fillPairs(pairs, n);
   quadElements<KIND == kQuadHcurl>(p, terms, e0, live, X, geom, orient);
   if (be)
@@ -641,6 +642,7 @@ __global__ void __launch_bounds__(kQuadThreads, UNIFORM ? 4 : 2)
   int *orient = reinterpret_cast<int *>(qsm + L.orient);
   const int64_t e0 = (int64_t)blockIdx.x * a.NE;
   const int live = (int)min((int64_t)a.NE, p.E - e0);
+  gridTrigger();
   fillPairs(pairs, ns);
   quadElements<false>(p, terms, e0, live, X, geom, orient);
   double acc[MAXP][NS];

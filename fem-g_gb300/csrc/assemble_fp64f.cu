@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(256) k_element_factored_fp64(const PlanDev p, 
   double *Ts = stage + EC * ncomp * nn2 + (EC * nn2 & 1);  // [kp][np]
   double *F = Ts + kp * np;                     // [kFacTile][fLd]
   uint16_t *pairs = reinterpret_cast<uint16_t *>(F + kFacTile * fLd);  // [np] i << 8 | j
+  gridTrigger();
   const int4 tile = tiles[blockIdx.x];
   const double *To = T + (size_t)tile.x * kp * nn2;
   for (int k = tid; k < np; k += 256) {

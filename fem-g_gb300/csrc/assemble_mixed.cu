@@ -195,6 +195,7 @@ __device__ __forceinline__ void factorsScalar(const PlanDev &p, const DevTerms *
 template <bool TENSOR>
 __global__ void k_factors(const PlanDev p, const DevTerms *__restrict__ terms, const int32_t *__restrict__ rankOf, float *__restrict__ A,
                           int ncomp, int rowsPerElem, int rowOff) {
+  gridTrigger();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e < p.E) factorsScalar<TENSOR>(p, terms, rankOf, A, ncomp, rowsPerElem, rowOff, e);
 }
@@ -300,6 +301,7 @@ __device__ __forceinline__ void factorsElastic(const PlanDev &p, const DevTerms 
 
 __global__ void k_factors_elastic(const PlanDev p, const DevTerms *__restrict__ terms, const int32_t *__restrict__ rankOf,
                                   float *__restrict__ A, int ncomp, int rowsPerElem, int rowOff) {
+  gridTrigger();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e < p.E) factorsElastic(p, terms, rankOf, A, ncomp, rowsPerElem, rowOff, e);
 }
@@ -372,6 +374,7 @@ __device__ __forceinline__ void factorsHcurl(const PlanDev &p, const DevTerms *_
 
 __global__ void k_factors_hcurl(const PlanDev p, const DevTerms *__restrict__ terms, const int32_t *__restrict__ rankOf,
                                 float *__restrict__ A, int ncomp, int rowsPerElem, int rowOff) {
+  gridTrigger();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e < p.E) factorsHcurl(p, terms, rankOf, A, ncomp, rowsPerElem, rowOff, e);
 }
@@ -579,12 +582,17 @@ __global__ void __launch_bounds__(kThreadsGemm, 2)
     t = sc.ctaStart[blockIdx.x];
     ce = sc.ctaStart[blockIdx.x + 1];
   }
+  gridTrigger();
   if (t < ce) {
     const int4 T = sc.tiles[t];
     if (tid == 0) gs = sc.probs[T.x];
     __syncthreads();
     loadB(gs, Bs, T.y, tid, bBar);
     bPending = 1;
+  }
+  gridWait();  // the factor rows
+  if (t < ce) {
+    const int4 T = sc.tiles[t];
     issueATile(sc, gs, As0, T.z, T.w, tid, &aBar[0]);
     aPending |= 1u;
   }
@@ -915,9 +923,13 @@ int launchContract(const void *probsDev, const int4 *tilesDev, const int32_t *ct
     sc.chunk = std::max(1, chunk);
   }
   ProfScope prof("k_contract_tf32x3", s);
-  k_contract_tf32x3<<<std::max(1, nCta), kThreadsGemm, smem, s>>>(sc, maxK3, tmemCols);
+  if (next) {  // a batch: its launches are also recorded in a graph
+    k_contract_tf32x3<<<std::max(1, nCta), kThreadsGemm, smem, s>>>(sc, maxK3, tmemCols);
+    FG_CUDA(cudaGetLastError());
+  } else {
+    FG_CUDA(launchDependent(true, k_contract_tf32x3, (unsigned)std::max(1, nCta), kThreadsGemm, smem, s, sc, maxK3, tmemCols));
+  }
   countLaunch();
-  FG_CUDA(cudaGetLastError());
   return FG_OK;
 }
 

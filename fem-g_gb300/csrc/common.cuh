@@ -60,6 +60,44 @@ inline cudaError_t allowSmem(K kern, size_t smem, SmemAllowance &a) {
   return e;
 }
 
+// Programmatic dependent launch: a kernel launched this way may start while
+// the one before it on the stream still runs, once all of that one's blocks
+// have started and said so (gridTrigger) or ended. It loads what no kernel of
+// the call writes (the plan's tables), then waits for the other's end and
+// memory (gridWait) before it reads its results or writes anything. After
+// anything but a kernel the launch is an ordinary one. It hides the launch and
+// the first loads: a mesh of 50 triangles, two kernels a call, 37.6 to
+// 34.9 us.
+template <typename... P, typename... A>
+inline cudaError_t launchDependent(bool early, void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A &&...args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute a[1];
+  a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = a;
+  // a caller's stream capture gets plain dependencies
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+  if (early && cudaStreamIsCapturing(s, &capture) != cudaSuccess) {
+    cudaGetLastError();
+    capture = cudaStreamCaptureStatusActive;
+  }
+  c.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kern, static_cast<P>(args)...);
+}
+__device__ __forceinline__ void gridTrigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void gridWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// p, but not known to be before the wait: a read-only load through it cannot
+// be moved ahead of the wait
+template <typename T>
+__device__ __forceinline__ T *afterWait(T *p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
+
 constexpr int kMaxDofs = 64;         // element DOFs (basis x multiplicity) handled on device
 constexpr int kMaxNodes = 10;        // geometric nodes per element
 constexpr int kMaxTerms = 6;

@@ -167,8 +167,12 @@ __device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *__restric
   KT vr[U][J * VW], vi[U][KCPLX ? J * VW : 1];
   double2 vb[U];  // the element vectors' entries (first lane of a row)
   loadRec(v.z, 0, (int)(v.w >> 16), cur);
-  loadKe(cur, vr, vi, vb);
   loadRec(v.z, U, (int)(v.w >> 16), nxt);
+  gridWait();  // the kernel that writes the element matrices and vectors
+  ke = afterWait(ke);
+  be = afterWait(be);
+  uD = afterWait(uD);
+  loadKe(cur, vr, vi, vb);
   __syncwarp();
   for (int64_t base = v0 + (blk * wpb + warp) * R; base < v1; base += stride) {
     const int64_t idx = base + sub;
@@ -324,6 +328,7 @@ struct GatherLaunch {
   GatherShape g;
   int slotBytes, kcplx;
   bool acc, simple;
+  bool early;  // may start before the element kernel ends
   int64_t blocks;
   cudaStream_t s;
   // a single plan
@@ -352,9 +357,8 @@ int launchGatherKernel(const GatherLaunch &a) {
   auto kern = k_gather<SlotT, KCPLX, KT, VW, J, BLOCKS, ACC, SIMPLE>;
   static SmemAllowance allowed;
   FG_CUDA(allowSmem(kern, a.g.smem, allowed));
-  kern<<<(unsigned)a.blocks, 32u * (unsigned)a.g.wpb, a.g.smem, a.s>>>(*a.p, (const KT *)a.ke, a.be, a.uD, a.values, a.rhs, a.g.lanes,
-                                                                      a.lay, a.v0, a.v1);
-  FG_CUDA(cudaGetLastError());
+  FG_CUDA(launchDependent(a.early, kern, (unsigned)a.blocks, 32u * (unsigned)a.g.wpb, a.g.smem, a.s, *a.p, (const KT *)a.ke, a.be, a.uD,
+                          a.values, a.rhs, a.g.lanes, a.lay, a.v0, a.v1));
   return FG_OK;
 }
 template <typename SlotT, bool KCPLX, typename KT, int VW, int J, bool BLOCKS>

@@ -140,8 +140,8 @@ __global__ void __launch_bounds__(256) k_gather_multi(const PlanDev p, const Mul
   Step cur, nxt;
   Values val;
   loadRec(v.z, 0, (int)(v.w >> 16), cur);
-  loadKe(cur, val);
   loadRec(v.z, U, (int)(v.w >> 16), nxt);
+  loadKe(cur, val);
   for (int64_t base = base0; base < nRows; base += stride) {
     const int64_t idx = base + sub;
     const bool live = laneLive && idx < nRows;
