@@ -283,25 +283,33 @@ __global__ void __launch_bounds__(256) k_gather_multi(const PlanDev p, const Mul
       }
     }
     if (in.rhs) {
-      double2 tot[GM];
+      // without fixed columns every right-hand side is the element vectors'
+      // sum, and zero without those: the products by the frequencies' factors
+      // would cost FP64 instructions on every row (a quarter of the pipe's
+      // time, and of the kernel's, at 8 frequencies)
+      if (SIMPLE || !in.uD) {
+        if (live && lt == 0)
+          for (int r = 0; r < in.R; ++r) in.rhs[r][v.x] = bsum;
+      } else {
+        double2 tot[GM];
 #pragma unroll
-      for (int gr = 0; gr < GM; ++gr) {
-        tot[gr] = dc[gr];
-        if (!SIMPLE && in.uD)
+        for (int gr = 0; gr < GM; ++gr) {
+          tot[gr] = dc[gr];
           for (int t = 1; t < L; ++t) {
             const int src = laneLive ? sub * L + t : lane;
             tot[gr].x += __shfl_sync(0xffffffffu, dc[gr].x, src);
             tot[gr].y += __shfl_sync(0xffffffffu, dc[gr].y, src);
           }
-      }
-      if (live && lt == 0)
-        for (int r = 0; r < in.R; ++r) {
-          double2 b = bsum;
-#pragma unroll
-          for (int gr = 0; gr < GM; ++gr)
-            if (gr < G) b = cadd(b, cmul(in.rcoef[r * G + gr], tot[gr]));
-          in.rhs[r][v.x] = b;
         }
+        if (live && lt == 0)
+          for (int r = 0; r < in.R; ++r) {
+            double2 b = bsum;
+#pragma unroll
+            for (int gr = 0; gr < GM; ++gr)
+              if (gr < G) b = cadd(b, cmul(in.rcoef[r * G + gr], tot[gr]));
+            in.rhs[r][v.x] = b;
+          }
+      }
     }
     __syncwarp();
     v = vN;
