@@ -424,8 +424,13 @@ __global__ void k_factors_hcurl(const PlanDev p, const DevTerms *__restrict__ te
 }
 
 // Factor rows of many plans in one launch: thread -> (job, element) through
-// the jobs' element offsets
-__global__ void k_factors_batch(const FactorJob *__restrict__ jobs, int nJobs, int64_t total) {
+// the jobs' element offsets.
+//
+// Four blocks per SM: left alone, the compiler gave the branches over the
+// terms' kinds 188 registers, so two blocks' loads were in flight. Over 12
+// problems of 384 to 24,576 tets: 64.1 us without the bound, 51.0 at four
+// blocks, 51.0, 50.5 and 51.8 at 6, 8 and 10, which spill more.
+__global__ void __launch_bounds__(128, 4) k_factors_batch(const FactorJob *__restrict__ jobs, int nJobs, int64_t total) {
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= total) return;
   int lo = 0, hi = nJobs - 1;
