@@ -46,17 +46,15 @@ sys.path.insert(0, ROOT)
 METRIC = "element matrices/s and CSR nnz/s: mixed vs FP64 GPU at <=1e-6 rel error, 1 GB300"
 
 # DRAM bytes (read + write) per CSR nonzero of one reduction launch on the 3D
-# P3 Helmholtz meshes, from ncu captures of the 30^3 x 6 mesh (162,000 tets,
-# 35,811,451 nonzeros); the per-launch traffic of other sizes of that family
-# is this figure times their nonzeros. k_gather: 555.2 MB read + 550.5 MB
-# written; k_gather_v4: 566.2 MB read + 548.5 MB written.
-GATHER_TRAFFIC_PER_NNZ_P3 = {"k_gather": (555.207680e6 + 550.488064e6) / 35811451,
-                             "k_gather_v4": (566.168064e6 + 548.542976e6) / 35811451}
+# P3 Helmholtz meshes, from an ncu capture of the 30^3 x 6 mesh (162,000 tets,
+# 35,811,451 nonzeros: 5.37 TB/s over 186.1 us); the per-launch traffic of
+# other sizes of that family is this figure times their nonzeros.
+GATHER_TRAFFIC_PER_NNZ_P3 = {"k_gather_v4": 999e6 / 35811451}
 
-# FP64-pipe activity of the plain FP64 element kernel (k_element_fp64<8, 0>,
-# the quadrature loop) in an ncu capture on the 30^3 x 6 P3 mesh: the loop is
+# FP64-pipe activity of the plain FP64 element kernel (k_element_fp64, the
+# quadrature loop) in an ncu capture on the 16^3 x 6 P3 mesh: the loop is
 # bound by GB300's FP64 pipe
-ELEMENT_FP64_PIPE_ACTIVE_P3 = 0.910
+ELEMENT_FP64_PIPE_ACTIVE_P3 = 0.921
 
 
 def load_femg():
