@@ -25,17 +25,20 @@ static int limitRows(int nc, bool vec4) {
 // the element matrices keep them aligned. J vectors per lane: one, so that
 // most rows share a warp (32 / L), but three from 12 vectors per row on (30
 // columns: 6 rows of 5 lanes instead of 2 of 15), and 3 or 5 single columns.
+// Rows of four columns take pieces of two: a row of one lane leaves a warp 32
+// rows, and few warps (16,464 order-1 tetrahedra 16.2 us against 12.5, 384,000
+// of them 30.7 against 27.0; with three components 26.6 against 20.4).
 GatherShape gatherShape(const PlanDev &p, int maxRowLen, int kcplx, int isFloat, KeLayout lay, int wpb) {
   GatherShape g;
   const int nc = p.nc;
   g.blocks3 = lay.kind == kKeBlocks3;
   if (g.blocks3) {
     const int nb = nc / 3;
-    g.VW = nb % 4 == 0 ? 4 : nb % 2 == 0 ? 2 : 1;
+    g.VW = nb % 4 == 0 && nb > 4 ? 4 : nb % 2 == 0 ? 2 : 1;
     g.J = 3;
     g.lanes.L = (nb + g.VW - 1) / g.VW;
   } else {
-    g.VW = isFloat && nc % 4 == 0 && lay.ld % 4 == 0 ? 4 : nc % 2 == 0 && lay.ld % 2 == 0 ? 2 : 1;
+    g.VW = isFloat && nc % 4 == 0 && nc > 4 && lay.ld % 4 == 0 ? 4 : nc % 2 == 0 && lay.ld % 2 == 0 ? 2 : 1;
     const int pieces = (nc + g.VW - 1) / g.VW;
     g.J = g.VW == 4 ? 1 : g.VW == 2 ? (pieces >= 12 ? 3 : 1) : (nc <= 24 ? 3 : 5);
     g.lanes.L = (pieces + g.J - 1) / g.J;
@@ -83,8 +86,12 @@ static int launchGatherRange(const PlanDev &p, const double *ke, int keComplex, 
   a.blocks = std::max<int64_t>(1, std::min<int64_t>(groups, (int64_t)smCount() * kGatherWarpsPerSm / a.g.wpb));
   // small systems only: blocks that come to an SM beside the contraction's run
   // with its division of L1 and shared memory, and 384,000 order-3 tetrahedra
-  // took 0.773 ms a call instead of 0.632
-  a.early = groups <= (int64_t)smCount() * kGatherWarpsPerSm / a.g.wpb;
+  // took 0.773 ms a call instead of 0.632. Nor where the contraction runs over
+  // more than one tile of 128 rows per SM, which the waiting blocks sit
+  // through: three components on 16,464 order-1 tetrahedra 86 us a call against
+  // 74, on 48,000 184 against 152; one component, 129 tiles, 26 against 35
+  const int64_t rows = keIsFloat ? p.E * (a.g.blocks3 ? 9 : 1) * (keComplex ? 2 : 1) : 0;
+  a.early = groups <= (int64_t)smCount() * kGatherWarpsPerSm / a.g.wpb && rows <= (int64_t)smCount() * 128;
   a.s = s;
   a.p = &p;
   a.ke = ke;
