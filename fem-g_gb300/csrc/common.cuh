@@ -90,8 +90,9 @@ inline cudaError_t launchDependent(bool early, void (*kern)(P...), unsigned grid
 }
 __device__ __forceinline__ void gridTrigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void gridWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// p, but not known to be before the wait: a read-only load through it cannot
-// be moved ahead of the wait
+// p, but not known to be before the wait: a load through it cannot be moved
+// ahead of the wait. The loads have to be coherent ones (no ld.global.nc):
+// what they read was written while this kernel may already have run.
 template <typename T>
 __device__ __forceinline__ T *afterWait(T *p) {
   asm volatile("" : "+l"(p)::"memory");

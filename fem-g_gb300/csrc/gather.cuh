@@ -39,22 +39,22 @@ namespace femg {
 
 constexpr uint32_t kRecNone = 0xFFFFFFFFu;  // packed (element, local row) of no entry
 
-// VW values of type KT, naturally aligned to the whole vector (16 bytes at most)
+// VW values of type KT, naturally aligned to the whole vector (16 bytes at
+// most), by ordinary (coherent) loads: the kernel that writes the element
+// matrices may still run when this one starts, so they are not read-only over
+// this kernel's life, which ld.global.nc (__ldg) asks for. asm, so that a load
+// is known to be from global memory and can be placed among the shared-memory
+// adds; it stays behind gridWait() because its address comes from afterWait().
 template <typename KT, int VW>
 __device__ __forceinline__ void loadValues(const KT *p, KT *out) {
-  if constexpr (sizeof(KT) * VW == 16) {
-    if constexpr (VW == 4) {
-      const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
-      out[0] = v.x, out[1] = v.y, out[2] = v.z, out[3] = v.w;
-    } else {
-      const double2 v = __ldg(reinterpret_cast<const double2 *>(p));
-      out[0] = v.x, out[1] = v.y;
-    }
-  } else if constexpr (VW == 2) {
-    const float2 v = __ldg(reinterpret_cast<const float2 *>(p));
-    out[0] = v.x, out[1] = v.y;
+  const size_t g = __cvta_generic_to_global(p);
+  if constexpr (sizeof(KT) == 4) {
+    if constexpr (VW == 4) asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(out[0]), "=f"(out[1]), "=f"(out[2]), "=f"(out[3]) : "l"(g));
+    else if constexpr (VW == 2) asm("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(out[0]), "=f"(out[1]) : "l"(g));
+    else asm("ld.global.f32 %0, [%1];" : "=f"(out[0]) : "l"(g));
   } else {
-    out[0] = __ldg(p);
+    if constexpr (VW == 2) asm("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(out[0]), "=d"(out[1]) : "l"(g));
+    else asm("ld.global.f64 %0, [%1];" : "=d"(out[0]) : "l"(g));
   }
 }
 
@@ -90,10 +90,9 @@ struct SlotWords {
 // share one, and there are no element vectors (p.cleanSlots, p.plainSlots, be
 // null): the hot case, in half the registers.
 template <typename SlotT, bool KCPLX, typename KT, int VW, int J, bool BLOCKS, bool ACC, bool SIMPLE>
-__device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *__restrict__ ke, const double2 *__restrict__ be,
-                                           const double2 *__restrict__ uD, double2 *__restrict__ values,
-                                           double2 *__restrict__ rhs, const GatherLanes g, KeLayout lay, int64_t blk, int64_t nblk,
-                                           int64_t v0, int64_t v1) {
+__device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *ke, const double2 *be, const double2 *uD,
+                                           double2 *__restrict__ values, double2 *__restrict__ rhs, const GatherLanes g,
+                                           KeLayout lay, int64_t blk, int64_t nblk, int64_t v0, int64_t v1) {
   constexpr int SS = KCPLX ? 2 : 1;
   constexpr int U = VW * J * (int)sizeof(KT) * SS <= 16 ? 2 : 1;  // entries per step
   constexpr uint32_t kIgnore = sizeof(SlotT) == 1 ? 0xFEu : kSlotIgnore, kFixed = sizeof(SlotT) == 1 ? 0xFFu : kSlotFixed;
@@ -146,7 +145,11 @@ __device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *__restric
           const uint32_t ib = i / 3, a = i - 3 * ib;
           row = (a * 3 * nb + ib) * nb;
         }
-        if (!SIMPLE && be && lt == 0) vb[u] = __ldg(&be[(size_t)e * n + i]);
+        if (!SIMPLE && be && lt == 0) {
+          double b[2];
+          loadValues<double, 2>(&be[(size_t)e * n + i].x, b);
+          vb[u] = make_double2(b[0], b[1]);
+        }
         const KT *K = ke + ((uint64_t)e * (SS * ld) + row);
 #pragma unroll
         for (int c = 0; c < J; ++c)
@@ -172,6 +175,10 @@ __device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *__restric
   ke = afterWait(ke);
   be = afterWait(be);
   uD = afterWait(uD);
+  if (ACC) {  // what the values and right-hand sides held before this plan
+    values = afterWait(values);
+    rhs = afterWait(rhs);
+  }
   loadKe(cur, vr, vi, vb);
   __syncwarp();
   for (int64_t base = v0 + (blk * wpb + warp) * R; base < v1; base += stride) {
@@ -304,8 +311,8 @@ constexpr int gatherBlocksPerSm(int laneBytes, bool simple) { return simple && l
 
 template <typename SlotT, bool KCPLX, typename KT, int VW, int J, bool BLOCKS, bool ACC, bool SIMPLE>
 __global__ void __launch_bounds__(256, gatherBlocksPerSm(VW * J * (int)sizeof(KT), SIMPLE))
-    k_gather(const PlanDev p, const KT *__restrict__ ke, const double2 *__restrict__ be, const double2 *__restrict__ uD,
-             double2 *__restrict__ values, double2 *__restrict__ rhs, const GatherLanes g, KeLayout lay, int64_t v0, int64_t v1) {
+    k_gather(const PlanDev p, const KT *ke, const double2 *be, const double2 *uD, double2 *__restrict__ values,
+             double2 *__restrict__ rhs, const GatherLanes g, KeLayout lay, int64_t v0, int64_t v1) {
   gatherRows<SlotT, KCPLX, KT, VW, J, BLOCKS, ACC, SIMPLE>(p, ke, be, uD, values, rhs, g, lay, blockIdx.x, gridDim.x, v0, v1);
 }
 
