@@ -13,19 +13,24 @@
 // GB300's FP64 pipe takes 64 cycles per warp instruction and scheduler,
 // whether one lane is active or 32, so what counts is the number of FP64
 // warp instructions and how full their lanes are. Hence:
-//  - The geometry and the coefficients of a point become one small matrix D
-//    in reference coordinates, e.g. w det c J^-1 J^-T, that maps the unknown's
-//    reference tables once (H = D t_j); an entry is then a plain dot product
-//    with the test function's reference table, Ke[i][j] += t_i . H_j.
+//  - At each point the functions are mapped once, to physical gradients (or
+//    curls and values) and, scaled by w det c, to what they are multiplied
+//    by; an entry is then a plain dot product. Both functions of a product are
+//    physical: through det J^-1 J^-T in reference coordinates the mapping
+//    would cost a little less, but on flat elements the large entries of that
+//    matrix cancel, and an entry's error grows as the square of the aspect
+//    ratio instead of the ratio (1:1,000: 5e-10 instead of 3e-13).
 //  - Blocks work on several elements, and every phase spreads its items over
-//    all threads: elements (Jacobians), (element, point) pairs (D), (element,
-//    point, function) triples (H), and (element, entry) pairs (the sums).
+//    all threads: elements (Jacobians), (element, point) pairs (D, the coefficients),
+//    (element, point, function) triples (H, the mapped functions), and
+//    (element, entry) pairs (the sums).
 //    The entries of all elements of a block are numbered through, so that
 //    small element matrices fill the lanes too.
 //
 // The element matrices and vectors then go through the deterministic CSR
 // reduction of gather.cu.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "common.cuh"
@@ -35,34 +40,43 @@ namespace femg {
 constexpr int kQuadThreads = 128;
 constexpr int kQuadMaxElems = 64;             // elements per block
 constexpr size_t kQuadSmem = 30 * 1024;       // shared memory of a block: seven blocks per SM
-constexpr int kQuadGeom = 31;                 // per element: J, J^-1, det, det J^-1 J^-T, J^T J / det (HCurl)
+// per element: det, J^-1, then J / det (HCurl), or J where the points' geometry
+// follows from it (modified elements)
+constexpr int kGeomDet = 0, kGeomJi = 1, kGeomJd = 10, kGeomJ = 10;
+__host__ __device__ constexpr int quadGeom(int affine, int own, bool hcurl) { return !affine ? 0 : own || hcurl ? 19 : 10; }
 
 // Shape and switches of one launch
 struct QuadArgs {
   int NE;          // elements per block
   int QD, QC;      // points per chunk of D, and of H within it
+  int nd;          // doubles per point of D: coefficients, then the point's own geometry
   int nEnt;        // entries accumulated per element: the upper triangle, or all n x nc
-  int comps;       // mask of the table components that contribute (see tableComps)
+  int comps;       // mask of the test functions' physical components that contribute
+  int flat;        // planar elements as they are: J is a 2 x 2 matrix beside the normal
+  int own;         // the geometry differs from point to point (curved or modified elements)
+  int ng;          // doubles per element of the geometry
+  int tensor;      // kQuadSym, kQuadHcurl: coefficients are symmetric tensors
   int uniform;     // the scalar bilinear coefficients are constant on each element
   int realSource;  // the scalar sources are real
   int needX;       // some coefficient or modificator reads the physical point
 };
 
-// Kinds of element matrices. The table components of a function: H1, the
-// reference gradient and the value (4); HCurl, the reference curl and value
-// (6). D: kQuadSym S (00 11 22 01 02 12) and the mass weight (7); kQuadHcurl
-// the same for curls and for values (12); kQuadFull a 4 x 4 matrix.
+// Kinds of element matrices. The components of a function: H1, the physical
+// gradient and the value (4); HCurl, curl and value (6). Coefficients of a
+// point, all times w det: kQuadSym and kQuadHcurl one per term kind, or the six
+// entries (00 11 22 01 02 12) of a tensor; kQuadFull M (9), b' (3), v (3), m.
 enum { kQuadSym = 0, kQuadHcurl = 1, kQuadFull = 2 };
 __host__ __device__ constexpr int quadComps(int kind) { return kind == kQuadHcurl ? 6 : 4; }
-__host__ __device__ constexpr int quadD(int kind) { return kind == kQuadSym ? 7 : kind == kQuadHcurl ? 12 : 16; }
+__host__ __device__ constexpr int quadCoefs(int kind, bool tensor) {
+  return kind == kQuadFull ? 16 : !tensor ? 2 : kind == kQuadHcurl ? 12 : 7;
+}
 
 // Offsets (in doubles) of a block's shared memory
 struct QuadLayout {
   int X, geom, coef, D, src, be, H, pairs, orient, total;
 };
-// nd: doubles per point, nh: doubles per (point, unknown function), n: test
-// functions (right-hand side entries), nU: unknown functions
-__host__ __device__ inline QuadLayout quadLayout(int NE, int QD, int QC, int nn, int n, int nU, int nd, int nh, bool be, int nPairs) {
+// ng: doubles per element, nd, nh: per point of D and H, n: right-hand side entries
+__host__ __device__ inline QuadLayout quadLayout(int NE, int QD, int QC, int nn, int n, int ng, int nd, int nh, bool be, int nPairs) {
   QuadLayout L;
   int o = 0;
   L.be = o;  // double2
@@ -70,7 +84,7 @@ __host__ __device__ inline QuadLayout quadLayout(int NE, int QD, int QC, int nn,
   L.X = o;
   o += NE * nn * 3;
   L.geom = o;
-  o += NE * kQuadGeom;
+  o += NE * ng;
   L.coef = o;
   o += NE * 6;
   L.D = o;
@@ -78,7 +92,7 @@ __host__ __device__ inline QuadLayout quadLayout(int NE, int QD, int QC, int nn,
   L.src = o;
   o += be ? NE * QD * 8 : 0;
   L.H = o;
-  o += NE * QC * nh * nU;
+  o += NE * QC * nh;
   L.pairs = o;
   o += (nPairs * 2 + 7) / 8;
   L.orient = o;
@@ -133,37 +147,16 @@ __device__ inline void scalarCoefs(const DevTerms *terms, int g, const CoefPoint
   }
 }
 
-// J^-1, det J^-1 J^-T and (HCurl fields) J^T J / det, six entries each (00 11
-// 22 01 02 12), from J and its determinant. With the cofactors C,
-// J^-1 = C^T / det, so det J^-1 J^-T = (C^T C) / det. One division: a lane's
-// FP64 instructions here cost the block as much as full warps' do.
-template <bool HCURL>
-__device__ inline void geomMaps(const double *J, double det, double *Ji, double *K6, double *M6) {
-  auto Jm = [&](int r, int c) { return J[3 * c + r]; };
-  double C[9];  // C[3a + r] = (adj J)(a, r)
-  C[0] = Jm(1, 1) * Jm(2, 2) - Jm(1, 2) * Jm(2, 1);
-  C[1] = Jm(0, 2) * Jm(2, 1) - Jm(0, 1) * Jm(2, 2);
-  C[2] = Jm(0, 1) * Jm(1, 2) - Jm(0, 2) * Jm(1, 1);
-  C[3] = Jm(1, 2) * Jm(2, 0) - Jm(1, 0) * Jm(2, 2);
-  C[4] = Jm(0, 0) * Jm(2, 2) - Jm(0, 2) * Jm(2, 0);
-  C[5] = Jm(0, 2) * Jm(1, 0) - Jm(0, 0) * Jm(1, 2);
-  C[6] = Jm(1, 0) * Jm(2, 1) - Jm(1, 1) * Jm(2, 0);
-  C[7] = Jm(0, 1) * Jm(2, 0) - Jm(0, 0) * Jm(2, 1);
-  C[8] = Jm(0, 0) * Jm(1, 1) - Jm(0, 1) * Jm(1, 0);
+// J / det
+__device__ inline void overDet(const double *J, double det, double *Jd) {
   const double id = 1.0 / det;
-  for (int k = 0; k < 9; ++k) Ji[k] = C[k] * id;
-  const int ab[6][2] = {{0, 0}, {1, 1}, {2, 2}, {0, 1}, {0, 2}, {1, 2}};
-  for (int k = 0; k < 6; ++k) {
-    const int a = ab[k][0], b = ab[k][1];
-    K6[k] = (C[3 * a] * C[3 * b] + C[3 * a + 1] * C[3 * b + 1] + C[3 * a + 2] * C[3 * b + 2]) * id;
-    if (HCURL) M6[k] = (J[3 * a] * J[3 * b] + J[3 * a + 1] * J[3 * b + 1] + J[3 * a + 2] * J[3 * b + 2]) * id;
-  }
+  for (int k = 0; k < 9; ++k) Jd[k] = J[k] * id;
 }
 
-// The same from the nodes of a planar 2D element: J is [[a b 0], [c d 0],
-// [0 0 s]] with s = +-1 the normal, so no square root, and one division
-template <bool HCURL>
-__device__ inline double planarMaps(int nn, bool p1, const double *X, const double *dN, double *J, double *Ji, double *K6, double *M6) {
+// J, its inverse and determinant from the nodes of a planar 2D element: J is
+// [[a b 0], [c d 0], [0 0 s]] with s = +-1 the normal, so no square root, and
+// one division
+__device__ inline double planarMaps(int nn, bool p1, const double *X, const double *dN, double *J, double *Ji) {
   double a = 0.0, b = 0.0, c = 0.0, d = 0.0;  // dx/du dy/du dx/dv dy/dv
   if (p1) {
     a = X[3] - X[0];
@@ -190,26 +183,13 @@ __device__ inline double planarMaps(int nn, bool p1, const double *X, const doub
   Ji[3] = -b * sid;
   Ji[4] = a * sid;
   Ji[8] = s;
-  const double aa = a * a + b * b, cc = c * c + d * d, ac = a * c + b * d;  // J^T J
-  K6[0] = cc * id;
-  K6[1] = aa * id;
-  K6[2] = det;
-  K6[3] = -ac * id;
-  K6[4] = K6[5] = 0.0;
-  if (HCURL) {
-    M6[0] = aa * id;
-    M6[1] = cc * id;
-    M6[2] = id;
-    M6[3] = ac * id;
-    M6[4] = M6[5] = 0.0;
-  }
   return det;
 }
 
 // Nodes and, for affine elements, the geometry of the block's elements
-// (J, J^-1, det, det J^-1 J^-T and J^T J / det)
 template <bool HCURL>
-__device__ inline void quadElements(const PlanDev &p, const DevTerms *terms, int64_t e0, int live, double *X, double *geom, int *orient) {
+__device__ inline void quadElements(const PlanDev &p, const DevTerms *terms, const QuadArgs &a, int64_t e0, int live, double *X,
+                                    double *geom, int *orient) {
   // the term list (its first 16 KB: the scalar terms) towards L1 while the
   // nodes come in: small meshes are bound by the latency of such loads
   static_assert(sizeof(DevTerms) >= 128 * kQuadThreads, "one 128-byte line per thread");
@@ -223,34 +203,31 @@ __device__ inline void quadElements(const PlanDev &p, const DevTerms *terms, int
   __syncthreads();
   if (p.affine) {
     for (int t = threadIdx.x; t < live; t += kQuadThreads) {
-      double *g = geom + t * kQuadGeom;
-      double J[9], Ji[9];
-      double det;
+      double *g = geom + t * a.ng;
+      double J[9], det;
       if (p.planar) {
-        det = planarMaps<HCURL>(p.nn, p.p1geom != 0, X + t * p.nn * 3, p.geoGrad, J, Ji, g + 19, g + 25);
+        det = planarMaps(p.nn, p.p1geom != 0, X + t * p.nn * 3, p.geoGrad, J, g + kGeomJi);
       } else {
         det = p.p1geom ? jacobianP1(p.dim, X + t * p.nn * 3, J) : jacobian(p.dim, p.nn, X + t * p.nn * 3, p.geoGrad, J);
-        geomMaps<HCURL>(J, det, Ji, g + 19, g + 25);
+        jacobianInverse(J, det, g + kGeomJi);
       }
-      for (int k = 0; k < 9; ++k) {
-        g[k] = J[k];
-        g[9 + k] = Ji[k];
-      }
-      g[18] = det;
+      g[kGeomDet] = det;
+      if (a.own)
+        for (int k = 0; k < 9; ++k) g[kGeomJ + k] = J[k];
+      else if (HCURL)
+        overDet(J, det, g + kGeomJd);
     }
     __syncthreads();
   }
 }
 
-// Geometry of one (element, point) for the terms of modificator group g, laid
-// out as an element's: that one where the Jacobian is constant and
-// unmodified, else formed in `own`. x: the physical point.
-constexpr int kGeomJ = 0, kGeomJi = 9, kGeomDet = 18, kGeomK = 19, kGeomM = 25;
+// det and the physical point x of one (element, point) for the terms of
+// modificator group g. own (null where the element's geometry holds, see
+// QuadArgs): the point's J^-1 and J / det
 template <bool HCURL>
-__device__ inline const double *quadPoint(const PlanDev &p, const DevTerms *terms, int g, int q, const double *X, const double *geom,
-                                          bool needX, double *own, double *x) {
+__device__ inline double quadPoint(const PlanDev &p, const DevTerms *terms, int g, int q, const double *X, const double *geom,
+                                   bool needX, double *own, double *x) {
   x[0] = x[1] = x[2] = 0.0;
-  const DevJacMod &m = terms->mods[g];
   if (needX)
     for (int k = 0; k < p.nn; ++k) {
       const double v = p.geoVal[q * p.nn + k];
@@ -258,18 +235,21 @@ __device__ inline const double *quadPoint(const PlanDev &p, const DevTerms *term
       x[1] += v * X[3 * k + 1];
       if (!p.planar || !zeroBits(X[2])) x[2] += v * X[3 * k + 2];
     }
-  if (p.affine && m.kind == FG_JACMOD_NONE) return geom;
-  double det;
+  if (!own) return geom[kGeomDet];
+  double J[9], det;
   if (p.affine) {
-    for (int k = 0; k < 9; ++k) own[k] = geom[k];
+    for (int k = 0; k < 9; ++k) J[k] = geom[kGeomJ + k];
     det = geom[kGeomDet];
+  } else if (p.planar) {
+    det = planarMaps(p.nn, false, X, p.geoGrad + (size_t)q * p.nn * 3, J, own);
   } else {
-    det = jacobian(p.dim, p.nn, X, p.geoGrad + (size_t)q * p.nn * 3, own);
+    det = jacobian(p.dim, p.nn, X, p.geoGrad + (size_t)q * p.nn * 3, J);
   }
-  if (m.kind != FG_JACMOD_NONE && !applyJacMod(m, x, own, det)) atomicOr(p.jmErr, 1);
-  geomMaps<HCURL>(own, det, own + kGeomJi, own + kGeomK, own + kGeomM);
-  own[kGeomDet] = det;
-  return own;
+  const DevJacMod &m = terms->mods[g];
+  if (m.kind != FG_JACMOD_NONE && !applyJacMod(m, x, J, det)) atomicOr(p.jmErr, 1);
+  if (m.kind != FG_JACMOD_NONE || p.affine || !p.planar) jacobianInverse(J, det, own);
+  if (HCURL) overDet(J, det, own + 9);
+  return det;
 }
 
 // Upper-triangle entry k -> (i << 8 | j), i <= j, row-major
@@ -285,54 +265,77 @@ __device__ inline void fillPairs(uint16_t *pairs, int n) {
   }
 }
 
-// h = S g; flat: g2 vanishes and h[2] is not wanted (triangles)
-__device__ __forceinline__ void sym3(const double *S, double g0, double g1, double g2, double *h, bool flat) {
+// The physical gradient J^-T g (M = J^-1), or curl J g / det (M = J / det).
+// flat: planar elements, the components of `comps` alone
+__device__ __forceinline__ void mapVector(const double *M, double g0, double g1, double g2, bool flat, int comps, double *o) {
   if (flat) {
-    h[0] = S[0] * g0 + S[3] * g1;
-    h[1] = S[3] * g0 + S[1] * g1;
+    o[0] = o[1] = o[2] = 0.0;
+    if (comps & 3) {
+      o[0] = M[0] * g0 + M[3] * g1;
+      o[1] = M[1] * g0 + M[4] * g1;
+    }
+    if (comps & 4) o[2] = M[8] * g2;
     return;
   }
-  h[0] = S[0] * g0 + S[3] * g1 + S[4] * g2;
-  h[1] = S[3] * g0 + S[1] * g1 + S[5] * g2;
-  h[2] = S[4] * g0 + S[5] * g1 + S[2] * g2;
+#pragma unroll
+  for (int r = 0; r < 3; ++r) o[r] = M[r] * g0 + M[3 + r] * g1 + M[6 + r] * g2;
+}
+// h = c g, c a scalar or the six entries of a symmetric tensor
+__device__ __forceinline__ void scaleVector(const double *c, bool tensor, const double *g, double *h) {
+  if (tensor) {
+    h[0] = c[0] * g[0] + c[3] * g[1] + c[4] * g[2];
+    h[1] = c[3] * g[0] + c[1] * g[1] + c[5] * g[2];
+    h[2] = c[4] * g[0] + c[5] * g[1] + c[2] * g[2];
+  } else {
+#pragma unroll
+    for (int r = 0; r < 3; ++r) h[r] = c[0] * g[r];
+  }
 }
 
 // The element matrices and vectors of blocks of NE elements.
-//   kQuadSym:   scalar H1, symmetric: D = (w det c J^-1 A J^-T, w det c_m)
+//   kQuadSym:   scalar H1, symmetric: G_i . (w det A G_j) + phi_i (w det m phi_j)
+//               with the physical gradients G = J^-T grad phi
 //   kQuadHcurl: HCurl values P = J^-T v and curls C = J c / det
 //               (FieldEvaluator<Form1/Form2>, src/term/evaluator/FieldEvaluator.h:59-105):
-//               D = (w J^T A J / det, w det J^-1 B J^-T)
+//               C_i . (w det A C_j) + P_i . (w det B P_j)
 //   kQuadFull:  scalar H1, terms whose element matrix is not symmetric (a
 //               general TensorFunction, VectorFunction terms) or a two-field
 //               plan (BilinearTerm with _field[0] != _field[1],
 //               src/term/BilinearTerm.cpp:304-343; test functions from the
 //               test tables, unknown functions from the unknown field's):
-//               Ke[i][j] = G_i . (M G_j + b' phi_j) + phi_i (v . G_j + m phi_j),
-//               D = w det [J^-1 M J^-T, J^-1 b'; (J^-1 v)^T, m].
+//               Ke[i][j] = G_i . w det (M G_j + b' phi_j) + phi_i w det (v . G_j + m phi_j).
+// H holds, per point, the unknown functions' rows (what is multiplied, per
+// part) and the test functions' rows.
 // CPLX: complex D. SPLIT: complex coefficients that are constant on each
 // element: the real integrals of the two term kinds are summed apart and
-// combined at the end, half the FP64 work of complex D. MASKED: some table
-// components vanish or have no term (a.comps); otherwise all contribute.
+// combined at the end, half the FP64 work of complex D. MASKED: some components
+// vanish or have no term (a.comps); otherwise all contribute.
 // Bound by the FP64 pipe: 82,944 tetrahedra of order 3 (24 points, real,
-// constant on each element) take 3.72 ms, of which the entries' products
+// constant on each element) take 3.91 ms, of which the entries' products
 // alone are 2.7 ms at one warp instruction per 64 cycles and scheduler; a warp
 // per element, with the geometry and coefficients on its first lane, took
-// 9.93 ms. Order 2 with complex coefficients that vary inside the elements
-// (55,566 tetrahedra): 1.32 ms, before 7.93. HCurl of order 1 (34,992
-// tetrahedra): 1.57 ms, before 5.32. Seven blocks per SM in 72 registers: the
-// phases of one block fill the barriers of the others, and the spills, which
-// are around the (element, point) phase, cost less than that. Three blocks in
-// 168 registers took 4.06, 1.49 and 1.67 ms, five 3.82, 1.40 and 1.58, eight
-// 3.71, 1.42 and 1.58.
+// 9.93 ms, and one function of each product left in reference coordinates
+// 3.72 ms (13 instructions to map a function instead of 10), at the loss of
+// accuracy told at the top. Order 2 with complex coefficients that vary inside
+// the elements (55,566 tetrahedra): 1.22 ms, with a warp per element 7.93.
+// HCurl of order 1 (34,992 tetrahedra): 1.67 ms, 5.32. Seven blocks per SM in
+// 72 registers: the phases of one block fill the barriers of the others, which
+// costs spills of 0.5 (real kQuadSym) to 2.4 KB a thread (complex kQuadHcurl,
+// MASKED), most around the (element, point) phase. Three blocks in 168
+// registers took 4.12, 1.42 and 1.76 ms, five 3.92, 1.42 and 1.72, six 3.90,
+// 1.40 and 1.67, eight 3.93, 1.21 and 1.67. A call of kQuadFull on 10,368
+// order-3 tetrahedra: 2.37 ms with seven, 2.33 with three, 2.17 with six, 2.32
+// with eight; of complex kQuadHcurl 0.584, 0.590, 0.584 and 0.586.
 template <int KIND, bool CPLX, bool SPLIT, bool MASKED, int MAXE>
 __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 7)
     k_element_fp64(const PlanDev p, const DevTerms *__restrict__ terms, const QuadArgs a, double *__restrict__ ke, double2 *__restrict__ be) {
-  constexpr int R = quadComps(KIND), ND = quadD(KIND);
-  constexpr int NC = CPLX ? 2 : 1;           // parts of D and H
+  constexpr int R = quadComps(KIND);
+  constexpr int NC = CPLX ? 2 : 1;           // parts of the coefficients
   constexpr int NA = (CPLX || SPLIT) ? 2 : 1;  // sums per entry
   extern __shared__ __align__(16) double qsm[];
   const int n = p.nb, nU = p.nbU, tid = threadIdx.x;
-  const QuadLayout L = quadLayout(a.NE, a.QD, a.QC, p.nn, n, nU, ND * NC, R * NC, be != nullptr, KIND == kQuadFull ? 0 : a.nEnt);
+  const int S = R * (NC * nU + n);  // doubles of H per point: unknown functions, then test functions
+  const QuadLayout L = quadLayout(a.NE, a.QD, a.QC, p.nn, n, a.ng, a.nd, S, be != nullptr, KIND == kQuadFull ? 0 : a.nEnt);
   double *X = qsm + L.X, *geom = qsm + L.geom, *D = qsm + L.D, *src = qsm + L.src, *H = qsm + L.H;
   double2 *bs = reinterpret_cast<double2 *>(qsm + L.be);
   double *coef = qsm + L.coef;
@@ -342,28 +345,30 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 7)
   const int live = (int)min((int64_t)a.NE, p.E - e0);
   gridTrigger();
   if (KIND != kQuadFull && ke) fillPairs(pairs, n);
-  quadElements<KIND == kQuadHcurl>(p, terms, e0, live, X, geom, orient);
+  quadElements<KIND == kQuadHcurl>(p, terms, a, e0, live, X, geom, orient);
   if (be)
     for (int t = tid; t < live * n; t += kQuadThreads) bs[t] = make_double2(0.0, 0.0);
 
-  // this thread's entries: test row in the tables, unknown column in H
+  // this thread's entries: the test and unknown functions' places in H (below
+  // 48 KB / 8 each), in one register
   double acc[NA][MAXE];
-  int offT[MAXE], offH[MAXE], mine = 0;
+  uint32_t off[MAXE];
+  int mine = 0;
 #pragma unroll
   for (int m = 0; m < MAXE; ++m) {
 #pragma unroll
     for (int c = 0; c < NA; ++c) acc[c][m] = 0.0;
-    offT[m] = offH[m] = 0;
+    off[m] = 0;
     const int k = tid + kQuadThreads * m;
     if (ke && k < live * a.nEnt) {
       const int el = k / a.nEnt, r = k - el * a.nEnt;
       const int i = KIND == kQuadFull ? r / nU : pairs[r] >> 8, j = KIND == kQuadFull ? r % nU : pairs[r] & 255;
-      offT[m] = orient[2 * el] * p.nq * n + i;
-      offH[m] = el * a.QC * (R * NC) * nU + j;
+      off[m] = (uint32_t)(el * a.QC * S + j) << 16 | (uint32_t)(el * a.QC * S + R * NC * nU + i);
       mine = m + 1;
     }
   }
-  const bool tensor = terms->tensorTerm >= 0 || terms->tensorMassTerm >= 0;
+  const int nCoef = quadCoefs(KIND, a.tensor != 0);
+  const bool flat = MASKED && a.flat;
   const int nG = terms->nMod > 1 ? terms->nMod : 1;
   for (int g = 0; g < nG; ++g) {
     if (a.uniform && ke)
@@ -382,9 +387,10 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 7)
       // D (and the source) of every (element, point)
       for (int t = tid; t < live * dn; t += kQuadThreads) {
         const int el = t / dn, qd = t - el * dn, q = d0 + qd;
-        double own[kQuadGeom], x[3];
-        const double *P = quadPoint<KIND == kQuadHcurl>(p, terms, g, q, X + el * p.nn * 3, geom + el * kQuadGeom, a.needX != 0, own, x);
-        const double w = p.w[q], wd = w * P[kGeomDet];
+        double x[3];
+        double *d = D + (size_t)(el * a.QD + qd) * a.nd;
+        const double wd = p.w[q] * quadPoint<KIND == kQuadHcurl>(p, terms, g, q, X + el * p.nn * 3, geom + el * a.ng, a.needX != 0,
+                                                                 a.own ? d + nCoef * NC : nullptr, x);
         CoefPoint cp = {e0 + el, x, nullptr, 0, q, p.nq};
         if (KIND != kQuadHcurl) {  // field-node coefficients read the point's row of the basis table
           cp.phi = p.bval + ((size_t)orient[2 * el] * p.nq + q) * n;
@@ -399,43 +405,30 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 7)
         } else {
           scalarCoefs(terms, g, cp, c);
         }
-        double *d = D + (size_t)(el * a.QD + qd) * (ND * NC);
         if (!ke) {
-          // the right-hand side alone: no D
+          // the right-hand side alone: no coefficients
         } else if (KIND != kQuadFull) {
-          double2 A[6], B[6];
-          if (tensor) {
+          if (a.tensor) {
+            double2 A[6], B[6];
             tensorAt(terms, terms->tensorTerm, terms->tensor, g, cp, c[0], A);
             if (KIND == kQuadHcurl) tensorAt(terms, terms->tensorMassTerm, terms->tensorMass, g, cp, c[1], B);
-          }
 #pragma unroll
-          for (int part = 0; part < NC; ++part) {
-            const double cg = w * (part ? c[0].y : c[0].x), cm = w * (part ? c[1].y : c[1].x);
-            double *dp = d + part * ND;
-            if (tensor) {
-              double F[6];
-              if (KIND == kQuadSym) {
-                congruence6(P + kGeomJi, A, part, F);
-                for (int k = 0; k < 6; ++k) dp[k] = wd * F[k];
-                dp[6] = cm * P[kGeomDet];
-              } else {
-                congruence6(P + kGeomJ, A, part, F);
-                for (int k = 0; k < 6; ++k) dp[k] = w * F[k] / P[kGeomDet];
-                congruence6(P + kGeomJi, B, part, F);
-                for (int k = 0; k < 6; ++k) dp[6 + k] = wd * F[k];
-              }
-            } else if (KIND == kQuadSym) {
-              for (int k = 0; k < 6; ++k) dp[k] = cg * P[kGeomK + k];
-              dp[6] = cm * P[kGeomDet];
-            } else {
+            for (int part = 0; part < NC; ++part) {
+              double *dp = d + part * nCoef;
               for (int k = 0; k < 6; ++k) {
-                dp[k] = cg * P[kGeomM + k];
-                dp[6 + k] = cm * P[kGeomK + k];
+                dp[k] = wd * (part ? A[k].y : A[k].x);
+                if (KIND == kQuadHcurl) dp[6 + k] = wd * (part ? B[k].y : B[k].x);
               }
+              if (KIND == kQuadSym) dp[6] = wd * (part ? c[1].y : c[1].x);
+            }
+          } else {
+#pragma unroll
+            for (int part = 0; part < NC; ++part) {
+              d[2 * part] = wd * (part ? c[0].y : c[0].x);
+              d[2 * part + 1] = wd * (part ? c[1].y : c[1].x);
             }
           }
         } else {
-          const double *Ji = P + kGeomJi;
           double2 A6[6], M[9], v[3], vb[3];
           tensorAt(terms, terms->tensorTerm, terms->tensor, g, cp, c[0], A6);  // c_gg I (+ the symmetric tensor term)
           const int sym[9] = {0, 3, 4, 3, 1, 5, 4, 5, 2};
@@ -458,16 +451,12 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 7)
           }
 #pragma unroll
           for (int part = 0; part < NC; ++part) {
-            double *dp = d + part * ND;
+            double *dp = d + part * nCoef;
             auto re = [&](double2 z) { return part ? z.y : z.x; };
-            for (int r = 0; r < 3; ++r) {
-              double QM[3];  // row r of J^-1 M
-              for (int s = 0; s < 3; ++s)
-                QM[s] = Ji[3 * r] * re(M[s]) + Ji[3 * r + 1] * re(M[3 + s]) + Ji[3 * r + 2] * re(M[6 + s]);
-              for (int s = 0; s < 3; ++s)
-                dp[4 * r + s] = wd * (QM[0] * Ji[3 * s] + QM[1] * Ji[3 * s + 1] + QM[2] * Ji[3 * s + 2]);
-              dp[4 * r + 3] = wd * (Ji[3 * r] * re(vb[0]) + Ji[3 * r + 1] * re(vb[1]) + Ji[3 * r + 2] * re(vb[2]));
-              dp[12 + r] = wd * (Ji[3 * r] * re(v[0]) + Ji[3 * r + 1] * re(v[1]) + Ji[3 * r + 2] * re(v[2]));
+            for (int k = 0; k < 9; ++k) dp[k] = wd * re(M[k]);
+            for (int k = 0; k < 3; ++k) {
+              dp[9 + k] = wd * re(vb[k]);
+              dp[12 + k] = wd * re(v[k]);
             }
             dp[15] = wd * re(c[1]);
           }
@@ -480,15 +469,14 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 7)
           s[0] = wd * f.x;
           s[1] = wd * f.y;
           if (KIND == kQuadFull) {
-            const double *Ji = P + kGeomJi;
             double2 sg[3] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
             if (terms->srcGradTerm >= 0 && terms->t[terms->srcGradTerm].mod == g) {
               const double2 fc = evalAt(terms->t[terms->srcGradTerm].coef, cp);
               for (int k = 0; k < 3; ++k) sg[k] = cmul(fc, evalAt(terms->srcGrad[k], cp));
             }
             for (int r = 0; r < 3; ++r) {
-              s[2 + r] = wd * (Ji[3 * r] * sg[0].x + Ji[3 * r + 1] * sg[1].x + Ji[3 * r + 2] * sg[2].x);
-              s[5 + r] = wd * (Ji[3 * r] * sg[0].y + Ji[3 * r + 1] * sg[1].y + Ji[3 * r + 2] * sg[2].y);
+              s[2 + r] = wd * sg[r].x;
+              s[5 + r] = wd * sg[r].y;
             }
           }
         }
@@ -507,8 +495,11 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 7)
             if (!a.realSource) b.y += s[1] * ph;
             if (KIND == kQuadFull && terms->srcGradTerm >= 0) {
               const double *gr = p.bgrad + 3 * row;
-              b.x += s[2] * gr[0] + s[3] * gr[1] + s[4] * gr[2];
-              b.y += s[5] * gr[0] + s[6] * gr[1] + s[7] * gr[2];
+              const double *Ji = a.own ? D + (size_t)(el * a.QD + qd) * a.nd + nCoef * NC : geom + el * a.ng + kGeomJi;
+              double G[3];
+              mapVector(Ji, gr[0], gr[1], gr[2], false, 7, G);
+              b.x += s[2] * G[0] + s[3] * G[1] + s[4] * G[2];
+              b.y += s[5] * G[0] + s[6] * G[1] + s[7] * G[2];
             }
           }
           bs[t] = b;
@@ -517,33 +508,47 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 7)
       for (int q0 = d0; ke && q0 < d0 + dn; q0 += a.QC) {
         const int qn = min(a.QC, d0 + dn - q0);
         if (q0 > d0) __syncthreads();  // H has been read
-        // H = D t_j of every (element, point, unknown function)
-        for (int t = tid; t < live * qn * nU; t += kQuadThreads) {
-          const int ep = t / nU, j = t - ep * nU, el = ep / qn, qc = ep - el * qn, q = q0 + qc;
-          const size_t row = ((size_t)orient[2 * el + 1] * p.nq + q) * nU + j;
-          const double *d = D + (size_t)(el * a.QD + q - d0) * (ND * NC);
-          double *h = H + (size_t)(el * a.QC + qc) * (R * NC) * nU + j;
-          const double *gr = p.bgradU + 3 * row;
-          const double g0 = gr[0], g1 = gr[1], g2 = gr[2];
-          double v[3] = {0.0, 0.0, 0.0};
+        // H of every (element, point, function): the unknown functions, which
+        // are the test functions too but in two-field plans
+        const int nF = KIND == kQuadFull && p.coupled ? nU + n : nU;
+        for (int t = tid; t < live * qn * nF; t += kQuadThreads) {
+          const int ep = t / nF, f = t - ep * nF, el = ep / qn, qc = ep - el * qn, q = q0 + qc;
+          const bool testOnly = KIND == kQuadFull && f >= nU;
+          const double *d = D + (size_t)(el * a.QD + q - d0) * a.nd;
+          const double *Ji = a.own ? d + nCoef * NC : geom + el * a.ng + kGeomJi;
+          double *h = H + (size_t)(el * a.QC + qc) * S;
+          const size_t row = testOnly ? ((size_t)orient[2 * el] * p.nq + q) * n + f - nU : ((size_t)orient[2 * el + 1] * p.nq + q) * nU + f;
+          const double *gr = (testOnly ? p.bgrad : p.bgradU) + 3 * row;
+          const double *va = testOnly ? p.bval : p.bvalU;
+          double *ht = h + R * NC * nU + (testOnly ? f - nU : f);
+          h += f;
+          double G[3], v[3];
           if (KIND == kQuadHcurl) {
-            v[0] = p.bvalU[3 * row];
-            v[1] = p.bvalU[3 * row + 1];
-            v[2] = p.bvalU[3 * row + 2];
+            const double *Jd = a.own ? Ji + 9 : geom + el * a.ng + kGeomJd;
+            if (!MASKED || (a.comps & 7)) mapVector(Jd, gr[0], gr[1], gr[2], flat, a.comps, G);
+            if (!MASKED || (a.comps & 56)) mapVector(Ji, va[3 * row], va[3 * row + 1], va[3 * row + 2], flat, a.comps >> 3, v);
           } else {
-            v[0] = p.bvalU[row];
+            if (KIND == kQuadFull || !MASKED || (a.comps & 7)) mapVector(Ji, gr[0], gr[1], gr[2], flat, KIND == kQuadFull ? 7 : a.comps, G);
+            v[0] = va[row];
           }
+          if (KIND != kQuadFull || testOnly || !p.coupled) {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+              if (!MASKED || (a.comps >> r & 1)) ht[r * n] = r < 3 ? G[r] : v[r - 3];
+          }
+          if (testOnly) continue;
 #pragma unroll
           for (int part = 0; part < NC; ++part) {
-            const double *dp = d + part * ND;
+            const double *dp = d + part * nCoef;
             double o[6];
             if (KIND == kQuadFull) {
 #pragma unroll
-              for (int r = 0; r < 4; ++r) o[r] = dp[4 * r] * g0 + dp[4 * r + 1] * g1 + dp[4 * r + 2] * g2 + dp[4 * r + 3] * v[0];
+              for (int r = 0; r < 3; ++r) o[r] = dp[3 * r] * G[0] + dp[3 * r + 1] * G[1] + dp[3 * r + 2] * G[2] + dp[9 + r] * v[0];
+              o[3] = dp[12] * G[0] + dp[13] * G[1] + dp[14] * G[2] + dp[15] * v[0];
             } else {
-              if (!MASKED || (a.comps & 7)) sym3(dp, g0, g1, g2, o, MASKED && KIND == kQuadSym && !(a.comps & 4));
-              if (KIND == kQuadSym) o[3] = dp[6] * v[0];
-              else if (!MASKED || (a.comps & 56)) sym3(dp + 6, v[0], v[1], v[2], o + 3, false);
+              if (!MASKED || (a.comps & 7)) scaleVector(dp, a.tensor != 0, G, o);
+              if (KIND == kQuadSym) o[3] = dp[nCoef - 1] * v[0];
+              else if (!MASKED || (a.comps & 56)) scaleVector(dp + nCoef / 2, a.tensor != 0, v, o + 3);
             }
 #pragma unroll
             for (int r = 0; r < R; ++r)
@@ -554,17 +559,15 @@ __global__ void __launch_bounds__(kQuadThreads, MAXE > 10 ? 2 : 7)
         // Ke[i][j] += t_i . H_j. The next D may be written meanwhile: it is
         // read after the barrier that follows.
         for (int qc = 0; qc < qn; ++qc) {
-          const double *bg = p.bgrad + 3 * (size_t)(q0 + qc) * n;
-          const double *bv = p.bval + (size_t)(KIND == kQuadHcurl ? 3 : 1) * (q0 + qc) * n;
-          const double *Hq = H + (size_t)qc * (R * NC) * nU;
+          const double *Hq = H + (size_t)qc * S;
 #pragma unroll
           for (int m = 0; m < MAXE; ++m)
             if (m < mine) {
-              const double *gi = bg + 3 * offT[m], *vi = bv + (KIND == kQuadHcurl ? 3 : 1) * offT[m], *h = Hq + offH[m];
+              const double *ti = Hq + (off[m] & 0xFFFFu), *h = Hq + (off[m] >> 16);
 #pragma unroll
               for (int r = 0; r < R; ++r) {
                 if (MASKED && !(a.comps >> r & 1)) continue;
-                const double t = r < 3 ? gi[r] : vi[r - 3];
+                const double t = ti[r * n];
                 if (SPLIT) {
                   acc[r < 3 ? 0 : NA - 1][m] = fma(t, h[r * nU], acc[r < 3 ? 0 : NA - 1][m]);
                 } else {
@@ -636,7 +639,7 @@ __global__ void __launch_bounds__(kQuadThreads, UNIFORM ? 4 : 2)
   constexpr int NS = UNIFORM ? 10 : 19 * NC;       // sums per pair
   extern __shared__ __align__(16) double qsm[];
   const int ns = p.nb, n = 3 * ns, tid = threadIdx.x;
-  const QuadLayout L = quadLayout(a.NE, a.QD, a.QC, p.nn, 0, ns, ND, NH, false, a.nEnt);
+  const QuadLayout L = quadLayout(a.NE, a.QD, a.QC, p.nn, 0, a.ng, ND, NH * ns, false, a.nEnt);
   double *X = qsm + L.X, *geom = qsm + L.geom, *D = qsm + L.D, *H = qsm + L.H, *coef = qsm + L.coef;
   uint16_t *pairs = reinterpret_cast<uint16_t *>(qsm + L.pairs);
   int *orient = reinterpret_cast<int *>(qsm + L.orient);
@@ -644,7 +647,7 @@ __global__ void __launch_bounds__(kQuadThreads, UNIFORM ? 4 : 2)
   const int live = (int)min((int64_t)a.NE, p.E - e0);
   gridTrigger();
   fillPairs(pairs, ns);
-  quadElements<false>(p, terms, e0, live, X, geom, orient);
+  quadElements<false>(p, terms, a, e0, live, X, geom, orient);
   double acc[MAXP][NS];
   int offI[MAXP], offJ[MAXP], rowI[MAXP], mine = 0;
 #pragma unroll
@@ -680,11 +683,12 @@ __global__ void __launch_bounds__(kQuadThreads, UNIFORM ? 4 : 2)
       const int dn = min(a.QD, p.nq - d0);
       for (int t = tid; t < live * dn; t += kQuadThreads) {
         const int el = t / dn, qd = t - el * dn, q = d0 + qd;
-        double own[kQuadGeom], x[3];
-        const double *P = quadPoint<false>(p, terms, g, q, X + el * p.nn * 3, geom + el * kQuadGeom, a.needX != 0, own, x);
+        double x[3];
         double *d = D + (size_t)(el * a.QD + qd) * ND;
-        const double wd = p.w[q] * P[kGeomDet];
-        for (int k = 0; k < 9; ++k) d[k] = P[kGeomJi + k];
+        const double wd = p.w[q] * quadPoint<false>(p, terms, g, q, X + el * p.nn * 3, geom + el * a.ng, a.needX != 0,
+                                                    a.own ? d : nullptr, x);
+        if (!a.own)
+          for (int k = 0; k < 9; ++k) d[k] = geom[el * a.ng + kGeomJi + k];
         d[9] = wd;
         if (!UNIFORM) {
           double2 c[3];
@@ -815,48 +819,59 @@ __global__ void __launch_bounds__(kQuadThreads, UNIFORM ? 4 : 2)
 // Elements per block and points per chunk: the fewest FP64 instructions that
 // an SM's fullest warps run one after the other. A block takes, per point,
 // one product per table component for every entry of a thread (comps), hCost
-// instructions per round of (element, point, function) triples, dCost per
-// round of (element, point) pairs, and about 60 for the elements' geometry; an
-// SM runs blocks / SMs of them. So small meshes get few elements per block
-// (all SMs busy), large ones what fills the rounds best. D is formed for QD
-// points at a time, H for what the remaining shared memory holds.
-// Measured: 55,566 order-2 tetrahedra, complex D inside the elements, 1.31 to
-// 1.33 ms with 6, 9 or 24 elements, whose rounds are full, 1.43 with 12 and
-// 1.74 with 18.
-static bool quadShape(const PlanDev &p, int nEnt, int n, int nU, int nd, int nh, bool be, int nPairs, int maxItems, int comps,
-                      int hCost, int dCost, QuadArgs *a) {
+// instructions per round of (element, point, function) triples of a chunk,
+// dCost per round of (element, point) pairs, about as long as kBarrier
+// instructions at each barrier, and about 60 for the elements' geometry; an
+// SM runs blocks / SMs of them, of which those that are resident at once hide
+// each other's gaps (kBusy: how busy one alone keeps the pipe). So small
+// meshes get few elements per block, large ones what fills the rounds best. D
+// is formed for QD points at a time, H for QC of these.
+// Measured: with kBusy 0.3 and 0.6, and barriers of 12 instructions, a dozen
+// calls take the same time but for 10 to 35% more on one or two small meshes
+// each; without the blocks' overlap (kBusy 1) triangles of order 3 (8,192)
+// take 125 us a call instead of 101, of order 6 (512) 232 instead of 170.
+static bool quadShape(const PlanDev &p, int nEnt, int n, int nF, int nd, int nh, bool be, int nPairs, int maxItems, int comps,
+                      int hCost, int dCost, int blocksPerSm, QuadArgs *a) {
+  constexpr int kBarrier = 4;
+  constexpr double kBusy = 0.45;
   const int64_t sms = smCount();
-  auto bytes = [&](int NE, int QD, int QC) { return (size_t)quadLayout(NE, QD, QC, p.nn, n, nU, nd, nh, be, nPairs).total * 8; };
+  auto bytes = [&](int NE, int QD, int QC) { return (size_t)quadLayout(NE, QD, QC, p.nn, n, a->ng, nd, nh, be, nPairs).total * 8; };
   auto rounds = [](int64_t items) { return (items + kQuadThreads - 1) / kQuadThreads; };
-  auto even = [&](int chunks) { return (p.nq + chunks - 1) / chunks; };
+  auto parts = [](int of, int by) { return (of + by - 1) / by; };
   double best = 0.0;
   a->NE = 0;
   for (int NE = 1; NE <= kQuadMaxElems && (int64_t)NE * nEnt <= (int64_t)kQuadThreads * maxItems; ++NE) {
-    // the fewest chunks of D that fit beside two points of H, or one or two more
-    int chunks = 1;
-    while (chunks < p.nq && bytes(NE, even(chunks), std::min(2, even(chunks))) > kQuadSmem) ++chunks;
-    if (bytes(NE, even(chunks), 1) > kQuadSmem && NE > 1) break;
-    const int64_t blocks = (p.E + NE - 1) / NE;
-    for (int c = chunks; c <= chunks + 2 && c <= p.nq; ++c) {
-      const int64_t d = (int64_t)((p.nq + even(c) - 1) / even(c)) * rounds((int64_t)NE * even(c)) * dCost;
-      const int64_t block = rounds((int64_t)NE * nEnt) * p.nq * comps + rounds((int64_t)NE * p.nq * nU) * hCost + d + 60;
-      const double cost = (double)((blocks + sms - 1) / sms) * (double)block;
-      if (a->NE == 0 || cost < best) {
-        best = cost;
-        a->NE = NE;
-        a->QD = even(c);
+    if (NE > 1 && bytes(NE, 1, 1) > kQuadSmem) break;
+    const int64_t blocks = (p.E + NE - 1) / NE, perSm = (blocks + sms - 1) / sms;
+    const int resident = (int)std::min<int64_t>(perSm, blocksPerSm);
+    const double busy = 1.0 - std::pow(1.0 - kBusy, resident);
+    for (int c = 1, last = 0; c <= p.nq; ++c) {
+      const int QD = parts(p.nq, c), nD = parts(p.nq, QD);
+      if (QD == last || bytes(NE, QD, 1) > kQuadSmem) continue;
+      last = QD;
+      int QC = std::min(QD, 16);
+      while (QC > 1 && bytes(NE, QD, QC) > kQuadSmem) --QC;
+      const int least = parts(QD, QC);
+      for (int h = least; h <= least + 3 && h <= QD; ++h) {
+        QC = parts(QD, h);
+        const int nH = parts(QD, QC);
+        const int64_t block = rounds((int64_t)NE * nEnt) * p.nq * comps + nD * nH * rounds((int64_t)NE * QC * nF) * hCost +
+                              nD * rounds((int64_t)NE * QD) * dCost + 60 + kBarrier * nD * (1 + nH);
+        const double cost = (double)perSm * (double)block / busy;
+        if (a->NE == 0 || cost < best) {
+          best = cost;
+          a->NE = NE;
+          a->QD = QD;
+          a->QC = QC;
+        }
       }
     }
   }
-  if (a->NE == 0 || bytes(a->NE, a->QD, 1) > kQuadSmem) {
+  if (a->NE == 0) {
     // the widest element matrices: one element and one point at a time
-    a->NE = a->QD = 1;
+    a->NE = a->QD = a->QC = 1;
     if (nEnt > kQuadThreads * maxItems || bytes(1, 1, 1) > 48 * 1024) return false;
   }
-  int QC = std::min(a->QD, 16);
-  while (QC > 1 && bytes(a->NE, a->QD, QC) > kQuadSmem) --QC;
-  const int parts = (a->QD + QC - 1) / QC;
-  a->QC = (a->QD + parts - 1) / parts;
   a->nEnt = nEnt;
   return true;
 }
@@ -905,11 +920,14 @@ static int quadFail() {
 template <int KIND, bool CPLX, bool SPLIT, bool MASKED, int MAXE>
 static int quadLaunch(const PlanDev &p, const DevTerms *dterms, QuadArgs a, int nEnt, int coefCost, double *ke, double2 *be, cudaStream_t s) {
   constexpr int NC = CPLX ? 2 : 1;
-  const int nPairs = KIND == kQuadFull ? 0 : nEnt, nd = quadD(KIND) * NC, nh = quadComps(KIND) * NC;
-  const int hCost = (KIND == kQuadSym ? 10 : KIND == kQuadHcurl ? 18 : 16) * NC;
-  if (!quadShape(p, nEnt, p.nb, p.nbU, nd, nh, be != nullptr, nPairs, MAXE, quadComps(KIND) * NC, hCost, nd + coefCost, &a))
+  const int nPairs = KIND == kQuadFull ? 0 : nEnt, nh = quadComps(KIND) * (NC * p.nbU + p.nb);
+  a.nd = quadCoefs(KIND, a.tensor != 0) * NC + (a.own ? (KIND == kQuadHcurl ? 18 : 9) : 0);
+  const int map = a.flat ? 5 : 9, scale = a.tensor ? 15 : 3;
+  const int nF = p.coupled ? p.nb + p.nbU : p.nbU;  // functions mapped per point
+  const int hCost = KIND == kQuadSym ? map + (scale + 1) * NC : KIND == kQuadHcurl ? 2 * (map + scale * NC) : map + 16 * NC * p.nbU / nF;
+  if (!quadShape(p, nEnt, p.nb, nF, a.nd, nh, be != nullptr, nPairs, MAXE, quadComps(KIND) * NC, hCost, a.nd + coefCost, MAXE > 10 ? 2 : 7, &a))
     return quadFail();
-  const size_t smem = (size_t)quadLayout(a.NE, a.QD, a.QC, p.nn, p.nb, p.nbU, nd, nh, be != nullptr, nPairs).total * 8;
+  const size_t smem = (size_t)quadLayout(a.NE, a.QD, a.QC, p.nn, p.nb, a.ng, a.nd, nh, be != nullptr, nPairs).total * 8;
   k_element_fp64<KIND, CPLX, SPLIT, MASKED, MAXE>
       <<<(unsigned)((p.E + a.NE - 1) / a.NE), kQuadThreads, smem, s>>>(p, dterms, a, ke, be);
   countLaunch();
@@ -924,7 +942,16 @@ static int quadKind(const PlanDev &p, const DevTerms &terms, const DevTerms *dte
   QuadArgs a;
   std::memset(&a, 0, sizeof(a));
   const int full = (1 << quadComps(KIND)) - 1;
+  a.own = !p.affine || terms.hasJacMod;
+  a.ng = quadGeom(p.affine, a.own, KIND == kQuadHcurl);
+  a.flat = p.planar && !terms.hasJacMod;
+  a.tensor = KIND != kQuadFull && (terms.tensorTerm >= 0 || terms.tensorMassTerm >= 0);
   a.comps = p.tableComps & ((u.grad ? 7 : 0) | (u.mass ? full & ~7 : 0));
+  // mapping mixes a vector's components, but for planar elements those of the
+  // plane with the normal one
+  const int inPlane = a.flat ? 3 : 7;
+  for (int v = 0; v < (KIND == kQuadHcurl ? 6 : 3); v += 3)
+    if (a.comps >> v & inPlane) a.comps |= inPlane << v;
   a.uniform = !u.pointBilinear;
   a.realSource = u.realSource;
   a.needX = (ke && u.pointBilinear) || (be && u.pointSource) || terms.hasJacMod;
@@ -947,8 +974,9 @@ template <bool UNIFORM, bool CPLX, int MAXP>
 static int quadElastic(const PlanDev &p, const DevTerms *dterms, QuadArgs a, int nEnt, double *ke, double2 *be, cudaStream_t s) {
   constexpr int NC = (!UNIFORM && CPLX) ? 2 : 1, ND = 10 + (UNIFORM ? 0 : 3 * NC), NH = UNIFORM ? 7 : 3 + 7 * NC;
   const int sums = UNIFORM ? 10 : 19 * NC;
-  if (!quadShape(p, nEnt, 0, p.nb, ND, NH, false, nEnt, MAXP, sums, 9 + NH, ND + (UNIFORM ? 0 : 80), &a)) return quadFail();
-  const size_t smem = (size_t)quadLayout(a.NE, a.QD, a.QC, p.nn, 0, p.nb, ND, NH, false, nEnt).total * 8;
+  a.nd = ND;
+  if (!quadShape(p, nEnt, 0, p.nb, ND, NH * p.nb, false, nEnt, MAXP, sums, 9 + NH, ND + (UNIFORM ? 0 : 80), UNIFORM ? 4 : 2, &a)) return quadFail();
+  const size_t smem = (size_t)quadLayout(a.NE, a.QD, a.QC, p.nn, 0, a.ng, ND, NH * p.nb, false, nEnt).total * 8;
   k_element_elastic_fp64<UNIFORM, CPLX, MAXP><<<(unsigned)((p.E + a.NE - 1) / a.NE), kQuadThreads, smem, s>>>(p, dterms, a, ke, be);
   countLaunch();
   FG_CUDA(cudaGetLastError());
@@ -1001,6 +1029,8 @@ static int launchElementKernels(fg_plan *plan, const DevTerms &terms, const DevT
     std::memset(&a, 0, sizeof(a));
     a.comps = (u.grad ? 1 : 0) | (u.mass ? 2 : 0);
     a.needX = u.pointBilinear || terms.hasJacMod;
+    a.own = !p.affine || terms.hasJacMod;
+    a.ng = quadGeom(p.affine, a.own, false);
     // the element's sums are scaled once at the end: one group of terms
     a.uniform = !u.pointBilinear && terms.nMod <= 1;
     const bool cplx = terms.complexKe != 0;
