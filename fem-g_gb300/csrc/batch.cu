@@ -162,9 +162,9 @@ int uploadJobs(GatherClass &c, cudaStream_t s) {
 }
 
 int runGatherClass(fg_batch *b, GatherClass &c, cudaStream_t s) {
-  bool simple = true;
-  for (size_t k = 0; k < c.probs.size(); ++k) simple = simple && gatherSimple(c.jobsHost[k].p, c.jobsHost[k].be);
-  return launchGatherBatch(c.jobsDev, (int)c.probs.size(), c.blocks, c.slotBytes, c.kcplx, b->mixed ? 1 : 0, c.shape, simple, s);
+  int mode = kGatherClean;
+  for (size_t k = 0; k < c.probs.size(); ++k) mode = std::min(mode, gatherMode(c.jobsHost[k].p, c.jobsHost[k].be));
+  return launchGatherBatch(c.jobsDev, (int)c.probs.size(), c.blocks, c.slotBytes, c.kcplx, b->mixed ? 1 : 0, c.shape, mode, s);
 }
 
 int runElements(fg_batch *b, cudaStream_t s) {

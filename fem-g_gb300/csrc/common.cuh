@@ -345,15 +345,20 @@ struct GatherShape {
   size_t smem = 0;
   bool ok = false;
 };
-// wpb (warps per block) <= 0: the default
-GatherShape gatherShape(const PlanDev &p, int maxRowLen, int kcplx, int keIsFloat, KeLayout lay, int wpb);
-// whether the reduction's hot kernel (gather.cuh, SIMPLE) applies to real element matrices
-inline bool gatherSimple(const PlanDev &p, const void *be) { return p.cleanSlots && p.plainSlots && !p.lscale && !be; }
+// wpb (warps per block) <= 0: the default; acc: the rows are added to
+GatherShape gatherShape(const PlanDev &p, int maxRowLen, int kcplx, int keIsFloat, KeLayout lay, int wpb, bool acc = false);
+// the leanest kernel of the reduction that covers a plan and its element
+// vectors (gather.cuh, MODE); kernels cover what those after them cover
+enum { kGatherGeneral = 0, kGatherOpen = 1, kGatherClean = 2 };
+inline int gatherMode(const PlanDev &p, const void *be) {
+  if (p.lscale || be || !p.plainSlots) return kGatherGeneral;
+  return p.cleanSlots ? kGatherClean : p.nFixed ? kGatherGeneral : kGatherOpen;
+}
 // the records of the visiting order, from its (element, local row) list
 int buildRecords(const PlanDev &p, const uint32_t *visitElem, int64_t entries, uint32_t *rec);
-// simple: gatherSimple() of every job
+// mode: the least gatherMode() of the jobs
 int launchGatherBatch(const GatherJob *jobsDev, int nJobs, int64_t blocks, int slotBytes, int kcplx, int keIsFloat,
-                      const GatherShape &g, bool simple, cudaStream_t s);
+                      const GatherShape &g, int mode, cudaStream_t s);
 
 // One problem (element bucket) of a tensor-core contraction launch
 struct GemmProblem {

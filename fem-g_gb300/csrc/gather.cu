@@ -27,8 +27,12 @@ static int limitRows(int nc, bool vec4) {
 // columns: 6 rows of 5 lanes instead of 2 of 15), and 3 or 5 single columns.
 // Rows of four columns take pieces of two: a row of one lane leaves a warp 32
 // rows, and few warps (16,464 order-1 tetrahedra 16.2 us against 12.5, 384,000
-// of them 30.7 against 27.0; with three components 26.6 against 20.4).
-GatherShape gatherShape(const PlanDev &p, int maxRowLen, int kcplx, int isFloat, KeLayout lay, int wpb) {
+// of them 30.7 against 27.0; with three components 26.6 against 20.4). At most
+// eight rows where they add to what is there: it is read row after row at the
+// end (three components on 16,464 order-1 tetrahedra 77 us a call, with 16 rows
+// 86; one component on 82,944 of them 51.5 and 54.6), but in complex FP64, where
+// eight take longer (63.7 and 59.5).
+GatherShape gatherShape(const PlanDev &p, int maxRowLen, int kcplx, int isFloat, KeLayout lay, int wpb, bool acc) {
   GatherShape g;
   const int nc = p.nc;
   g.blocks3 = lay.kind == kKeBlocks3;
@@ -44,6 +48,7 @@ GatherShape gatherShape(const PlanDev &p, int maxRowLen, int kcplx, int isFloat,
     g.lanes.L = (pieces + g.J - 1) / g.J;
   }
   g.lanes.R = 32 / g.lanes.L;
+  if (acc && (isFloat || !kcplx)) g.lanes.R = std::min(g.lanes.R, 8);
   const size_t rowBytes = (size_t)std::max(maxRowLen, 1) * (kcplx ? 2 : 1) * (isFloat ? 4 : 8);
   const bool vec4 = isFloat && !kcplx && !g.blocks3 && nc % 4 == 0 && nc <= 32 && p.slotBytes == 1;
   g.ok = rowBytes * limitRows(nc, vec4) <= kGatherSmemMax;
@@ -73,7 +78,7 @@ static int launchGatherRange(const PlanDev &p, const double *ke, int keComplex, 
   }
   GatherLaunch a;
   std::memset(&a, 0, sizeof(a));
-  a.g = gatherShape(p, p.maxRowLen, keComplex, keIsFloat, lay, 0);
+  a.g = gatherShape(p, p.maxRowLen, keComplex, keIsFloat, lay, 0, acc);
   if (!a.g.ok) {
     setLastError("gather: CSR row too long for shared memory");
     return FG_ERR_UNSUPPORTED;
@@ -81,9 +86,14 @@ static int launchGatherRange(const PlanDev &p, const double *ke, int keComplex, 
   a.slotBytes = p.slotBytes;
   a.kcplx = keComplex;
   a.acc = acc;
-  a.simple = gatherSimple(p, be);
+  a.mode = gatherMode(p, be);
   const int64_t groups = (v1 - v0 + a.g.rowsPerBlock - 1) / a.g.rowsPerBlock;
   a.blocks = std::max<int64_t>(1, std::min<int64_t>(groups, (int64_t)smCount() * kGatherWarpsPerSm / a.g.wpb));
+  a.capped = a.blocks < groups;
+  // complex FP32 in 16-byte pieces: on large plans the general kernel, 16
+  // warps per SM in place of 28 (order 3, 105,456 tetrahedra 350 us a call and
+  // 368, 48,000 179 and 182; 10,368, which fit the grid, 69 and 62)
+  if (keIsFloat && keComplex && a.g.VW == 4 && !a.g.blocks3 && a.capped && !acc && a.mode == kGatherClean) a.mode = kGatherGeneral;
   // small systems only: blocks that come to an SM beside the contraction's run
   // with its division of L1 and shared memory, and 384,000 order-3 tetrahedra
   // took 0.773 ms a call instead of 0.632. Nor where the contraction runs over
@@ -141,7 +151,7 @@ int gatherToOutputs(fg_plan *plan, const double *ke, int keComplex, int keIsFloa
 }
 
 int launchGatherBatch(const GatherJob *jobsDev, int nJobs, int64_t blocks, int slotBytes, int kcplx, int keIsFloat,
-                      const GatherShape &g, bool simple, cudaStream_t s) {
+                      const GatherShape &g, int mode, cudaStream_t s) {
   if (blocks <= 0) return FG_OK;
   countLaunch();
   GatherLaunch a;
@@ -151,7 +161,7 @@ int launchGatherBatch(const GatherJob *jobsDev, int nJobs, int64_t blocks, int s
   a.kcplx = kcplx;
   a.blocks = blocks;
   a.s = s;
-  a.simple = simple;
+  a.mode = mode;
   a.jobs = jobsDev;
   a.nJobs = nJobs;
   ProfScope prof(g.VW == 4 && !g.blocks3 ? "k_gather_batch_v4" : "k_gather_batch", s);

@@ -33,6 +33,9 @@
 // scalar adds through atomics and narrow stores); 162,000 of them in FP64
 // 0.240 ms (0.365); 55,566 order-2 ones, complex FP64 0.091 ms (0.106).
 #pragma once
+#include <algorithm>
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace femg {
@@ -86,14 +89,17 @@ struct SlotWords {
 // VW columns. BLOCKS (compound fields on the tensor-core path): it owns the
 // scalar columns VW lt .. VW lt + VW - 1 of the three component blocks
 // (J = 3), which are 3 VW consecutive DOF columns and so consecutive slots.
-// SIMPLE: every slot is a column of the row, no two columns of an element row
-// share one, and there are no element vectors (p.cleanSlots, p.plainSlots, be
-// null): the hot case, in half the registers.
-template <typename SlotT, bool KCPLX, typename KT, int VW, int J, bool BLOCKS, bool ACC, bool SIMPLE>
+// MODE: kGatherClean and kGatherOpen are for plans without linked DOFs and
+// fixed columns whose element rows have no two columns in one slot
+// (p.plainSlots), and no element vectors: half the registers of
+// kGatherGeneral. kGatherClean: every slot is a column of the row
+// (p.cleanSlots); kGatherOpen: some columns are not stored (upper storage).
+template <typename SlotT, bool KCPLX, typename KT, int VW, int J, bool BLOCKS, bool ACC, int MODE>
 __device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *ke, const double2 *be, const double2 *uD,
                                            double2 *__restrict__ values, double2 *__restrict__ rhs, const GatherLanes g,
                                            KeLayout lay, int64_t blk, int64_t nblk, int64_t v0, int64_t v1) {
   constexpr int SS = KCPLX ? 2 : 1;
+  constexpr bool SIMPLE = MODE != kGatherGeneral;
   constexpr int U = VW * J * (int)sizeof(KT) * SS <= 16 ? 2 : 1;  // entries per step
   constexpr uint32_t kIgnore = sizeof(SlotT) == 1 ? 0xFEu : kSlotIgnore, kFixed = sizeof(SlotT) == 1 ? 0xFFu : kSlotFixed;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -106,7 +112,7 @@ __device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *ke, const
   KT *A = Aw + (laneLive ? sub : 0) * p.maxRowLen * SS;
   const int n = p.n, nc = p.nc, nb = BLOCKS ? p.nb : nc;
   const uint32_t ld = (uint32_t)lay.ld;  // entries per component
-  const bool clean = SIMPLE || p.cleanSlots != 0, plain = SIMPLE || p.plainSlots != 0;
+  const bool clean = MODE == kGatherClean || (!SIMPLE && p.cleanSlots != 0), plain = SIMPLE || p.plainSlots != 0;
   const uint8_t *recs = p.rec;
   const uint32_t recLd = (uint32_t)p.recLd;
   bool ok[J];  // the lane's pieces that exist
@@ -190,6 +196,18 @@ __device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *ke, const
     const int steps = max(1, ((int)__reduce_max_sync(0xffffffffu, (unsigned)cnt) + U - 1) / U);
     Step nextRow;
     loadRec(vN.z, 0, cntN, nextRow);
+    if (ACC) {  // what the rows hold, towards L2 while they are summed
+#pragma unroll 1
+      for (int r = lane >> g.lgOL; r - (lane >> g.lgOL) < R; r += 32 >> g.lgOL) {
+        const int rc = r < R ? r : 0;
+        const int rLen = __shfl_sync(0xffffffffu, len, rc * L);
+        const uint32_t start = __shfl_sync(0xffffffffu, v.y, rc * L);
+        // eight values to a line of 128 bytes
+        if (r < R)
+          for (int s = 8 * lo; s < rLen + 7; s += 8 * g.OL)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(values + ((size_t)start + min(s, rLen - 1))));
+      }
+    }
     double2 dc = make_double2(0.0, 0.0), bsum = make_double2(0.0, 0.0);
 #pragma unroll 1
     for (int st = 0; st < steps; ++st) {
@@ -236,7 +254,13 @@ __device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *ke, const
                 // plan says otherwise; successive element rows are ordered by
                 // the __syncwarp below
                 KT *at = A + (int)s * SS;
-                if (plain) {
+                if constexpr (SIMPLE && KCPLX) {  // both parts by one access
+                  using Pair = typename std::conditional<sizeof(KT) == 4, float2, double2>::type;
+                  Pair sum = *reinterpret_cast<Pair *>(at);
+                  sum.x += ar;
+                  sum.y += ai;
+                  *reinterpret_cast<Pair *>(at) = sum;
+                } else if (plain) {
                   at[0] += ar;
                   if (KCPLX) at[1] += ai;
                 } else {
@@ -304,21 +328,31 @@ __device__ __forceinline__ void gatherRows(const PlanDev &p, const KT *ke, const
 }
 
 // Blocks of 256 threads per SM the compiler makes room for: four (64
-// registers) where a lane holds one vector per element row; with more it
-// spills (30 columns in FP64: 0.113 ms with four, 0.090 without the bound;
-// 20 columns in FP64: 0.250 and 0.341 ms)
-constexpr int gatherBlocksPerSm(int laneBytes, bool simple) { return simple && laneBytes <= 24 ? 4 : 1; }
+// registers) where a lane holds few bytes of an element row and the kernel is
+// a lean one, else two, which leaves the others as many warps as their loads
+// need: with four blocks they spill (35 columns: complex FP32 127 us a call on
+// 6,000 order-4 tetrahedra, two 99.8; complex FP64 370 and 293), without a
+// bound the general kernel takes up to 174 registers (35 columns in complex
+// FP64 with element vectors 526 us, two 424, three 689).
+// The lean kernels against the general one, which took these calls before:
+// complex 35 columns in FP32 (10,368 tetrahedra) 288 us a call, now 147; upper
+// storage on 48,000 order-3 tetrahedra 139 and 101, outputs added to 244 and
+// 160.
+constexpr int gatherBlocksPerSm(int laneBytes, int mode) {
+  return mode == kGatherGeneral ? 2 : laneBytes <= 24 ? 4 : 2;
+}
 
-template <typename SlotT, bool KCPLX, typename KT, int VW, int J, bool BLOCKS, bool ACC, bool SIMPLE>
-__global__ void __launch_bounds__(256, gatherBlocksPerSm(VW * J * (int)sizeof(KT), SIMPLE))
+template <typename SlotT, bool KCPLX, typename KT, int VW, int J, bool BLOCKS, bool ACC, int MODE>
+__global__ void __launch_bounds__(256, gatherBlocksPerSm(VW * J * (int)sizeof(KT) * (KCPLX ? 2 : 1), MODE))
     k_gather(const PlanDev p, const KT *ke, const double2 *be, const double2 *uD, double2 *__restrict__ values,
              double2 *__restrict__ rhs, const GatherLanes g, KeLayout lay, int64_t v0, int64_t v1) {
-  gatherRows<SlotT, KCPLX, KT, VW, J, BLOCKS, ACC, SIMPLE>(p, ke, be, uD, values, rhs, g, lay, blockIdx.x, gridDim.x, v0, v1);
+  gatherRows<SlotT, KCPLX, KT, VW, J, BLOCKS, ACC, MODE>(p, ke, be, uD, values, rhs, g, lay, blockIdx.x, gridDim.x, v0, v1);
 }
 
 // Many plans in one launch: job q owns blocks [blockStart, blockStart + nBlocks)
-template <typename SlotT, bool KCPLX, typename KT, int VW, int J, bool BLOCKS, bool SIMPLE>
-__global__ void __launch_bounds__(256, gatherBlocksPerSm(VW * J * (int)sizeof(KT), SIMPLE)) k_gather_batch(const GatherJob *__restrict__ jobs, int nJobs, const GatherLanes g) {
+template <typename SlotT, bool KCPLX, typename KT, int VW, int J, bool BLOCKS, int MODE>
+__global__ void __launch_bounds__(256, gatherBlocksPerSm(VW * J * (int)sizeof(KT) * (KCPLX ? 2 : 1), MODE))
+    k_gather_batch(const GatherJob *__restrict__ jobs, int nJobs, const GatherLanes g) {
   int lo = 0, hi = nJobs - 1;
   while (lo < hi) {  // last job whose blockStart <= blockIdx.x
     const int mid = (lo + hi + 1) >> 1;
@@ -326,7 +360,7 @@ __global__ void __launch_bounds__(256, gatherBlocksPerSm(VW * J * (int)sizeof(KT
     else hi = mid - 1;
   }
   const GatherJob &Jb = jobs[lo];
-  gatherRows<SlotT, KCPLX, KT, VW, J, BLOCKS, false, SIMPLE>(Jb.p, (const KT *)Jb.ke, Jb.be, Jb.uD, Jb.values, Jb.rhs, g, Jb.lay,
+  gatherRows<SlotT, KCPLX, KT, VW, J, BLOCKS, false, MODE>(Jb.p, (const KT *)Jb.ke, Jb.be, Jb.uD, Jb.values, Jb.rhs, g, Jb.lay,
                                                              (int64_t)blockIdx.x - Jb.blockStart, Jb.nBlocks, 0, (int64_t)Jb.p.nRows);
 }
 
@@ -334,9 +368,11 @@ __global__ void __launch_bounds__(256, gatherBlocksPerSm(VW * J * (int)sizeof(KT
 struct GatherLaunch {
   GatherShape g;
   int slotBytes, kcplx;
-  bool acc, simple;
+  bool acc;
+  int mode;
   bool early;  // may start before the element kernel ends
   int64_t blocks;
+  bool capped;  // fewer blocks than row groups
   cudaStream_t s;
   // a single plan
   const PlanDev *p;
@@ -350,34 +386,46 @@ struct GatherLaunch {
   int nJobs;
 };
 
-template <typename SlotT, bool KCPLX, typename KT, int VW, int J, bool BLOCKS, bool SIMPLE>
+template <typename SlotT, bool KCPLX, typename KT, int VW, int J, bool BLOCKS, int MODE>
 int launchGatherBatchKernel(const GatherLaunch &a) {
-  auto kern = k_gather_batch<SlotT, KCPLX, KT, VW, J, BLOCKS, SIMPLE>;
+  auto kern = k_gather_batch<SlotT, KCPLX, KT, VW, J, BLOCKS, MODE>;
   static SmemAllowance allowed;
   FG_CUDA(allowSmem(kern, a.g.smem, allowed));
   kern<<<(unsigned)a.blocks, 32u * (unsigned)a.g.wpb, a.g.smem, a.s>>>(a.jobs, a.nJobs, a.g.lanes);
   FG_CUDA(cudaGetLastError());
   return FG_OK;
 }
-template <typename SlotT, bool KCPLX, typename KT, int VW, int J, bool BLOCKS, bool ACC, bool SIMPLE>
+template <typename SlotT, bool KCPLX, typename KT, int VW, int J, bool BLOCKS, bool ACC, int MODE>
 int launchGatherKernel(const GatherLaunch &a) {
-  auto kern = k_gather<SlotT, KCPLX, KT, VW, J, BLOCKS, ACC, SIMPLE>;
+  auto kern = k_gather<SlotT, KCPLX, KT, VW, J, BLOCKS, ACC, MODE>;
   static SmemAllowance allowed;
   FG_CUDA(allowSmem(kern, a.g.smem, allowed));
-  FG_CUDA(launchDependent(a.early, kern, (unsigned)a.blocks, 32u * (unsigned)a.g.wpb, a.g.smem, a.s, *a.p, (const KT *)a.ke, a.be, a.uD,
+  int64_t blocks = a.blocks;
+  if (a.capped) {
+    // whole rounds of the blocks that are resident at once: with 28 warps per
+    // SM of 64 in the grid the last round was a quarter full (complex order 3,
+    // 48,000 tetrahedra 190 us a call, with 56 in the grid 182)
+    int resident = 0;
+    FG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, 32 * a.g.wpb, a.g.smem));
+    const int warps = std::max(resident, 1) * a.g.wpb;
+    blocks = (int64_t)smCount() * std::max(resident, 1) * std::max(1, (kGatherWarpsPerSm + warps / 2) / warps);
+  }
+  FG_CUDA(launchDependent(a.early, kern, (unsigned)blocks, 32u * (unsigned)a.g.wpb, a.g.smem, a.s, *a.p, (const KT *)a.ke, a.be, a.uD,
                           a.values, a.rhs, a.g.lanes, a.lay, a.v0, a.v1));
   return FG_OK;
 }
 template <typename SlotT, bool KCPLX, typename KT, int VW, int J, bool BLOCKS>
 int launchGatherShape(const GatherLaunch &a) {
-  if constexpr (!KCPLX) {
-    if (a.simple && !a.acc)
-      return a.jobs ? launchGatherBatchKernel<SlotT, KCPLX, KT, VW, J, BLOCKS, true>(a)
-                    : launchGatherKernel<SlotT, KCPLX, KT, VW, J, BLOCKS, false, true>(a);
+#define FG_GATHER_MODE(M)                                                              \
+  (a.jobs  ? launchGatherBatchKernel<SlotT, KCPLX, KT, VW, J, BLOCKS, M>(a)            \
+   : a.acc ? launchGatherKernel<SlotT, KCPLX, KT, VW, J, BLOCKS, true, M>(a)           \
+           : launchGatherKernel<SlotT, KCPLX, KT, VW, J, BLOCKS, false, M>(a))
+  switch (a.mode) {
+    case kGatherClean: return FG_GATHER_MODE(kGatherClean);
+    case kGatherOpen: return FG_GATHER_MODE(kGatherOpen);
+    default: return FG_GATHER_MODE(kGatherGeneral);
   }
-  if (a.jobs) return launchGatherBatchKernel<SlotT, KCPLX, KT, VW, J, BLOCKS, false>(a);
-  return a.acc ? launchGatherKernel<SlotT, KCPLX, KT, VW, J, BLOCKS, true, false>(a)
-               : launchGatherKernel<SlotT, KCPLX, KT, VW, J, BLOCKS, false, false>(a);
+#undef FG_GATHER_MODE
 }
 
 int launchGatherF32(const GatherLaunch &a);

@@ -338,7 +338,7 @@ int launchMultiShape(const MultiLaunch &a) {
 template <typename SlotT, typename KT, int VW, int J, bool BLOCKS>
 int launchMultiReal(const MultiLaunch &a) {
   if (a.in.G != 2) return launchMultiShape<SlotT, KT, VW, J, BLOCKS, 3, false>(a);
-  return gatherSimple(*a.p, a.in.be) ? launchMultiShape<SlotT, KT, VW, J, BLOCKS, 2, false, true>(a)
+  return gatherMode(*a.p, a.in.be) == kGatherClean ? launchMultiShape<SlotT, KT, VW, J, BLOCKS, 2, false, true>(a)
                                      : launchMultiShape<SlotT, KT, VW, J, BLOCKS, 2, false>(a);
 }
 
