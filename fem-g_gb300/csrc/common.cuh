@@ -354,6 +354,8 @@ inline int gatherMode(const PlanDev &p, const void *be) {
   if (p.lscale || be || !p.plainSlots) return kGatherGeneral;
   return p.cleanSlots ? kGatherClean : p.nFixed ? kGatherGeneral : kGatherOpen;
 }
+// frees ptr if it is the columns of an fg_pattern_build call (pattern.cu)
+bool freePatternColumns(void *ptr);
 // the records of the visiting order, from its (element, local row) list
 int buildRecords(const PlanDev &p, const uint32_t *visitElem, int64_t entries, uint32_t *rec);
 // mode: the least gatherMode() of the jobs

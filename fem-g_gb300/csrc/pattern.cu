@@ -28,6 +28,8 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <mutex>
+#include <unordered_set>
 #include <vector>
 
 #include "common.cuh"
@@ -348,7 +350,25 @@ void *hostColumns(size_t bytes) {
   return p;
 }
 
+// The columns that callers hold: plain memory, which fg_host_free must not
+// tell from its page-locked buffers by what CUDA says of the address, as a
+// caller may have page-locked them since
+std::mutex g_columnsMutex;
+std::unordered_set<void *> g_columns;
+
 }  // namespace
+
+bool femg::freePatternColumns(void *ptr) {
+  {
+    std::lock_guard<std::mutex> lk(g_columnsMutex);
+    if (g_columns.erase(ptr) == 0) return false;
+  }
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, ptr) != cudaSuccess) cudaGetLastError();
+  else if (a.type == cudaMemoryTypeHost && cudaHostUnregister(ptr) != cudaSuccess) cudaGetLastError();
+  std::free(ptr);
+  return true;
+}
 
 extern "C" int fg_pattern_build(const uint64_t *elem_dof_idx, const int32_t *elem_dof_type, int64_t n_elements, int32_t n_dofs,
                                 uint64_t n_rows, uint64_t *ai, uint64_t **aj, int32_t upper, const uint64_t *linked_row,
@@ -484,6 +504,10 @@ extern "C" int fg_pattern_build(const uint64_t *elem_dof_idx, const int32_t *ele
     std::free(out);
     setLastError("fg_pattern_build: copy of the pattern failed");
     return FG_ERR_CUDA;
+  }
+  {
+    std::lock_guard<std::mutex> lk(g_columnsMutex);
+    g_columns.insert(out);
   }
   *aj = (uint64_t *)out;
   return FG_OK;

@@ -14,7 +14,6 @@
 #include <algorithm>
 #include <atomic>
 #include <complex>
-#include <cstdlib>
 #include <cstring>
 #include <mutex>
 
@@ -1159,16 +1158,8 @@ int fg_host_alloc(void **ptr, size_t bytes) {
   return FG_OK;
 }
 
-// fg_host_alloc's buffers are page-locked, fg_pattern_build's columns plain
-// host memory
 void fg_host_free(void *ptr) {
-  if (!ptr) return;
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, ptr) == cudaSuccess && a.type == cudaMemoryTypeUnregistered) {
-    std::free(ptr);
-    return;
-  }
-  cudaGetLastError();
+  if (!ptr || freePatternColumns(ptr)) return;
   cudaFreeHost(ptr);
 }
 

@@ -429,7 +429,8 @@ const char *fg_batch_tuning(const fg_batch *batch);
  * that have I, Fixed DOFs take no column, and the bubble rows of an element
  * after its first alias that row. elem_dof_idx / elem_dof_type as in
  * fg_system_desc ([n_elements][n_dofs]). ai: [n_rows + 1], the caller's;
- * *aj: [ai[n_rows]] allocated by the call (free it with fg_host_free).
+ * *aj: [ai[n_rows]] allocated by the call, pageable memory (free it with
+ * fg_host_free, which also undoes a cudaHostRegister of it).
  * upper = 1: symmetric storage, only the columns J >= I of a row (for an
  * aliased bubble row, those of the first bubble's row). linked_row
  * ([n_linked], as in fg_system_desc): an FG_AT_LINKED DOF is a row and a
@@ -467,7 +468,8 @@ int64_t fg_launch_count(void);
 int fg_profile_enable(int on);
 int fg_profile_read(char *names, int32_t name_bytes, int64_t *launches, double *total_ms, int32_t cap);
 
-/* page-locked host buffers for end-to-end transfers */
+/* page-locked host buffers for end-to-end transfers; fg_host_free also frees
+ * the columns of fg_pattern_build */
 int fg_host_alloc(void **ptr, size_t bytes);
 void fg_host_free(void *ptr);
 
