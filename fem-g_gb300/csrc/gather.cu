@@ -194,7 +194,9 @@ int buildRecords(const PlanDev &p, const uint32_t *visitElem, int64_t entries, u
                                                       words, p.n, recWords, rec);
   countLaunch();
   FG_CUDA(cudaGetLastError());
-  FG_CUDA(cudaDeviceSynchronize());
+  // the kernel's own stream alone: a wait for the device would end captures
+  // that other streams have under way
+  FG_CUDA(cudaStreamSynchronize(nullptr));
   return FG_OK;
 }
 
