@@ -22,7 +22,6 @@
 namespace femg {
 
 constexpr int kFacTile = 64;  // elements per tile (one orientation)
-constexpr int kFacMax = 12;   // factors per element row
 
 struct FactoredState {
   int built = 0;
@@ -173,6 +172,7 @@ static size_t factoredSmem(int n, int kp, int ncomp, int EC) {
   return (EC * ncomp * nn2 + 1 + kp * np + (size_t)kFacTile * (kp + 4)) * 8 + (np * 2 + 7) / 8 * 8;
 }
 constexpr size_t kFacSmem = 54 * 1024;
+constexpr size_t kFacSmemMax = 220 * 1024;  // (a block may hold 227 KB)
 static int factoredRound(int n, int kp, int ncomp) {
   const int np = n * (n + 1) / 2;
   int best = 1;
@@ -262,10 +262,10 @@ bool factoredFp64Applies(const fg_plan *plan, const DevTerms &terms) {
     return false;
   for (int t = 0; t < terms.n; ++t)
     if (terms.t[t].kind != FG_TERM_SOURCE && terms.t[t].coef.cls == kExprPoint) return false;
-  // the reference tensors have to fit a block's shared memory whole (HCurl of
-  // order 2 on tetrahedra, 45 functions, does not: the quadrature loop applies)
-  const size_t kp = p.form == FG_FORM_1 ? 12 : 7;
-  return (kp * p.n * p.n + (size_t)kFacTile * 2 * kFacMax) * sizeof(double) <= 200 * 1024;
+  // the upper triangles of an orientation's reference tensors and one element
+  // have to fit a block's shared memory: all H1 elements, HCurl ones up to 61
+  // functions (real) or 57 (complex)
+  return factoredSmem(p.n, p.form == FG_FORM_1 ? 12 : 7, terms.complexKe ? 2 : 1, 1) <= kFacSmemMax;
 }
 
 bool factoredFp64Ready(const fg_plan *plan) {
@@ -285,11 +285,7 @@ int launchFactoredFp64(fg_plan *plan, const DevTerms &terms, const DevTerms *dte
   if (f->nTiles == 0) return FG_OK;
   const bool cplx = terms.complexKe != 0;
   const int EC = factoredRound(p.n, f->kp, cplx ? 2 : 1);
-  const size_t smem = factoredSmem(p.n, f->kp, cplx ? 2 : 1, EC);
-  if (smem > 220 * 1024) {
-    setLastError("FP64 factored kernel: reference tensors larger than shared memory");
-    return FG_ERR_UNSUPPORTED;
-  }
+  const size_t smem = factoredSmem(p.n, f->kp, cplx ? 2 : 1, EC);  // within the limit by factoredFp64Applies
   auto kern = cplx ? k_element_factored_fp64<true> : k_element_factored_fp64<false>;
   static SmemAllowance allowed[2];
   FG_CUDA(allowSmem(kern, smem, allowed[cplx]));
