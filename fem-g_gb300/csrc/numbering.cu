@@ -9,7 +9,9 @@
 // of (key, input index) by eight bits a pass, least first, each pass stable.
 // The numbering sorts every DOF by one more pass over its class (Unknown,
 // Unknown bubble, other), so that the host neither picks out nor spreads the
-// DOFs: on 195,112 DOFs, 0.63 ms a call in place of 2.4.
+// DOFs: on 195,112 DOFs, 0.63 ms a call in place of 2.4. A radix sort is 18 to
+// 29 launches whatever the size; up to kBlockSort items are sorted by one
+// block instead.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -19,7 +21,10 @@
 
 namespace femg {
 
-constexpr int kRadixThreads = 256, kRadixWarps = 8, kRadixTile = 4096;  // 512 consecutive items per warp
+constexpr int kRadixThreads = 256, kRadixWarps = 8;
+constexpr int kRadixTile = 4096, kRadixTileSmall = 1024;  // 512 or 128 consecutive items per warp
+constexpr uint32_t kRadixSmall = 65536;  // up to so many items: small tiles, whose counts the scatter scans itself
+constexpr uint32_t kBlockSort = 8192;  // up to so many: one block
 
 struct HilbertDev {
   uint8_t code[24][8];
@@ -27,10 +32,12 @@ struct HilbertDev {
 };
 
 // Keys of the points pts [n][stride], index i beside each. cls (may be null):
-// the class of DOF i by its assemble type
+// the class of DOF i by its assemble type. count (may be null): for the sort by
+// one block, the classes go with the indices, and DOFs that get no number are
+// left out (the order of the others does not matter to that sort)
 __global__ void k_hilbert_keys(int dim, uint64_t n, const float *__restrict__ pts, int stride, float3 scale, float3 scaleMin,
                                const HilbertDev tab, uint64_t *__restrict__ keys, uint32_t *__restrict__ idx,
-                               const int32_t *__restrict__ type, uint8_t *__restrict__ cls) {
+                               const int32_t *__restrict__ type, uint8_t *__restrict__ cls, uint32_t *__restrict__ count) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float sc[3] = {scale.x, scale.y, scale.z}, sm[3] = {scaleMin.x, scaleMin.y, scaleMin.z};
@@ -46,9 +53,87 @@ __global__ void k_hilbert_keys(int dim, uint64_t n, const float *__restrict__ pt
     h ^= tab.code[ed][l];
     ed = tab.next[ed][l];
   }
+  const uint32_t c = !cls ? 0u : type[i] == FG_AT_UNKNOWN ? 0u : type[i] == FG_AT_UNKNOWN_BUBBLE ? 1u : 2u;
+  if (count) {
+    if (c == 2u) return;
+    const uint32_t at = atomicAdd(count, 1u);
+    keys[at] = h;
+    idx[at] = c << 30 | (uint32_t)i;
+    return;
+  }
   keys[i] = h;
   idx[i] = (uint32_t)i;
-  if (cls) cls[i] = type[i] == FG_AT_UNKNOWN ? 0 : type[i] == FG_AT_UNKNOWN_BUBBLE ? 1 : 2;
+  if (cls) cls[i] = (uint8_t)c;
+}
+
+struct SortItem {
+  uint64_t key;
+  uint32_t idx;  // class << 30 | index
+};
+__device__ __forceinline__ void sortPair(SortItem &a, SortItem &b, bool up) {
+  const uint32_t ca = a.idx >> 30, cb = b.idx >> 30;
+  // no two items are equal but the padding
+  const bool after = ca != cb ? ca > cb : a.key != b.key ? a.key > b.key : a.idx > b.idx;
+  if (after == up) {
+    const SortItem t = a;
+    a = b;
+    b = t;
+  }
+}
+
+// Sort of up to kBlockSort items by (class, key, index) in one block: a bitonic
+// network over `padded` (a power of two) items in shared memory, two strides
+// at a time; then the order itself, or numbers from 1 on. Shared memory skips a
+// place after every 16 items, which takes most of the small strides' bank
+// conflicts away.
+__device__ __forceinline__ uint32_t sortPlace(uint32_t i) { return i + (i >> 4); }
+__global__ void __launch_bounds__(1024) k_sort_block(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ idx, uint32_t n,
+                                                    uint32_t padded, uint32_t *__restrict__ perm, uint64_t *__restrict__ num) {
+  extern __shared__ __align__(16) uint64_t sk[];
+  uint32_t *si = reinterpret_cast<uint32_t *>(sk + sortPlace(padded));
+  for (uint32_t t = threadIdx.x; t < padded; t += blockDim.x) {
+    sk[sortPlace(t)] = t < n ? keys[t] : ~0ull;
+    si[sortPlace(t)] = t < n ? idx[t] : 0xFFFFFFFFu;  // after every item
+  }
+  __syncthreads();
+  for (uint32_t lgk = 1; (1u << lgk) <= padded; ++lgk) {
+    const uint32_t k = 1u << lgk;
+    uint32_t lgj = lgk;  // the strides below 2^lgj are left
+    if (lgk & 1) {       // an odd number of them: the largest by itself
+      --lgj;
+      const uint32_t j = 1u << lgj;
+      for (uint32_t t = threadIdx.x; t < padded / 2; t += blockDim.x) {
+        const uint32_t lo = 2 * t - (t & (j - 1)), pl = sortPlace(lo), ph = sortPlace(lo + j);
+        SortItem a = {sk[pl], si[pl]}, b = {sk[ph], si[ph]};
+        sortPair(a, b, (lo & k) == 0);
+        sk[pl] = a.key, si[pl] = a.idx;
+        sk[ph] = b.key, si[ph] = b.idx;
+      }
+      __syncthreads();
+    }
+    for (; lgj > 0; lgj -= 2) {
+      const uint32_t q = 1u << (lgj - 2);  // strides 2q, then q
+      for (uint32_t t = threadIdx.x; t < padded / 4; t += blockDim.x) {
+        const uint32_t lo = 4 * t - 3 * (t & (q - 1));
+        const bool up = (lo & k) == 0;
+        SortItem v[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) v[c] = {sk[sortPlace(lo + c * q)], si[sortPlace(lo + c * q)]};
+        sortPair(v[0], v[2], up);
+        sortPair(v[1], v[3], up);
+        sortPair(v[0], v[1], up);
+        sortPair(v[2], v[3], up);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) sk[sortPlace(lo + c * q)] = v[c].key, si[sortPlace(lo + c * q)] = v[c].idx;
+      }
+      __syncthreads();
+    }
+  }
+  for (uint32_t t = threadIdx.x; t < n; t += blockDim.x) {
+    const uint32_t i = si[sortPlace(t)] & 0x3FFFFFFFu;
+    if (perm) perm[t] = i;
+    else num[i] = t + 1;
+  }
 }
 
 // The digit of item k in a pass: eight bits of its key, or its DOF's class
@@ -61,12 +146,12 @@ struct RadixDigit {
 };
 
 // Digit counts of a tile into hist[digit][tile]
-__global__ void __launch_bounds__(kRadixThreads) k_radix_count(const RadixDigit d, uint64_t n, uint32_t tiles, uint32_t *__restrict__ hist) {
+__global__ void __launch_bounds__(kRadixThreads) k_radix_count(const RadixDigit d, uint64_t n, uint32_t tile, uint32_t tiles, uint32_t *__restrict__ hist) {
   __shared__ uint32_t h[256];
   h[threadIdx.x] = 0;
   __syncthreads();
-  const uint64_t end = min(n, ((uint64_t)blockIdx.x + 1) * kRadixTile);
-  for (uint64_t k = (uint64_t)blockIdx.x * kRadixTile + threadIdx.x; k < end; k += kRadixThreads) atomicAdd(&h[d.at(k)], 1u);
+  const uint64_t end = min(n, ((uint64_t)blockIdx.x + 1) * tile);
+  for (uint64_t k = (uint64_t)blockIdx.x * tile + threadIdx.x; k < end; k += kRadixThreads) atomicAdd(&h[d.at(k)], 1u);
   __syncthreads();
   hist[(uint64_t)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
@@ -100,8 +185,10 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scan(uint32_t *__restri
 
 // The items of a tile to their places: after all items of smaller digits,
 // those of the digit in earlier tiles, in earlier warps of this one (a warp
-// has 512 consecutive items) and earlier in the warp (32 at a time, the equal
-// digits of which are matched)
+// has consecutive items) and earlier in the warp (32 at a time, the equal
+// digits of which are matched). SMALL: hist holds the tiles' counts as they
+// are, and there are few enough of them to be summed here.
+template <bool SMALL>
 __global__ void __launch_bounds__(kRadixThreads)
     k_radix_scatter(const RadixDigit d, uint64_t n, uint32_t tiles, const uint32_t *__restrict__ hist, const uint32_t *__restrict__ totals,
                     uint64_t *__restrict__ keysOut, uint32_t *__restrict__ idxOut) {
@@ -110,12 +197,23 @@ __global__ void __launch_bounds__(kRadixThreads)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int w = 0; w < kRadixWarps; ++w) place[w][tid] = 0;
   __syncthreads();
-  constexpr int kPer = kRadixTile / kRadixWarps;
-  const uint64_t w0 = (uint64_t)blockIdx.x * kRadixTile + (uint64_t)warp * kPer;
+  constexpr int kTile = SMALL ? kRadixTileSmall : kRadixTile, kPer = kTile / kRadixWarps;
+  const uint64_t w0 = (uint64_t)blockIdx.x * kTile + (uint64_t)warp * kPer;
   for (int r = 0; r < kPer; r += 32)
     if (w0 + r + lane < n) atomicAdd(&place[warp][d.at(w0 + r + lane)], 1u);
   // exclusive scan of the digits' totals, one digit per thread
-  const uint32_t total = totals[tid];
+  uint32_t total = 0, earlier = 0;  // of the digit, and in earlier tiles
+  if (SMALL) {
+#pragma unroll 4
+    for (uint32_t t = 0; t < tiles; ++t) {
+      const uint32_t c = hist[(uint64_t)tid * tiles + t];
+      total += c;
+      earlier += t < blockIdx.x ? c : 0u;
+    }
+  } else {
+    total = totals[tid];
+    earlier = hist[(uint64_t)tid * tiles + blockIdx.x];
+  }
   uint32_t inc = total;
   for (int off = 1; off < 32; off <<= 1) {
     const uint32_t o = __shfl_up_sync(0xffffffffu, inc, off);
@@ -123,7 +221,7 @@ __global__ void __launch_bounds__(kRadixThreads)
   }
   if (lane == 31) warpSum[warp] = inc;
   __syncthreads();
-  uint32_t at = inc - total + hist[(uint64_t)tid * tiles + blockIdx.x];
+  uint32_t at = inc - total + earlier;
   for (int w = 0; w < warp; ++w) at += warpSum[w];
   for (int w = 0; w < kRadixWarps; ++w) {
     const uint32_t c = place[w][tid];
@@ -154,10 +252,16 @@ __global__ void k_number(const uint32_t *__restrict__ idx, uint64_t n, const uin
 }
 
 // Stable Hilbert order of n points (float [n][stride], in host memory) in the
-// box [mn, mx]: into perm; or, with the assemble types, the DOFs' numbers
-// into num.
+// box [mn, mx]: into perm; or, with the assemble types, the numbers of the
+// DOFs, `sorted` of which get one, into num.
+// One block up to kBlockSort items: 25 DOFs 149 us a call and 281 by the radix
+// sort of 4,096-item tiles, 5,101 DOFs to number among 10,201 234 and 427; at
+// 9,000 points, 16,384 places of the network, it would be past the radix
+// sort, which took 263 there by small tiles and 390 by large ones. Those are
+// worth it up to kRadixSmall (60,000 points 318 and 405), beyond which the sum
+// over the tiles' counts in every block grows too long.
 static int hilbertOrderGpu(int dim, uint64_t n, const float *pts, int stride, const float *mn, const float *mx, uint32_t *perm,
-                           const int32_t *type, uint64_t *num) {
+                           const int32_t *type, uint64_t *num, uint64_t sorted) {
   if (n == 0) return FG_OK;
   // scale as the host sort computes it (float)
   const unsigned nbrBits = 64 / dim;
@@ -169,7 +273,8 @@ static int hilbertOrderGpu(int dim, uint64_t n, const float *pts, int stride, co
   }
   HilbertDev tab;
   hilbertTableData(dim, &tab.code[0][0], &tab.next[0][0]);
-  const uint32_t tiles = (uint32_t)((n + kRadixTile - 1) / kRadixTile);
+  const bool small = n <= kRadixSmall;
+  const uint32_t tile = small ? kRadixTileSmall : kRadixTile, tiles = (uint32_t)((n + tile - 1) / tile);
   size_t bytes = 0;
   auto part = [&](size_t b) {
     const size_t at = bytes;
@@ -178,7 +283,8 @@ static int hilbertOrderGpu(int dim, uint64_t n, const float *pts, int stride, co
   };
   const size_t oPts = part(n * stride * sizeof(float)), oType = part(type ? n * 4 : 0), oCls = part(type ? n : 0),
                oNum = part(type ? n * 8 : 0), oK0 = part(n * 8), oK1 = part(n * 8), oI0 = part(n * 4), oI1 = part(n * 4),
-               oHist = part((size_t)256 * tiles * 4), oTotals = part(256 * 4);
+               oHist = part((size_t)256 * tiles * 4), oTotals = part(256 * 4), oCount = part(4);
+  const bool oneBlock = sorted <= kBlockSort && n <= (uint64_t(1) << 30);
   uint8_t *base = nullptr;
   if (cudaMalloc(&base, bytes) != cudaSuccess) {
     cudaGetLastError();
@@ -195,19 +301,37 @@ static int hilbertOrderGpu(int dim, uint64_t n, const float *pts, int stride, co
     if (e == cudaSuccess && type) e = cudaMemcpyAsync(base + oNum, num, n * 8, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return e;
     const unsigned nb = (unsigned)((n + 255) / 256);
+    uint32_t *count = oneBlock ? (uint32_t *)(base + oCount) : nullptr;
+    if (count && (e = cudaMemsetAsync(count, 0, 4)) != cudaSuccess) return e;
     k_hilbert_keys<<<nb, 256>>>(dim, n, (const float *)(base + oPts), stride, make_float3(sc[0], sc[1], sc[2]),
-                                make_float3(sm[0], sm[1], sm[2]), tab, keys[0], idx[0], (const int32_t *)(base + oType), cls);
+                                make_float3(sm[0], sm[1], sm[2]), tab, keys[0], idx[0], (const int32_t *)(base + oType), cls, count);
+    if (oneBlock) {
+      uint32_t padded = 64;
+      while (padded < sorted) padded <<= 1;
+      const size_t smem = (size_t)(padded + padded / 16) * 12;
+      static SmemAllowance allowed;
+      if ((e = allowSmem(k_sort_block, smem, allowed)) != cudaSuccess) return e;
+      k_sort_block<<<1, std::min(1024u, padded / 2), smem>>>(keys[0], idx[0], (uint32_t)sorted, padded, type ? nullptr : idx[1],
+                                                            (uint64_t *)(base + oNum));
+      countLaunch(2);
+      if ((e = cudaGetLastError()) != cudaSuccess) return e;
+      return type ? cudaMemcpy(num, base + oNum, n * 8, cudaMemcpyDeviceToHost) : cudaMemcpy(perm, idx[1], n * 4, cudaMemcpyDeviceToHost);
+    }
     const int passes = 8 + (type ? 1 : 0);
     for (int q = 0; q < passes; ++q) {
       const int a = q & 1;
       const RadixDigit d = {keys[a], idx[a], q == 8 ? cls : nullptr, 8 * q};
-      k_radix_count<<<tiles, kRadixThreads>>>(d, n, tiles, hist);
-      k_radix_scan<<<256, kRadixThreads>>>(hist, tiles, totals);
-      k_radix_scatter<<<tiles, kRadixThreads>>>(d, n, tiles, hist, totals, keys[a ^ 1], idx[a ^ 1]);
+      k_radix_count<<<tiles, kRadixThreads>>>(d, n, tile, tiles, hist);
+      if (small) {
+        k_radix_scatter<true><<<tiles, kRadixThreads>>>(d, n, tiles, hist, totals, keys[a ^ 1], idx[a ^ 1]);
+      } else {
+        k_radix_scan<<<256, kRadixThreads>>>(hist, tiles, totals);
+        k_radix_scatter<false><<<tiles, kRadixThreads>>>(d, n, tiles, hist, totals, keys[a ^ 1], idx[a ^ 1]);
+      }
     }
     const uint32_t *order = idx[passes & 1];
     if (type) k_number<<<nb, 256>>>(order, n, cls, (uint64_t *)(base + oNum));
-    countLaunch(1 + 3 * passes + (type ? 1 : 0));
+    countLaunch(1 + (small ? 2 : 3) * passes + (type ? 1 : 0));
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     return type ? cudaMemcpy(num, base + oNum, n * 8, cudaMemcpyDeviceToHost) : cudaMemcpy(perm, order, n * 4, cudaMemcpyDeviceToHost);
   };
@@ -234,7 +358,7 @@ extern "C" int fg_hilbert_order(int32_t dim, uint64_t n, const float *pts, const
     setLastError("fg_hilbert_order: no CUDA device");
     return FG_ERR_NO_DEVICE;
   }
-  return hilbertOrderGpu(dim, n, pts, dim, mn, mx, perm, nullptr, nullptr);
+  return hilbertOrderGpu(dim, n, pts, dim, mn, mx, perm, nullptr, nullptr, n);
 }
 
 extern "C" int fg_hilbert_numbering(int32_t dim, const double *bbox, uint64_t n_dofs, const float *xyz, const int32_t *assemble_type,
@@ -243,8 +367,10 @@ extern "C" int fg_hilbert_numbering(int32_t dim, const double *bbox, uint64_t n_
     setLastError("fg_hilbert_numbering: invalid arguments");
     return FG_ERR_ARG;
   }
-  uint64_t nUnknown = 0;  // without any, nothing is numbered and no device is needed
-  for (uint64_t i = 0; i < n_dofs && !nUnknown; ++i)
+  // the DOFs that get a number, as far as it matters: without any, no device
+  // is needed
+  uint64_t nUnknown = 0;
+  for (uint64_t i = 0; i < n_dofs && nUnknown <= kBlockSort; ++i)
     nUnknown += assemble_type[i] == FG_AT_UNKNOWN || assemble_type[i] == FG_AT_UNKNOWN_BUBBLE;
   if (nUnknown == 0) return FG_OK;
   // the box widened by a relative 1e-6, as the reference does (DofsManager.cpp)
@@ -263,5 +389,5 @@ extern "C" int fg_hilbert_numbering(int32_t dim, const double *bbox, uint64_t n_
     setLastError("fg_hilbert_numbering: no CUDA device");
     return FG_ERR_NO_DEVICE;
   }
-  return hilbertOrderGpu(dim, n_dofs, xyz, 3, mn, mx, nullptr, assemble_type, num_dof);
+  return hilbertOrderGpu(dim, n_dofs, xyz, 3, mn, mx, nullptr, assemble_type, num_dof, nUnknown);
 }
