@@ -30,7 +30,6 @@
 // The element matrices and vectors then go through the deterministic CSR
 // reduction of gather.cu.
 #include <algorithm>
-#include <cmath>
 #include <cstring>
 
 #include "common.cuh"
@@ -825,7 +824,8 @@ __global__ void __launch_bounds__(kQuadThreads, UNIFORM ? 4 : 2)
 // SM runs blocks / SMs of them, of which those that are resident at once hide
 // each other's gaps (kBusy: how busy one alone keeps the pipe). So small
 // meshes get few elements per block, large ones what fills the rounds best. D
-// is formed for QD points at a time, H for QC of these.
+// is formed for QD points at a time, H for QC of these. (The search takes 0.1
+// to 3 us of the host's time.)
 // Measured: with kBusy 0.3 and 0.6, and barriers of 12 instructions, a dozen
 // calls take the same time but for 10 to 35% more on one or two small meshes
 // each; without the blocks' overlap (kBusy 1) triangles of order 3 (8,192)
@@ -836,28 +836,29 @@ static bool quadShape(const PlanDev &p, int nEnt, int n, int nF, int nd, int nh,
   constexpr double kBusy = 0.45;
   const int64_t sms = smCount();
   auto bytes = [&](int NE, int QD, int QC) { return (size_t)quadLayout(NE, QD, QC, p.nn, n, a->ng, nd, nh, be, nPairs).total * 8; };
-  auto rounds = [](int64_t items) { return (items + kQuadThreads - 1) / kQuadThreads; };
   auto parts = [](int of, int by) { return (of + by - 1) / by; };
-  double best = 0.0;
+  auto rounds = [&](int items) { return parts(items, kQuadThreads); };
+  double best = 0.0, idles[8] = {1.0};
+  for (int k = 1; k < 8; ++k) idles[k] = idles[k - 1] * (1.0 - kBusy);
   a->NE = 0;
-  for (int NE = 1; NE <= kQuadMaxElems && (int64_t)NE * nEnt <= (int64_t)kQuadThreads * maxItems; ++NE) {
-    if (NE > 1 && bytes(NE, 1, 1) > kQuadSmem) break;
+  for (int NE = 1; NE <= kQuadMaxElems && NE * nEnt <= kQuadThreads * maxItems; NE += NE < 24 ? 1 : 4) {
+    // shared memory without D and H, and a point of each
+    const int rest = (int)bytes(NE, 0, 0), dPoint = (int)bytes(NE, 1, 0) - rest, hPoint = NE * nh * 8;
+    const int room = (int)kQuadSmem - rest;
+    if (room < dPoint + hPoint) break;
+    if (NE > 1 && (NE > 24 ? NE - 4 : NE - 1) * sms >= p.E) break;  // more elements per block would leave SMs without any
     const int64_t blocks = (p.E + NE - 1) / NE, perSm = (blocks + sms - 1) / sms;
-    const int resident = (int)std::min<int64_t>(perSm, blocksPerSm);
-    const double busy = 1.0 - std::pow(1.0 - kBusy, resident);
-    for (int c = 1, last = 0; c <= p.nq; ++c) {
+    const double each = (double)perSm / (1.0 - idles[std::min<int64_t>(perSm, blocksPerSm)]);
+    const double fixed = (double)(rounds(NE * nEnt) * p.nq * comps + 60);
+    if (a->NE && each * fixed >= best) continue;  // (without the chunks already as long)
+    const int fewest = parts(p.nq, std::min(p.nq, (room - hPoint) / dPoint));
+    for (int c = fewest; c <= fewest + 2 && c <= p.nq; ++c) {
       const int QD = parts(p.nq, c), nD = parts(p.nq, QD);
-      if (QD == last || bytes(NE, QD, 1) > kQuadSmem) continue;
-      last = QD;
-      int QC = std::min(QD, 16);
-      while (QC > 1 && bytes(NE, QD, QC) > kQuadSmem) --QC;
-      const int least = parts(QD, QC);
-      for (int h = least; h <= least + 3 && h <= QD; ++h) {
-        QC = parts(QD, h);
-        const int nH = parts(QD, QC);
-        const int64_t block = rounds((int64_t)NE * nEnt) * p.nq * comps + nD * nH * rounds((int64_t)NE * QC * nF) * hCost +
-                              nD * rounds((int64_t)NE * QD) * dCost + 60 + kBarrier * nD * (1 + nH);
-        const double cost = (double)perSm * (double)block / busy;
+      const int most = std::min(std::min(QD, 16), (room - QD * dPoint) / hPoint);
+      for (int h = parts(QD, most), end = std::min(h + 1, QD); h <= end; ++h) {
+        const int QC = parts(QD, h), nH = parts(QD, QC);
+        const int chunks = nD * (nH * rounds(NE * QC * nF) * hCost + rounds(NE * QD) * dCost + kBarrier * (1 + nH));
+        const double cost = each * (fixed + chunks);
         if (a->NE == 0 || cost < best) {
           best = cost;
           a->NE = NE;
