@@ -459,12 +459,17 @@ extern "C" int fg_batch_create(fg_plan *const *plans, const fg_term_desc *const 
       if ((st = ensureDevice((void **)&pl->ke, &pl->keBytes, (size_t)pl->d.E * ncomp * pl->d.n * pl->d.n * sizeof(double)))) return fail(st);
     }
   }
-  // reduction classes: (element type, order, rule, slot width, complex, field components)
-  std::map<std::tuple<int, int, int, int, int, int, int>, int> classOf;
+  // reduction classes: (element type, order, rule, slot width, complex, field
+  // components, element-matrix layout): one kernel instance each
+  std::map<std::tuple<int, int, int, int, int, int, int, int, int>, int> classOf;
+  std::vector<KeLayout> lays(n_problems);
+  std::vector<const void *> kes(n_problems);
   for (int q = 0; q < n_problems; ++q) {
     const PlanDev &p = plans[q]->d;
     const int kc = b->terms[q].complexKe ? 1 : 0;
-    auto key = std::make_tuple(p.dim, p.nn, p.n, p.nq, p.slotBytes, kc, p.mult);
+    lays[q] = keFull(p.n);
+    kes[q] = b->mixed ? (const void *)mixedKe(plans[q], &lays[q]) : (const void *)plans[q]->ke;
+    auto key = std::make_tuple(p.dim, p.nn, p.n, p.nq, p.slotBytes, kc, p.mult, (int)lays[q].kind, (int)lays[q].ld);
     auto it = classOf.find(key);
     if (it == classOf.end()) {
       GatherClass c;
@@ -490,8 +495,8 @@ extern "C" int fg_batch_create(fg_plan *const *plans, const fg_term_desc *const 
       fg_plan *pl = plans[q];
       GatherJob &J = c.jobsHost[k];
       J.p = pl->d;
-      J.lay = keFull(pl->d.n);
-      J.ke = b->mixed ? (const void *)mixedKe(pl, &J.lay) : (const void *)pl->ke;
+      J.lay = lays[q];
+      J.ke = kes[q];
       J.be = b->source[q] ? (const double2 *)pl->be : nullptr;
       J.uD = nullptr;
     }
