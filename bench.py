@@ -54,7 +54,7 @@ GATHER_TRAFFIC_PER_NNZ_P3 = {"k_gather_v4": 999e6 / 35811451}
 # FP64-pipe activity of the plain FP64 element kernel (k_element_fp64, the
 # quadrature loop) in an ncu capture on the 16^3 x 6 P3 mesh: the loop is
 # bound by GB300's FP64 pipe
-ELEMENT_FP64_PIPE_ACTIVE_P3 = 0.921
+ELEMENT_FP64_PIPE_ACTIVE_P3 = 0.930
 
 
 def load_femg():

@@ -18,7 +18,7 @@ static int limitRows(int nc, bool vec4) {
 
 // Warps per block: 4 took 0.423 ms on 384,000 order-3 tetrahedra (FP32
 // element matrices) where 8 took 0.443, and 0.091 against 0.108 ms on 55,566
-// order-2 ones (complex FP64). With 64 warps per SM in the grid; 128 took 4%
+// order-2 ones (complex FP64, the general kernel without a bound). With 64 warps per SM in the grid; 128 took 4%
 // and a block per row group 12% longer (the pipeline starts anew in every
 // block), 32 left the second example at 0.108.
 // Columns come by vectors of VW values (16 bytes at most) where the rows of

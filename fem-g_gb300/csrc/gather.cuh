@@ -28,10 +28,11 @@
 //  - A lane's columns come by 16- or 8-byte loads where the row length allows.
 //  - The finished rows are written by OL lanes each, which also clear the
 //    accumulator for the next rows.
-// 384,000 order-3 tetrahedra, FP32 element matrices: 0.423 ms, 2.40 GB of DRAM
-// traffic at 5.7 TB/s (0.570 ms with a row's loads started anew on every row,
+// 384,000 order-3 tetrahedra, FP32 element matrices: 0.423 ms, 2.36 GB of DRAM
+// traffic at 5.6 TB/s (0.570 ms with a row's loads started anew on every row,
 // scalar adds through atomics and narrow stores); 162,000 of them in FP64
-// 0.240 ms (0.365); 55,566 order-2 ones, complex FP64 0.091 ms (0.106).
+// 0.241 ms (0.365); 55,566 order-2 ones, complex FP64 with element vectors 0.081
+// ms (0.106).
 #pragma once
 #include <algorithm>
 #include <type_traits>

@@ -51,7 +51,8 @@ static int launchGatherMulti(fg_plan *plan, const MultiIn &in, bool isFloat, cud
     setLastError("multi-frequency gather: CSR row too long for shared memory");
     return FG_ERR_UNSUPPORTED;
   }
-  // measured on 48,000 order-2 Navier tetrahedra at 8 frequencies: 0.599 ms
+  // measured on 48,000 order-2 Navier tetrahedra at 8 frequencies, there alone
+  // and 0.02 ms each before the right-hand sides lost their products: 0.599 ms
   // with 4 warps and 32 lanes writing a row, 0.608 with 8 warps, 0.631 with 16
   // lanes, 0.678 and 0.794 with 4 and 2 rows per warp in place of 6
   g.wpb = 4;

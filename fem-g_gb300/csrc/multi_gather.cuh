@@ -1,6 +1,6 @@
 // The CSR reduction of several term groups and frequencies at once (device
 // code; multi_freq.cu picks the shapes, multi_f32.cu and multi_f64.cu hold the
-// instances). 48,000 order-2 Navier tetrahedra at 8 frequencies: 0.600 ms for
+// instances). 48,000 order-2 Navier tetrahedra at 8 frequencies: 0.580 ms for
 // 2.2 GB of values written (1.28 ms without the pipeline, an atomic per group
 // and column and a table lookup and two widenings per value written). The
 // launch bound is left to the compiler: at 64 or 80 registers it spills, and
