@@ -51,13 +51,18 @@ static int launchGatherMulti(fg_plan *plan, const MultiIn &in, bool isFloat, cud
     setLastError("multi-frequency gather: CSR row too long for shared memory");
     return FG_ERR_UNSUPPORTED;
   }
-  // measured on 48,000 order-2 Navier tetrahedra at 8 frequencies, there alone
-  // and 0.02 ms each before the right-hand sides lost their products: 0.599 ms
-  // with 4 warps and 32 lanes writing a row, 0.608 with 8 warps, 0.631 with 16
-  // lanes, 0.678 and 0.794 with 4 and 2 rows per warp in place of 6
+  // warps per block: 4; 8 took 0 to 8% longer on 30 sweeps and separate
+  // matrices, scalar and of three components, in FP32 and FP64. 4 or 2 rows per
+  // warp in place of 6 took 13 and 33% longer (48,000 order-2 tetrahedra of
+  // three components, 8 frequencies).
+  // Lanes that write a row, by the mean row: on 39,200 order-1 triangles (7
+  // entries a row), 3 frequencies in FP32, 8 lanes took 51 us a call, 16 58 and
+  // 32 62; on 16,464 order-2 tetrahedra (27), 6 frequencies, 63, 61 and 64; on
+  // 6,000 of order 3 (49) 118, 105 and 105, in FP64 446, 448 and 434
   g.wpb = 4;
-  g.lanes.lgOL = 5;
-  g.lanes.OL = 32;
+  const double mean = (double)p.nnz / (double)p.nRows;
+  g.lanes.lgOL = mean < 12.0 ? 3 : mean < 40.0 ? 4 : 5;
+  g.lanes.OL = 1 << g.lanes.lgOL;
   while (g.lanes.R > 1 && cfBytes + rowBytes * g.lanes.R * g.wpb > 100 * 1024) --g.lanes.R;
   while (g.wpb > 1 && cfBytes + rowBytes * g.lanes.R * g.wpb > 200 * 1024) g.wpb >>= 1;  // (a block may hold 227 KB)
   g.smem = cfBytes + rowBytes * g.lanes.R * g.wpb;
