@@ -822,18 +822,20 @@ __global__ void __launch_bounds__(kQuadThreads, UNIFORM ? 4 : 2)
 // dCost per round of (element, point) pairs, about as long as kBarrier
 // instructions at each barrier, and about 60 for the elements' geometry; an
 // SM runs blocks / SMs of them, of which those that are resident at once hide
-// each other's gaps (kBusy: how busy one alone keeps the pipe). So small
-// meshes get few elements per block, large ones what fills the rounds best. D
-// is formed for QD points at a time, H for QC of these. (The search takes 0.1
-// to 3 us of the host's time.)
-// Measured: with kBusy 0.3 and 0.6, and barriers of 12 instructions, a dozen
-// calls take the same time but for 10 to 35% more on one or two small meshes
-// each; without the blocks' overlap (kBusy 1) triangles of order 3 (8,192)
-// take 125 us a call instead of 101, of order 6 (512) 232 instead of 170.
+// each other's gaps (kBusy: how busy one alone keeps the pipe), the last ones,
+// fewer than an SM holds, less well. So small meshes get few elements per
+// block, large ones what fills the rounds best. D is formed for QD points at a
+// time, H for QC of these. (The search takes 0.1 to 3 us of the host's time.)
+// Measured on 54 calls (triangles of order 1 to 5, tetrahedra of order 1 to 4
+// and HCurl elements, three sizes each) with every number of elements: the
+// rule's choice takes 1.6% longer than the best one on average, 22% at most;
+// without the last blocks' part 3.3% and 37%, and without the overlap
+// (kBusy 1) 512 triangles of order 6 take 232 us a call instead of 170. kBusy
+// from 0.3 to 0.4 and barriers of 2 to 12 instructions make no difference.
 static bool quadShape(const PlanDev &p, int nEnt, int n, int nF, int nd, int nh, bool be, int nPairs, int maxItems, int comps,
                       int hCost, int dCost, int blocksPerSm, QuadArgs *a) {
   constexpr int kBarrier = 4;
-  constexpr double kBusy = 0.45;
+  constexpr double kBusy = 0.35;
   const int64_t sms = smCount();
   auto bytes = [&](int NE, int QD, int QC) { return (size_t)quadLayout(NE, QD, QC, p.nn, n, a->ng, nd, nh, be, nPairs).total * 8; };
   auto parts = [](int of, int by) { return (of + by - 1) / by; };
@@ -848,7 +850,9 @@ static bool quadShape(const PlanDev &p, int nEnt, int n, int nF, int nd, int nh,
     if (room < dPoint + hPoint) break;
     if (NE > 1 && (NE > 24 ? NE - 4 : NE - 1) * sms >= p.E) break;  // more elements per block would leave SMs without any
     const int64_t blocks = (p.E + NE - 1) / NE, perSm = (blocks + sms - 1) / sms;
-    const double each = (double)perSm / (1.0 - idles[std::min<int64_t>(perSm, blocksPerSm)]);
+    const int64_t tail = perSm % blocksPerSm;
+    double each = (double)(perSm - tail) / (1.0 - idles[blocksPerSm]);
+    if (tail) each += (double)tail / (1.0 - idles[tail]);
     const double fixed = (double)(rounds(NE * nEnt) * p.nq * comps + 60);
     if (a->NE && each * fixed >= best) continue;  // (without the chunks already as long)
     const int fewest = parts(p.nq, std::min(p.nq, (room - hPoint) / dPoint));
